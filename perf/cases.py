@@ -326,10 +326,14 @@ def _add(scene, verts, idx):
     return scene.AddGeom_Triangles3f(verts, len(verts), idx, idx.size, BUILD_HIGH, 12)
 
 
+def _hit_views(hits):
+    """The views of an array of hits that a program reads: t, the three ids, the coordinates."""
+    return {"t": hits[:, 0], "ids": hits.view(torch.int32)[:, 1:4], "coords": hits[:, 4:8]}
+
+
 def _hit_buffer(n):
-    """A device array of hits and the views of it that a program reads: t, the three ids, the coordinates."""
     hits = torch.zeros((n, 8), device="cuda")
-    return hits, {"t": hits[:, 0], "ids": hits.view(torch.int32)[:, 1:4], "coords": hits[:, 4:8]}
+    return hits, _hit_views(hits)
 
 
 def _segments(counts):
@@ -430,12 +434,19 @@ def _prepare_served(case, d, st):
     for k in st["scenes"]:
         if sv.scene_state(k, -1.0) != engine.SCENE_READY:
             raise RuntimeError("a served scene was not built")
-    st["requests"] = []
+    st["requests"], st["buffers"], st["out"] = [], [], []
     for k, r in enumerate(d["rays"]):
         kind = k % 2
-        out = torch.zeros((r.shape[0], 8), pin_memory=True) if kind == NEAREST else torch.zeros(
-            r.shape[0], dtype=torch.uint8, pin_memory=True)
-        st["requests"].append((st["scenes"][k % len(st["scenes"])], kind, r.cpu().pin_memory(), out))
+        if kind == NEAREST:
+            buffer = torch.zeros((r.shape[0], 8), pin_memory=True)
+            out = _hit_views(buffer)
+        else:
+            buffer = out = torch.zeros(r.shape[0], dtype=torch.uint8, pin_memory=True)
+        rays = r.cpu().pin_memory()
+        st["buffers"].append((rays, buffer))
+        st["requests"].append((st["scenes"][k % len(st["scenes"])], kind, rays.data_ptr(), r.shape[0],
+                               buffer.data_ptr()))
+        st["out"].append(out)
 
 
 _PREPARE = {"trace": _prepare_trace, "host": _prepare_trace, "build": _prepare_build, "refit": _prepare_refit,
@@ -456,14 +467,11 @@ def _run_trace(st):
     return st["out"]
 
 
-def _hit_arrays(h):
-    return {"t": h["t"], "ids": np.stack([h["primId"], h["instId"], h["geomId"]], axis=-1), "coords": h["coords"]}
-
-
 def _run_host(st):
     if st["kind"] == ANY:
         return st["scene"].RayQuery_AnyHit(st["rays"])
-    return _hit_arrays(st["scene"].RayQuery_NearestHit(st["rays"]))
+    h = st["scene"].RayQuery_NearestHit(st["rays"])
+    return {"t": h["t"], "ids": h.view(np.uint32).reshape(-1, 8)[:, 1:4], "coords": h["coords"]}
 
 
 def _trace_rays(st):
@@ -518,14 +526,11 @@ def _run_frame(st):
 
 def _run_served(st):
     sv = st["server"]
-    tickets = [sv.submit(scene, kind, rays.data_ptr(), rays.shape[0], out.data_ptr())
-               for scene, kind, rays, out in st["requests"]]
-    for t in tickets:
+    for t in [sv.submit(*r) for r in st["requests"]]:
         status, _ = sv.wait(t)
         if status != engine.HRT_OK:
             raise RuntimeError("a request failed")
-    return [{"t": o[:, 0], "ids": o.view(torch.int32)[:, 1:4], "coords": o[:, 4:8]} if kind == NEAREST else o
-            for _, kind, _, o in st["requests"]]
+    return st["out"]
 
 
 _RUN = {"trace": _run_trace, "host": _run_host, "build": _run_build, "refit": _run_refit, "instances": _run_instances,
