@@ -126,6 +126,10 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
 // Traversal view of a geometry under an instance transform (inv12: rows 0..2
 // of the inverse; identity when null).
 void make_instance_desc(const Geom& g, uint32_t geomId, uint32_t instId, const float* inv12, InstanceDesc& d);
+// Nearest hits of a renderer's eye rays, as hrt_query_nearest: neighbours in
+// the order given (imageWidth 0) or in a row-major image this wide see the
+// same part of the scene, and the launch shape may rely on it.
+int query_eye_rays(hrt_scene* s, const float* rays, uint64_t n, int imageWidth, hrt_hit* hits, cudaStream_t stream);
 // Column-major 4x4 -> rows 0..2 of its inverse (the reference checker's evaluation).
 void inverse4x4(const float* mc, float* inv12);
 bool is_identity(const float* m);

@@ -226,6 +226,8 @@ struct TraceConfig
   int stackEntries = 0;       // stack entries per lane in shared memory, the rest in local
                               // memory; 0 (or at least the depth bound): all in shared memory
   int imageWidth = 0;         // > 0: rays form row-major images this wide, traced in 4 x 8 tiles
+  int raysPerWarp = 32;       // one thread per ray: rays of a warp (its first lanes); set per launch
+  bool given = false;         // the caller set this shape; else a launch may choose its refill threshold
 };
 
 // kind 0: nearest, 1: any.  counting = 1 also accumulates counters (node

@@ -742,7 +742,8 @@ int hrt_frame_render_eye(hrt_frame* f, hrt_scene* s, const float projInv[16], co
   k_frame_eye_rays<<<grid_for(n, ctx->numSMs), kThreads, 0, cs>>>(p, v, width, height, packed, 0.0f, FLT_MAX, f->rays,
                                                                   f->pixel);
   HRT_CUDA(ctx, cudaGetLastError());
-  if ((st = hrt_query_nearest(s, reinterpret_cast<const float*>(f->rays), n, f->hits, stream))) return st;
+  if ((st = query_eye_rays(s, reinterpret_cast<const float*>(f->rays), n, packed ? 0 : (int)width, f->hits, cs)))
+    return st;
   uint32_t* out = nullptr;
   if ((st = color_target(f, colors, n, &out))) return st;
   k_eye_colors<<<grid_for(n, ctx->numSMs), kThreads, 0, cs>>>(f->hits, f->pixel, n, out);
@@ -802,7 +803,8 @@ int hrt_frame_render_rtao(hrt_frame* f, hrt_scene* s, const hrt_rtao_params* prm
   k_frame_eye_rays<<<grid, kThreads, 0, cs>>>(p, v, prm->width, prm->height, packed, prm->zNear, prm->zFar, f->rays,
                                               f->pixel);
   HRT_CUDA(ctx, cudaGetLastError());
-  if ((st = hrt_query_nearest(s, reinterpret_cast<const float*>(f->rays), n, f->hits, stream))) return st;
+  if ((st = query_eye_rays(s, reinterpret_cast<const float*>(f->rays), n, packed ? 0 : (int)prm->width, f->hits, cs)))
+    return st;
   k_rtao_positions<<<grid, kThreads, 0, cs>>>(f->rays, f->hits, f->pixel, n, f->dGeoms, (uint32_t)hg.size(),
                                               f->dNormMat, nInst, f->positions, f->flag, dErr);
   const uint32_t nBlocks = (uint32_t)((n + kThreads * kChunk - 1) / (kThreads * kChunk));

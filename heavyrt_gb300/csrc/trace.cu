@@ -14,11 +14,56 @@ cudaError_t trace_w1(const TraceArgs& a, int kind, int counting, const TraceConf
 cudaError_t trace_w2(const TraceArgs& a, int kind, int counting, const TraceConfig& c, int numSMs, cudaStream_t s);
 cudaError_t trace_w3(const TraceArgs& a, int kind, int counting, const TraceConfig& c, int numSMs, cudaStream_t s);
 
-cudaError_t trace(const TraceArgs& a, int kind, int counting, int layout, const TraceConfig& c, int numSMs,
+namespace
+{
+
+// Warps an SM that a small batch is spread over, and that hold a batch at once.
+constexpr int kSpreadWarps = 13, kResidentWarps = 36;
+// Idle lanes at which a warp refills unless the caller set a shape.
+constexpr int kRefillLanes = 8;
+
+// The shape of one launch.
+//
+// A batch that does not fill the GPU's warps is bound by the slowest warp's
+// chain of dependent instructions, and a warp of 32 rays that part ways runs
+// all their chains: such a batch is spread, the fewest rays a warp (a power of
+// two) for which 13 warps an SM suffice, one thread per ray.  Random rays into
+// a soup, us, 32 rays a warp against the spread: 96 rays into 2,003 triangles
+// 41 -> 27 (binary), 34 -> 20 (FP16 nodes); 1,000 rays into 20,000 triangles
+// 90 -> 62, 72 -> 45; 8,000 rays into 100,000 triangles 155 -> 125, 127 -> 103
+// (at 4 rays a warp; at 1: 143, 143); 30,000 rays 169 -> 156, 134 -> 127 (at
+// 16; at 8: 161, 158); 100,000 rays are faster at 32 (210 against 260 at 16).
+// A batch whose rays are all resident at once gains nothing from the pool and
+// goes without its counter and the memset before it (100,000 rays 210 -> 208,
+// FP16 nodes 180 -> 170); 262,144 eye rays are faster in the pool (binary 157
+// against 172).
+//
+// The refill threshold: incoherent rays want idle lanes filled early (500,000
+// random rays, 8-bit nodes: 652 us at 24 lanes, 555 at 8; FP16 582 -> 520),
+// and coherent ones do not care (full-HD eye rays 156 against 157).
+TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int numSMs)
+{
+  TraceConfig s = c;
+  if (!c.given && s.refillLanes > kRefillLanes) s.refillLanes = kRefillLanes;
+  int perWarp = 32;
+  while (perWarp > 1 && a.n <= (uint64_t)numSMs * kSpreadWarps * (perWarp / 2)) perWarp /= 2;
+  if (a.n <= (uint64_t)numSMs * kResidentWarps * 32)
+  {
+    s.raysPerWarp = perWarp;
+    s.persistent = 0;
+    s.threadsPerBlock = 64;
+  }
+  return s;
+}
+
+}  // namespace
+
+cudaError_t trace(const TraceArgs& a, int kind, int counting, int layout, const TraceConfig& config, int numSMs,
                   cudaStream_t s)
 {
   if (a.n == 0) return cudaSuccess;
   if (a.n > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // the pool's counter may overshoot n by a few warps
+  const TraceConfig c = counting ? config : launch_shape(a, config, numSMs);
   if (a.triTest == 1)
     switch (layout)
     {

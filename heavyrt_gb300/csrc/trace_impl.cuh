@@ -85,6 +85,7 @@ struct RayOrder
   uint32_t nWork;        // work items (>= rays; tiles that cross the image edge pad it)
   uint32_t width;        // 0: work item i is ray i
   uint32_t tilesPerRow;
+  uint32_t perWarp;      // work items of a warp of the one-thread-per-ray kernels (its first lanes)
 };
 
 __device__ __forceinline__ uint32_t work_ray(const RayOrder& o, uint32_t i, uint32_t n)
@@ -98,9 +99,22 @@ __device__ __forceinline__ uint32_t work_ray(const RayOrder& o, uint32_t i, uint
   return r < n ? (uint32_t)r : kNoRay;
 }
 
-__host__ __forceinline__ RayOrder ray_order(uint32_t n, int width)
+// Work item of a thread of the one-thread-per-ray kernels.
+template <int THREADS> __device__ __forceinline__ uint32_t grid_work(const RayOrder& o)
 {
-  RayOrder o{n, 0u, 0u};
+  const uint32_t lane = threadIdx.x & 31u;
+  return lane < o.perWarp ? (blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5)) * o.perWarp + lane : kNoRay;
+}
+
+template <int THREADS> __host__ __forceinline__ uint32_t grid_blocks(const RayOrder& o)
+{
+  const uint64_t perBlock = (uint64_t)(THREADS / 32) * o.perWarp;
+  return (uint32_t)((o.nWork + perBlock - 1) / perBlock);
+}
+
+__host__ __forceinline__ RayOrder ray_order(uint32_t n, int width, int perWarp)
+{
+  RayOrder o{n, 0u, 0u, (uint32_t)perWarp};
   if (width <= 0 || n == 0) return o;
   const uint64_t w = (uint64_t)width;
   const uint64_t tilesPerRow = (w + 3) / 4, rows = (n + w - 1) / w;
@@ -1240,7 +1254,7 @@ __global__ void __launch_bounds__(THREADS) k_trace_grid(const float4* __restrict
   uint32_t local[STACK != kStackShared ? StackDepth<LAYOUT, TLAS>::value : 1];
   Stack<THREADS, STACK> st{s_stack + threadIdx.x, local, stackShared};
   uint64_t nPairs = 0, nTris = 0;
-  const uint32_t w = blockIdx.x * THREADS + threadIdx.x;
+  const uint32_t w = grid_work<THREADS>(order);
   const uint32_t i = w < order.nWork ? work_ray(order, w, n) : kNoRay;
   Lane<LAYOUT> L;
   L.cur = kDone;
@@ -1431,7 +1445,7 @@ __global__ void __launch_bounds__(THREADS)
   extern __shared__ uint32_t s_stack[];  // stackShared * THREADS entries
   uint32_t local[STACK != kStackShared ? StackDepth<LAYOUT, false>::value : 1];
   Stack<THREADS, STACK> st{s_stack + threadIdx.x, local, stackShared};
-  const uint32_t w = blockIdx.x * THREADS + threadIdx.x;
+  const uint32_t w = grid_work<THREADS>(order);
   const uint32_t i = w < order.nWork ? work_ray(order, w, n) : kNoRay;
   if (i == kNoRay) return;
   Lane1<LAYOUT> L;
@@ -1457,7 +1471,7 @@ cudaError_t launch_one(const TraceArgs& a, const TraceConfig& c, int numSMs, cud
   const uint32_t n = (uint32_t)a.n;
   const int shared = STACK == kStackLocal ? 0 : shared_entries<StackDepth<LAYOUT, false>::value>(c.stackEntries);
   const size_t smem = sizeof(uint32_t) * (size_t)shared * THREADS;
-  const RayOrder order = ray_order(n, c.imageWidth);
+  const RayOrder order = ray_order(n, c.imageWidth, c.raysPerWarp);
   OneSource src = {};
   if (SEG)
   {
@@ -1494,7 +1508,7 @@ cudaError_t launch_one(const TraceArgs& a, const TraceConfig& c, int numSMs, cud
   {
     cudaError_t e = allow_smem(k_trace_one_grid<LAYOUT, TRI, ANY, THREADS, STACK, SEG>, smem);
     if (e != cudaSuccess) return e;
-    lc.gridDim = dim3((uint32_t)(((uint64_t)order.nWork + THREADS - 1) / THREADS));
+    lc.gridDim = dim3(grid_blocks<THREADS>(order));
     return cudaLaunchKernelEx(&lc, k_trace_one_grid<LAYOUT, TRI, ANY, THREADS, STACK, SEG>, a.rays, n, src, a.hits,
                               a.errorWord, shared, order);
   }
@@ -1553,7 +1567,7 @@ cudaError_t launch(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStr
                      : STACK == kStackSplit ? shared_entries<StackDepth<LAYOUT, TLAS>::value>(c.stackEntries)
                                             : StackDepth<LAYOUT, TLAS>::value;
   const size_t smem = sizeof(uint32_t) * (size_t)shared * THREADS;
-  const RayOrder order = ray_order(n, c.imageWidth);
+  const RayOrder order = ray_order(n, c.imageWidth, c.raysPerWarp);
   if (c.persistent && !COUNT)
   {
     cudaError_t e = allow_smem(k_trace_pool<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK>, smem);
@@ -1576,8 +1590,8 @@ cudaError_t launch(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStr
   {
     cudaError_t e = allow_smem(k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK>, smem);
     if (e != cudaSuccess) return e;
-    const uint64_t blocks = ((uint64_t)order.nWork + THREADS - 1) / THREADS;
-    k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK><<<(uint32_t)blocks, THREADS, smem, s>>>(
+    const uint32_t blocks = grid_blocks<THREADS>(order);
+    k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK><<<blocks, THREADS, smem, s>>>(
         a.rays, n, a.inst, sg, tl, a.hits, a.counters, a.errorWord, shared, order);
   }
   return cudaGetLastError();
