@@ -13,6 +13,7 @@
 // sort is the stable segmented radix sort; a run never crosses a segment.
 #include "build_common.cuh"
 #include "hrt_kernels.cuh"
+#include "leaf_tree.cuh"
 
 namespace hrt
 {
@@ -209,89 +210,13 @@ __global__ void __launch_bounds__(1024) k_seg_offsets(const uint32_t* __restrict
   }
 }
 
-// kernel1D_MakeLeavesFromTriangles per geometry (core/builders/lbvh.cpp:350-384),
-// plus the sorted triangle records and index buffer; a geometry with a single
-// leaf also gets its one record (leaf + empty slot) here.
-__global__ void __launch_bounds__(kThreads) k_seg_leaves(
-    const float4* __restrict__ v, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ vertOffsets,
-    const uint32_t* __restrict__ triOffsets, const uint32_t* __restrict__ leafOffsets,
-    const uint32_t* __restrict__ nodeOffsets, const uint32_t* __restrict__ recOffsets, uint32_t G,
-    const uint32_t* __restrict__ counts, const uint32_t* __restrict__ sortedTri, const uint32_t* __restrict__ runStarts,
-    BVHNode32* __restrict__ lr, uint32_t* __restrict__ lrCount, TriRec* __restrict__ tris,
-    uint32_t* __restrict__ sortedIdx, PairRec* __restrict__ recs, uint32_t* errorWord, int vertexRecords)
-{
-  const uint32_t Ltot = counts[0];
-  for (uint32_t g = blockIdx.x * kThreads + threadIdx.x; g < Ltot; g += gridDim.x * kThreads)
-  {
-    const uint32_t s = find_segment(leafOffsets, G, g);
-    const uint32_t L = leafOffsets[s + 1] - leafOffsets[s];
-    const uint32_t k = g - leafOffsets[s];
-    const uint32_t tb = triOffsets[s], vb = vertOffsets[s], nV = vertOffsets[s + 1] - vb;
-    const uint32_t start = runStarts[g];
-    const uint32_t end = (k + 1 < L) ? runStarts[g + 1] : triOffsets[s + 1];
-    if (k >= L || end > triOffsets[s + 1] || start >= end || start < tb)
-    {
-      atomicOr(errorWord, kErrLayout);
-      continue;
-    }
-    const uint32_t count = end - start;
-    if (count > 127u) atomicOr(errorWord, kErrLeafCount);
-    float mn[3] = {1e10f, 1e10f, 1e10f}, mx[3] = {-1e10f, -1e10f, -1e10f};
-    for (uint32_t j = start; j < end; j++)
-    {
-      const uint32_t tri = sortedTri[j];  // global triangle index
-      uint32_t ia = idx[3 * (size_t)tri + 0], ib = idx[3 * (size_t)tri + 1], ic = idx[3 * (size_t)tri + 2];
-      if (ia >= nV || ib >= nV || ic >= nV)
-      {
-        atomicOr(errorWord, kErrIndexRange);
-        ia = ib = ic = 0;
-      }
-      const float4 a = v[vb + ia], b = v[vb + ib], c = v[vb + ic];
-      mn[0] = lm_min(mn[0], lm_min(a.x, lm_min(b.x, c.x)));
-      mn[1] = lm_min(mn[1], lm_min(a.y, lm_min(b.y, c.y)));
-      mn[2] = lm_min(mn[2], lm_min(a.z, lm_min(b.z, c.z)));
-      mx[0] = lm_max(mx[0], lm_max(a.x, lm_max(b.x, c.x)));
-      mx[1] = lm_max(mx[1], lm_max(a.y, lm_max(b.y, c.y)));
-      mx[2] = lm_max(mx[2], lm_max(a.z, lm_max(b.z, c.z)));
-      TriRec r;
-      r.a = make_float4(a.x, a.y, a.z, __uint_as_float(j + 1 == end ? 3u : 0u));
-      r.e1 = make_float4(__fsub_rn(b.x, a.x), __fsub_rn(b.y, a.y), __fsub_rn(b.z, a.z), __uint_as_float(tri - tb));
-      r.e2 = make_float4(__fsub_rn(c.x, a.x), __fsub_rn(c.y, a.y), __fsub_rn(c.z, a.z), 0.0f);
-      if (vertexRecords)
-      {
-        r.e1 = make_float4(b.x, b.y, b.z, __uint_as_float(tri - tb));
-        r.e2 = make_float4(c.x, c.y, c.z, 0.0f);
-      }
-      tris[j] = r;
-      sortedIdx[3 * (size_t)j + 0] = ia;
-      sortedIdx[3 * (size_t)j + 1] = ib;
-      sortedIdx[3 * (size_t)j + 2] = ic;
-    }
-    BVHNode32 nd;
-    nd.boxMin[0] = mn[0]; nd.boxMin[1] = mn[1]; nd.boxMin[2] = mn[2];
-    nd.boxMax[0] = mx[0]; nd.boxMax[1] = mx[1]; nd.boxMax[2] = mx[2];
-    nd.leftOffset = pack_offset_and_size(start - tb, count);
-    nd.escapeIndex = 0xFFFFFFFFu;
-    lr[nodeOffsets[s] + L - 1 + k] = nd;
-    lrCount[nodeOffsets[s] + L - 1 + k] = 0;
-    if (L == 1u && recs != nullptr)
-    {
-      PairRec r;
-      r.a = make_float4(mn[0], mn[1], mn[2], mx[0]);
-      r.b = make_float4(mx[1], mx[2], 0.0f, 0.0f);
-      r.c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      r.d = make_uint4(kLeafBit | (start - tb), kEmptyRef, 0u, 0u);
-      recs[recOffsets[s]] = r;
-    }
-  }
-}
-
 __global__ void __launch_bounds__(kThreads) k_seg_karras(const uint32_t* __restrict__ compressed,
                                                          const uint32_t* __restrict__ leafOffsets,
                                                          const uint32_t* __restrict__ intOffsets,
                                                          const uint32_t* __restrict__ nodeOffsets, uint32_t G,
                                                          const uint32_t* __restrict__ counts, BVHNode32* __restrict__ lr,
-                                                         uint32_t* __restrict__ parent, uint32_t* __restrict__ rangeEnd)
+                                                         uint32_t* __restrict__ parent, uint32_t* __restrict__ visit,
+                                                         uint32_t* __restrict__ rangeEnd)
 {
   const uint32_t Itot = counts[1];
   // one node per thread; a warp's 32 consecutive internal nodes exchange
@@ -318,83 +243,7 @@ __global__ void __launch_bounds__(kThreads) k_seg_karras(const uint32_t* __restr
     parent[nb + left] = (uint32_t)i;
     parent[nb + right] = (uint32_t)i;
     rangeEnd[j] = (uint32_t)other;
-  }
-}
-
-// Bottom-up refit per geometry (as k_refit in build.cu, local numbering).
-__global__ void __launch_bounds__(bc::kRefitThreads, bc::kRefitMinBlocks) k_seg_refit(const uint32_t* __restrict__ leafOffsets,
-                                                        const uint32_t* __restrict__ intOffsets,
-                                                        const uint32_t* __restrict__ nodeOffsets, uint32_t G,
-                                                        const uint32_t* __restrict__ counts, BVHNode32* lr,
-                                                        uint32_t* lrCount, const uint32_t* __restrict__ parent,
-                                                        uint32_t* visit, const uint32_t* __restrict__ rangeEnd,
-                                                        uint32_t* errorWord)
-{
-  // A block owns the global leaves [lo, hi).  Internal node p of geometry s
-  // (leaf base lb) with range [a, b] lies in the slice when lb + a >= lo and
-  // lb + b < hi; such nodes finish with shared-memory counters indexed by
-  // lb + p (unique across geometries, inside the slice), the others with the
-  // device-wide counters, as in the single-geometry refit.
-  __shared__ uint32_t s_visit[bc::kRefitSlice];
-  const uint32_t Ltot = counts[0];
-  const uint32_t lo = blockIdx.x * bc::kRefitSlice;
-  if (lo >= Ltot) return;
-  const uint32_t hi = min(lo + bc::kRefitSlice, Ltot);
-  for (uint32_t k = threadIdx.x; k < bc::kRefitSlice; k += bc::kRefitThreads) s_visit[k] = 0u;
-  __syncthreads();
-  for (uint32_t g = lo + threadIdx.x; g < hi; g += bc::kRefitThreads)
-  {
-    const uint32_t s = find_segment(leafOffsets, G, g);
-    const uint32_t lb = leafOffsets[s];
-    const uint32_t L = leafOffsets[s + 1] - lb;
-    const uint32_t nb = nodeOffsets[s], ib = intOffsets[s];
-    uint32_t node = L - 1 + (g - lb);
-    bool inSlice = true;
-    while (node != 0)
-    {
-      const uint32_t p = parent[nb + node];
-      if (p + 1u >= L)
-      {
-        atomicOr(errorWord, kErrLayout);
-        break;
-      }
-      if (inSlice)
-      {
-        const uint32_t j = rangeEnd[ib + p];
-        inSlice = lb + (p < j ? p : j) >= lo && lb + (p > j ? p : j) < hi;
-      }
-      uint32_t l, r;
-      float4 alo, ahi, blo, bhi;
-      uint32_t cl, cr;
-      if (inSlice)
-      {
-        if (bc::atomic_add_acq_rel_cta(&s_visit[lb + p - lo], 1u) == 0u) break;
-        if (p == 0u) visit[ib] = 2u;  // the root finished inside the slice (k_seg_records checks the counter)
-        l = lr[nb + p].leftOffset;
-        r = lr[nb + p].escapeIndex;
-        const float4* a = reinterpret_cast<const float4*>(lr + nb + l);
-        const float4* b = reinterpret_cast<const float4*>(lr + nb + r);
-        alo = a[0];
-        ahi = a[1];
-        blo = b[0];
-        bhi = b[1];
-        cl = lrCount[nb + l];
-        cr = lrCount[nb + r];
-      }
-      else
-      {
-        if (bc::atomic_add_acq_rel(&visit[ib + p], 1u) == 0u) break;
-        l = __ldcg(&lr[nb + p].leftOffset);
-        r = __ldcg(&lr[nb + p].escapeIndex);
-        bc::load_node_cg(lr + nb + l, alo, ahi);
-        bc::load_node_cg(lr + nb + r, blo, bhi);
-        cl = __ldcg(&lrCount[nb + l]);
-        cr = __ldcg(&lrCount[nb + r]);
-      }
-      bc::store_parent(lr + nb + p, alo, ahi, blo, bhi, l, r);
-      lrCount[nb + p] = cl + cr + 2u;
-      node = p;
-    }
+    visit[j] = 0u;
   }
 }
 
@@ -427,12 +276,11 @@ __global__ void __launch_bounds__(kThreads) k_seg_records(const uint32_t* __rest
     const uint32_t i = j - intOffsets[s];
     if (i == 0 && visit[j] != 2u) atomicOr(errorWord, kErrLayout);  // the refit reached this root twice
     const uint32_t nb = nodeOffsets[s], tb = triOffsets[s], lb = leafOffsets[s];
-    const BVHNode32 n = lr[nb + i];
-    const BVHNode32 a = lr[nb + n.leftOffset];
-    const BVHNode32 b = lr[nb + n.escapeIndex];
-    const uint32_t lref = (n.leftOffset < L - 1) ? n.leftOffset : (kLeafBit | (runStarts[lb + n.leftOffset - (L - 1)] - tb));
-    const uint32_t rref =
-        (n.escapeIndex < L - 1) ? n.escapeIndex : (kLeafBit | (runStarts[lb + n.escapeIndex - (L - 1)] - tb));
+    const uint32_t left = lr[nb + i].leftOffset, right = lr[nb + i].escapeIndex;
+    const BVHNode32 a = bc::load_node(lr + nb + left);
+    const BVHNode32 b = bc::load_node(lr + nb + right);
+    const uint32_t lref = (left < L - 1) ? left : (kLeafBit | (runStarts[lb + left - (L - 1)] - tb));
+    const uint32_t rref = (right < L - 1) ? right : (kLeafBit | (runStarts[lb + right - (L - 1)] - tb));
     PairRec r;
     r.a = make_float4(a.boxMin[0], a.boxMin[1], a.boxMin[2], a.boxMax[0]);
     r.b = make_float4(a.boxMax[1], a.boxMax[2], b.boxMin[0], b.boxMin[1]);
@@ -506,18 +354,36 @@ cudaError_t build_lbvh_batch(const BatchBuffers& b, int numSMs, cudaStream_t s)
   k_seg_offsets<<<1, 1024, 0, s>>>(b.runStarts, b.triOffsets, G, b.counts, b.leafOffsets, b.intOffsets, b.nodeOffsets,
                                    b.recOffsets, b.params);
   const uint32_t g = grid_for(N, numSMs, 8);
-  e = cudaMemsetAsync(b.parent, 0xFF, sizeof(uint32_t) * 2 * (size_t)N, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(b.visit, 0, sizeof(uint32_t) * N, s);
-  if (e != cudaSuccess) return e;
-  k_seg_leaves<<<g, kThreads, 0, s>>>(b.verts, b.idx, b.vertOffsets, b.triOffsets, b.leafOffsets, b.nodeOffsets,
-                                      b.recOffsets, G, b.counts, b.vals, b.runStarts, b.lr, b.lrCount, b.tris,
-                                      b.sortedIdx, b.recs, b.errorWord, b.vertexRecords);
   k_seg_karras<<<g, kThreads, 0, s>>>(b.compressed, b.leafOffsets, b.intOffsets, b.nodeOffsets, G, b.counts, b.lr,
-                                      b.parent, b.visit + N);
-  k_seg_refit<<<(N + bc::kRefitSlice - 1) / bc::kRefitSlice, bc::kRefitThreads, 0, s>>>(
-      b.leafOffsets, b.intOffsets, b.nodeOffsets, G, b.counts, b.lr, b.lrCount, b.parent, b.visit, b.visit + N,
-      b.errorWord);
+                                      b.parent, b.visit, b.visit + N);
+  bc::LeafTree t = {};
+  t.verts = b.verts;
+  t.idx = b.idx;
+  t.sortedTri = b.vals;
+  t.runStarts = b.runStarts;
+  t.nTris = N;
+  t.lr = b.lr;
+  t.lrCount = b.lrCount;
+  t.tris = b.tris;
+  t.sortedIdx = b.sortedIdx;
+  t.parent = b.parent;
+  t.visit = b.visit;
+  t.rangeEnd = b.visit + N;
+  t.open = b.keysAlt;  // free after the sort
+  t.openCount = scanCounter + 1;
+  t.errorWord = b.errorWord;
+  t.vertexRecords = b.vertexRecords;
+  t.vertOffsets = b.vertOffsets;
+  t.triOffsets = b.triOffsets;
+  t.leafOffsets = b.leafOffsets;
+  t.intOffsets = b.intOffsets;
+  t.nodeOffsets = b.nodeOffsets;
+  t.recOffsets = b.recOffsets;
+  t.counts = b.counts;
+  t.G = G;
+  t.recs = b.recs;
+  bc::k_leaf_tree<true><<<(N + bc::kSlice - 1) / bc::kSlice, bc::kSlice, 0, s>>>(t);
+  bc::k_climb<true><<<bc::climb_blocks(N, numSMs), 128, 0, s>>>(t);
   k_seg_records<<<g, kThreads, 0, s>>>(b.triOffsets, b.leafOffsets, b.intOffsets, b.nodeOffsets, b.recOffsets, G,
                                        b.counts, b.lr, b.runStarts, b.visit, b.recs, b.errorWord);
   k_seg_localize<<<g, kThreads, 0, s>>>(b.triOffsets, b.leafOffsets, G, N, b.counts, b.runStarts, b.vals);

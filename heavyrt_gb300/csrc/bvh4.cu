@@ -15,13 +15,16 @@
 // under it (the leftmost of equals) into that slot's two children, in place.
 // The slots' shapes alone decide, so a refit (same topology) keeps the tree.
 // Which binary nodes become 4-wide nodes then depends on the choices above
-// them: the roles are found top down, one 4-wide level per launch, each level
-// a frontier list built with atomics (the roles do not depend on the order
-// within a level; the numbering is the same Karras-order scan as before).
+// them: the roles are found top down, by one block until some hundred 4-wide
+// nodes are in hand and then by a block for each of their subtrees (the roles
+// do not depend on the order; the numbering is the same Karras-order scan as
+// with the even-depth rule).
 //
 // Quantised boxes only ever contain the FP32 box they stand for, so a
 // traversal of the quantised tree visits every node the FP32 tree would and
 // can only add visits; the triangle test is unchanged.
+#include <algorithm>
+
 #include <cuda_fp16.h>
 
 #include "build_common.cuh"
@@ -48,10 +51,12 @@ __device__ __forceinline__ uint8_t node_depth(const uint32_t* __restrict__ paren
   return (uint8_t)d;
 }
 
-__global__ void __launch_bounds__(kThreads) k_depth(const BuildParams* __restrict__ params,
-                                                    const uint32_t* __restrict__ parent, uint8_t* __restrict__ depth)
+__global__ void __launch_bounds__(kThreads) k_depth(BuildParams* __restrict__ params,
+                                                    const uint32_t* __restrict__ parent,
+                                                    const uint32_t* __restrict__ visit, uint8_t* __restrict__ depth)
 {
   const uint32_t L = params->nLeaves;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && L >= 2u && visit[0] != 2u) atomicOr(&params->error, kErrLayout);
   for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i + 1 < L; i += gridDim.x * kThreads)
     depth[i] = node_depth(parent, L, i);
 }
@@ -115,145 +120,293 @@ __device__ __forceinline__ int collapse_slots(const BVHNode32* __restrict__ lr, 
     cand[3] = b1;
     return (in0 ? 2 : 1) + (in1 ? 2 : 1);
   }
+  // Links and counts are read a round ahead of the choices that need them:
+  // the children's, then those of the two nodes that the first opening brings.
+  // Three dependent rounds instead of six (a leaf's count reads 0 and it is
+  // never opened).
+  struct Link
+  {
+    uint32_t id, left, right, count;  // count 0: a leaf
+  };
+  auto link = [&](uint32_t id) {
+    Link q{id, 0u, 0u, 0u};
+    if (id + 1u < L)
+    {
+      q.left = lr[id].leftOffset;
+      q.right = lr[id].escapeIndex;
+      q.count = lrCount[id];
+    }
+    return q;
+  };
+  const Link a = link(k0), b = link(k1);
   cand[0] = k0;
   cand[1] = k1;
   cand[2] = cand[3] = 0u;
-  int n = 2;
-#pragma unroll
-  for (int it = 0; it < 2; it++)
+  if (a.count == 0u && b.count == 0u) return 2;
+  const bool open0 = a.count >= b.count;  // the leftmost of equals; a leaf's 0 is less than any node's 2
+  const Link x = link(open0 ? a.left : b.left), y = link(open0 ? a.right : b.right);
+  // slots now: x, y, b or a, x, y
+  const Link s0 = open0 ? x : a, s1 = open0 ? y : x, s2 = open0 ? b : y;
+  cand[0] = s0.id;
+  cand[1] = s1.id;
+  cand[2] = s2.id;
+  const uint32_t most = max(s0.count, max(s1.count, s2.count));
+  if (most == 0u) return 3;
+  if (s0.count == most)
   {
-    int best = -1;
-    uint32_t bestCount = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (k < n && cand[k] + 1u < L)
-      {
-        const uint32_t c = lrCount[cand[k]];
-        if (best < 0 || c > bestCount)
-        {
-          best = k;
-          bestCount = c;
-        }
-      }
-    if (best < 0) break;
-    uint32_t x = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (k == best) x = cand[k];
-    const uint32_t left = lr[x].leftOffset, right = lr[x].escapeIndex;
-    // slots after `best` move one place right; `best` becomes the two children
-#pragma unroll
-    for (int k = 3; k >= 1; k--)
-      if (k >= best + 2 && k <= n) cand[k] = cand[k - 1];
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-    {
-      if (k == best) cand[k] = left;
-      if (k == best + 1) cand[k] = right;
-    }
-    n++;
+    cand[0] = s0.left;
+    cand[1] = s0.right;
+    cand[2] = s1.id;
+    cand[3] = s2.id;
   }
-  return n;
+  else if (s1.count == most)
+  {
+    cand[1] = s1.left;
+    cand[2] = s1.right;
+    cand[3] = s2.id;
+  }
+  else
+  {
+    cand[2] = s2.left;
+    cand[3] = s2.right;
+  }
+  return 4;
 }
 
-// Appends each lane's `cnt` entries (up to four, in `item`) to a list with one
-// atomic per warp; all 32 lanes call it together.  Entries at or past `cap`
-// are dropped and reported.
-__device__ __forceinline__ void warp_append(const uint32_t (&item)[4], int cnt, uint32_t* __restrict__ list,
-                                            uint32_t* count, uint32_t cap, uint32_t* errorWord)
+// One geometry's tree, or one of a batch's (segment seg): internal node i of
+// it is node intBase + i of the role array.
+struct SegTree
+{
+  const BVHNode32* lr;
+  const uint32_t*  lrCount;
+  const uint32_t*  runStarts;
+  const uint32_t*  parent;
+  TriRec*          tris;
+  uint32_t         L, nTris, intBase, seg;
+};
+
+__device__ __forceinline__ SegTree seg_tree(const Bvh4Batch& b, uint32_t seg)
+{
+  SegTree t;
+  t.seg = seg;
+  t.lr = b.lr + b.nodeOffsets[seg];
+  t.lrCount = b.lrCount + b.nodeOffsets[seg];
+  t.parent = b.parent + b.nodeOffsets[seg];
+  t.runStarts = b.runStarts + b.leafOffsets[seg];
+  t.tris = b.tris + b.triOffsets[seg];
+  t.L = b.leafOffsets[seg + 1] - b.leafOffsets[seg];
+  t.nTris = b.triOffsets[seg + 1] - b.triOffsets[seg];
+  t.intBase = b.intOffsets[seg];
+  return t;
+}
+
+// What the role kernels walk: one tree (params) or a batch's trees.
+struct RoleTrees
+{
+  const BuildParams* params;  // one tree: its leaf count; null for a batch
+  SegTree            one;     // one tree (L from params)
+  Bvh4Batch          batch;
+  const uint32_t*    visit;  // one tree: arrivals at its root in the box refit
+  uint32_t           nInt;  // a batch's internal nodes
+  int                mergeMode;
+};
+
+__device__ __forceinline__ SegTree tree_of(const RoleTrees& r, uint32_t j)
+{
+  if (r.params != nullptr)
+  {
+    SegTree t = r.one;
+    t.L = r.params->nLeaves;
+    return t;
+  }
+  return seg_tree(r.batch, bc::find_segment(r.batch.intOffsets, r.batch.G, j));
+}
+
+// The internal slots of the largest-first 4-wide node of internal node i of
+// `t`: marked as 4-wide nodes (returned, as role-array indices) or merged
+// leaves.  Returns their count.
+__device__ __forceinline__ int mark_slots(const SegTree& t, int mergeMode, uint32_t i, uint8_t* __restrict__ role,
+                                          uint32_t (&next)[4])
+{
+  uint32_t cand[4];
+  const int nc = collapse_slots(t.lr, t.lrCount, t.L, kCollapseLargestFirst, i, cand);
+  int cnt = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+  {
+    if (k >= nc) break;
+    const uint32_t c = cand[k];
+    if (c + 1u >= t.L) continue;  // a leaf slot
+    const bool m = merges(t.lr, t.runStarts, t.L, t.nTris, mergeMode, c);
+    role[t.intBase + c] = m ? 2 : 1;
+    if (!m)
+    {
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (q == cnt) next[q] = t.intBase + c;
+      cnt++;
+    }
+  }
+  return cnt;
+}
+
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v)
 {
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t incl = (uint32_t)cnt;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1)
   {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-    if (lane >= (uint32_t)o) incl += y;
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if (lane >= (uint32_t)o) v += y;
   }
-  const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(count, total);
-  base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - (uint32_t)cnt;
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-    if (k < cnt)
-    {
-      if (base + k < cap)
-        list[base + k] = item[k];
-      else
-        atomicOr(errorWord, kErrLayout);
-    }
+  return v;
 }
 
-// One level of the largest-first roles: every 4-wide node of this level
-// (frontIn) marks its internal slots as 4-wide nodes (appended to frontOut)
-// or merged leaves.  role is zeroed beforehand and the root marked.  The
-// loop runs over warp-uniform bases so that whole warps append together.
-__global__ void __launch_bounds__(kThreads)
-    k_roles_level(const BuildParams* __restrict__ params, const BVHNode32* __restrict__ lr,
-                  const uint32_t* __restrict__ lrCount, const uint32_t* __restrict__ runStarts, uint32_t nTris,
-                  int mergeMode, const uint32_t* __restrict__ frontIn, const uint32_t* __restrict__ countIn,
-                  uint32_t* __restrict__ frontOut, uint32_t* countOut, uint8_t* __restrict__ role, uint32_t* errorWord)
+// A tree of distinct 30-bit codes is at most 31 binary levels deep, and a
+// 4-wide level descends at least one.
+constexpr int kCollapseLevels = 34;
+
+// The top of the largest-first roles, one block: level after level from the
+// roots until the level holds kTopFrontier 4-wide nodes or none.  The last
+// level is left in front[0 or 1]; state = {its size, which}.  role is zeroed
+// beforehand.  A level is a few dependent loads; one SM's loads bound larger ones.
+constexpr uint32_t kTopThreads = 1024, kTopFrontier = 512;
+
+__global__ void __launch_bounds__(kTopThreads)
+    k_roles_top(RoleTrees r, uint32_t* __restrict__ front0, uint32_t* __restrict__ front1, uint32_t* state,
+                uint8_t* __restrict__ role, uint32_t* errorWord)
 {
-  const uint32_t L = params->nLeaves;
-  const uint32_t cap = L > 0 ? L - 1 : 0u;  // internal nodes, each a slot of one 4-wide node at most
-  const uint32_t n = min(*countIn, cap);    // a count past the entries written is an error already reported
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warpBase = (blockIdx.x * kThreads + threadIdx.x) & ~31u;
-  for (uint32_t b0 = warpBase; b0 < n; b0 += gridDim.x * kThreads)
+  __shared__ uint32_t s_count[kCollapseLevels + 2];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  for (uint32_t k = tid; k < kCollapseLevels + 2; k += kTopThreads) s_count[k] = 0u;
+  __syncthreads();
+  uint32_t cap;
+  if (r.params != nullptr)
   {
-    const uint32_t f = b0 + lane;
-    uint32_t next[4] = {0u, 0u, 0u, 0u};
-    int cnt = 0;
-    if (f < n)
+    const uint32_t L = r.params->nLeaves;
+    cap = L > 0 ? L - 1 : 0u;
+    if (tid == 0 && L >= 2)
     {
-      uint32_t cand[4];
-      const int nc = collapse_slots(lr, lrCount, L, kCollapseLargestFirst, frontIn[f], cand);
+      if (r.visit[0] != 2u) atomicOr(errorWord, kErrLayout);
+      role[0] = 1;
+      front0[0] = 0u;
+      s_count[0] = 1u;
+    }
+  }
+  else
+  {
+    cap = r.nInt;
+    for (uint32_t seg = tid; seg < r.batch.G; seg += kTopThreads)
+      if (r.batch.leafOffsets[seg + 1] - r.batch.leafOffsets[seg] >= 2u)
+      {
+        const uint32_t j = r.batch.intOffsets[seg], at = atomicAdd(&s_count[0], 1u);
+        role[j] = 1;
+        if (at < cap) front0[at] = j;
+      }
+  }
+  __syncthreads();
+  int lvl = 0;
+  uint32_t n = min(s_count[0], cap);
+  while (n > 0 && n < kTopFrontier && lvl < kCollapseLevels)
+  {
+    const uint32_t* in = (lvl & 1) ? front1 : front0;
+    uint32_t* out = (lvl & 1) ? front0 : front1;
+    for (uint32_t b0 = tid & ~31u; b0 < n; b0 += kTopThreads)
+    {
+      const uint32_t f = b0 + lane;
+      uint32_t next[4] = {0u, 0u, 0u, 0u};
+      int cnt = 0;
+      if (f < n)
+      {
+        const uint32_t j = in[f];
+        const SegTree t = tree_of(r, j);
+        cnt = mark_slots(t, r.mergeMode, j - t.intBase, role, next);
+      }
+      const uint32_t incl = warp_inclusive((uint32_t)cnt);
+      uint32_t base = 0;
+      if (lane == 31 && incl) base = atomicAdd(&s_count[lvl + 1], incl);
+      base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - (uint32_t)cnt;
 #pragma unroll
       for (int k = 0; k < 4; k++)
-      {
-        if (k >= nc) break;
-        const uint32_t c = cand[k];
-        if (c + 1u >= L) continue;  // a leaf slot
-        const bool m = merges(lr, runStarts, L, nTris, mergeMode, c);
-        role[c] = m ? 2 : 1;
-        if (!m)
-        {
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (j == cnt) next[j] = c;
-          cnt++;
-        }
-      }
+        if (k < cnt && base + k < cap) out[base + k] = next[k];
     }
-    warp_append(next, cnt, frontOut, countOut, cap, errorWord);
+    __syncthreads();  // the level's list (global, this block's own) and count are complete
+    lvl++;
+    n = s_count[lvl];
+    if (n > cap)  // more nodes than the tree has: the links are inconsistent
+    {
+      if (tid == 0) atomicOr(errorWord, kErrLayout);
+      n = cap;
+    }
   }
-}
-
-// The root as the first level (L >= 2), every other level empty.
-__global__ void k_roles_level_init(const BuildParams* __restrict__ params, uint32_t* __restrict__ front,
-                                   uint32_t* __restrict__ counts, int levels, uint8_t* __restrict__ role)
-{
-  const uint32_t L = params->nLeaves;
-  for (int k = threadIdx.x; k <= levels; k += blockDim.x) counts[k] = (k == 0 && L >= 2) ? 1u : 0u;
-  if (threadIdx.x == 0 && L >= 2)
+  if (tid == 0)
   {
-    front[0] = 0;
-    role[0] = 1;
+    state[0] = n;
+    state[1] = (uint32_t)(lvl & 1);
   }
 }
 
-// A frontier left after the last level would mean a tree deeper than the
-// depth bound: reported, never silently cut.
-__global__ void k_roles_level_check(const uint32_t* __restrict__ counts, int levels, uint32_t* errorWord)
-{
-  if (counts[levels] != 0u) atomicOr(errorWord, kErrLayout);
-}
+// The subtrees below the top's last level, a block each: nodes wait on a stack
+// in shared memory, up to a block's threads are taken at a time.  Near the
+// stack's end fewer are taken, down to one: then it grows by at most three a
+// level, for which kSubReserve entries are kept.  (2M-triangle heightfield,
+// 555,081 4-wide nodes: one launch per level with a list in global memory took
+// 34 launches and 106 us of kernels; a top up to 4,096 nodes and a warp per
+// subtree 52 + 33 us, up to 512 nodes 16 + 83; a top up to 512 and a block per subtree 14 + 28 us.)
+constexpr int kSubThreads = 256, kSubStack = 4096, kSubReserve = 3 * kCollapseLevels + 8;
 
-// Depth bound of the largest-first levels: every 4-wide level descends at
-// least one binary level, and a tree of distinct 30-bit codes is at most 31
-// binary levels deep.
-constexpr int kCollapseLevels = 34;
+__global__ void __launch_bounds__(kSubThreads)
+    k_roles_sub(RoleTrees r, const uint32_t* __restrict__ front0, const uint32_t* __restrict__ front1,
+                const uint32_t* __restrict__ state, uint8_t* __restrict__ role, uint32_t* errorWord)
+{
+  __shared__ uint32_t s_stack[kSubStack];
+  __shared__ uint32_t s_size;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  const uint32_t n = state[0];
+  const uint32_t* front = state[1] ? front1 : front0;
+  for (uint32_t f = blockIdx.x; f < n; f += gridDim.x)
+  {
+    const uint32_t root = front[f];
+    const SegTree t = tree_of(r, root);
+    uint32_t size = 1, budget = t.L;  // a consistent subtree has fewer nodes
+    if (tid == 0) s_stack[0] = root;
+    __syncthreads();
+    while (size > 0)
+    {
+      const int room = ((int)kSubStack - kSubReserve - (int)size) / 3;
+      const uint32_t take = min(size, (uint32_t)min(max(room, 1), kSubThreads));
+      if (budget < take)
+      {
+        if (tid == 0) atomicOr(errorWord, kErrLayout);
+        break;
+      }
+      budget -= take;
+      const bool in = tid < take;
+      const uint32_t j = in ? s_stack[size - 1 - tid] : 0u;
+      size -= take;
+      if (tid == 0) s_size = size;
+      uint32_t next[4] = {0u, 0u, 0u, 0u};
+      const int cnt = in ? mark_slots(t, r.mergeMode, j - t.intBase, role, next) : 0;
+      const uint32_t incl = warp_inclusive((uint32_t)cnt);
+      __syncthreads();  // the taken entries are read, s_size is set
+      uint32_t base = 0;
+      if (lane == 31 && incl) base = atomicAdd(&s_size, incl);
+      base = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - (uint32_t)cnt;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (k < cnt && base + k < (uint32_t)kSubStack) s_stack[base + k] = next[k];
+      __syncthreads();
+      size = s_size;
+      if (size > (uint32_t)kSubStack)  // deeper than the depth bound
+      {
+        if (tid == 0) atomicOr(errorWord, kErrLayout);
+        break;
+      }
+      __syncthreads();  // s_size is read
+    }
+    __syncthreads();
+  }
+}
 
 __global__ void __launch_bounds__(kThreads) k_roles(const BuildParams* __restrict__ params,
                                                     const BVHNode32* __restrict__ lr,
@@ -270,29 +423,15 @@ __global__ void __launch_bounds__(kThreads) k_roles(const BuildParams* __restric
 // of each binary node that becomes one, in Karras order (the root gets 0); the
 // prefix is written at every position.  n = L - 1 of params, or nGiven when
 // params is null (the internal nodes of a whole batch, geometry after
-// geometry).  One block per 4096 nodes, decoupled look-back as in the run
+// geometry).  The 4-wide nodes' positions also go to `list`, in order: the
+// emission takes one per lane instead of asking every internal node.  One block per 4096 nodes, decoupled look-back as in the run
 // compaction.
 constexpr int      kScanItems  = 16;
 constexpr uint32_t kScanTile   = kThreads * kScanItems;
-constexpr uint32_t kFlagAgg    = 1u << 30;
-constexpr uint32_t kFlagPrefix = 2u << 30;
-constexpr uint32_t kValueMask  = (1u << 30) - 1u;
-constexpr uint32_t kSpinLimit  = 1u << 22;
-
-__device__ __forceinline__ void store_relaxed(uint32_t* p, uint32_t v)
-{
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t load_relaxed(const uint32_t* p)
-{
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 
 __global__ void __launch_bounds__(kThreads) k_scan_roles(const BuildParams* __restrict__ params, uint32_t nGiven,
                                                          const uint8_t* __restrict__ role, uint32_t* __restrict__ index,
-                                                         uint32_t* tileStatus, uint32_t* tileCounter, uint32_t* total,
+                                                         uint32_t* __restrict__ list, uint32_t* tileStatus, uint32_t* tileCounter, uint32_t* total,
                                                          uint32_t* errorWord)
 {
   __shared__ uint32_t s_tile, s_prefix;
@@ -306,15 +445,21 @@ __global__ void __launch_bounds__(kThreads) k_scan_roles(const BuildParams* __re
   const uint32_t tiles = (n + kScanTile - 1) / kScanTile;
   if (tile >= tiles) return;  // the grid is sized for the worst case
   const uint32_t base = tile * kScanTile + tid * kScanItems;
-  uint32_t flags = 0, cnt = 0;
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++)
+  // a thread's 16 roles are one 128-bit load (the array starts at a 256-byte boundary)
+  uint32_t flags = 0;
+  if (base + kScanItems <= n)
   {
-    const uint32_t i = base + k;
-    const bool f = i < n && role[i] == 1;
-    flags |= (f ? 1u : 0u) << k;
-    cnt += f ? 1u : 0u;
+    const uint4 v = *reinterpret_cast<const uint4*>(role + base);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) flags |= (((w[k >> 2] >> (8 * (k & 3))) & 0xFFu) == 1u ? 1u : 0u) << k;
   }
+  else
+  {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) flags |= (base + k < n && role[base + k] == 1 ? 1u : 0u) << k;
+  }
+  const uint32_t cnt = __popc(flags);
   uint32_t incl = cnt;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1)
@@ -324,58 +469,61 @@ __global__ void __launch_bounds__(kThreads) k_scan_roles(const BuildParams* __re
   }
   if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
-  if (tid == 0)
+  if (warp == 0)
   {
-    uint32_t run = 0;
-    for (int w = 0; w < kThreads / 32; w++)
+    constexpr int kWarps = kThreads / 32;
+    const uint32_t w = lane < kWarps ? s_warp[lane] : 0u;
+    uint32_t run = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
     {
-      const uint32_t t = s_warp[w];
-      s_warp[w] = run;
-      run += t;
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, run, o);
+      if (lane >= o) run += y;
     }
-    uint32_t* my = tileStatus + tile;
-    uint32_t excl = 0;
-    if (tile == 0)
-      store_relaxed(my, kFlagPrefix | run);
-    else
+    const uint32_t sum = __shfl_sync(0xFFFFFFFFu, run, 31);
+    if (lane < kWarps) s_warp[lane] = run - w;
+    const uint32_t excl = bc::warp_look_back(tileStatus, tile, sum, errorWord);
+    if (lane == 0)
     {
-      store_relaxed(my, kFlagAgg | run);
-      int64_t t = (int64_t)tile - 1;
-      uint32_t spins = 0;
-      while (t >= 0)
-      {
-        const uint32_t s = load_relaxed(tileStatus + t);
-        const uint32_t flag = s & ~kValueMask;
-        if (flag == 0u)
-        {
-          if (++spins > kSpinLimit)
-          {
-            atomicOr(errorWord, kErrWaitTimeout);
-            break;
-          }
-          if (spins > 64) __nanosleep(32);
-          continue;
-        }
-        excl += s & kValueMask;
-        if (flag == kFlagPrefix) break;
-        t--;
-      }
-      store_relaxed(my, kFlagPrefix | (excl + run));
+      s_prefix = excl;
+      if (tile == tiles - 1) *total = excl + sum;
     }
-    s_prefix = excl;
-    if (tile == tiles - 1) *total = excl + run;
   }
   __syncthreads();
   uint32_t pos = s_prefix + s_warp[warp] + incl - cnt;
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++)
+  if (base + kScanItems <= n)
   {
-    const uint32_t i = base + k;
-    if (i < n)
+    uint4* o = reinterpret_cast<uint4*>(index + base);
+#pragma unroll
+    for (int q = 0; q < kScanItems / 4; q++)
     {
-      index[i] = pos;
-      pos += (flags >> k) & 1u;
+      uint32_t v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+      {
+        v[k] = pos;
+        if ((flags >> (4 * q + k)) & 1u)
+        {
+          if (pos < n) list[pos] = base + 4 * q + k;
+          pos++;
+        }
+      }
+      o[q] = make_uint4(v[0], v[1], v[2], v[3]);
     }
+  }
+  else
+  {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++)
+      if (base + k < n)
+      {
+        index[base + k] = pos;
+        if ((flags >> k) & 1u)
+        {
+          if (pos < n) list[pos] = base + k;
+          pos++;
+        }
+      }
   }
 }
 
@@ -538,7 +686,7 @@ __device__ __forceinline__ int node4_slots(const BVHNode32* __restrict__ lr, con
   {
     if (k >= nc) break;
     const uint32_t s = cand[k];
-    const BVHNode32 n = lr[s];
+    const BVHNode32 n = bc::load_node(lr + s);
     for (int c = 0; c < 3; c++) { slot[k].lo[c] = n.boxMin[c]; slot[k].hi[c] = n.boxMax[c]; }
     if (s + 1u >= L)
       slot[k].ref = kLeafBit | runStarts[s - (L - 1)];
@@ -571,30 +719,24 @@ __global__ void __launch_bounds__(kThreads) k_emit4(const BuildParams* __restric
                                                     const uint32_t* __restrict__ lrCount,
                                                     const uint32_t* __restrict__ runStarts, uint32_t nTris,
                                                     int collapse, const uint8_t* __restrict__ role,
-                                                    const uint32_t* __restrict__ index, int format,
+                                                    const uint32_t* __restrict__ index,
+                                                    const uint32_t* __restrict__ list, int format,
                                                     void* __restrict__ nodes, uint32_t maxNodes,
                                                     TriRec* __restrict__ tris, uint32_t* errorWord)
 {
   const uint32_t L = params->nLeaves;
-  const uint32_t first = blockIdx.x * kThreads + threadIdx.x;
-  const uint32_t count = (L == 1u) ? 1u : L - 1u;
-  for (uint32_t i = first; i < count; i += gridDim.x * kThreads)
+  for (uint32_t o = blockIdx.x * kThreads + threadIdx.x; o < maxNodes; o += gridDim.x * kThreads)
   {
-    uint32_t outIdx = 0;
-    if (L != 1u)
+    const uint32_t i = L == 1u ? 0u : list[o];
+    if (L != 1u && (i + 1u >= L || role[i] != 1))  // only after a failed numbering (reported through the error word)
     {
-      if (role[i] != 1) continue;
-      outIdx = index[i];
-      if (outIdx >= maxNodes)  // only after a failed numbering (reported through the error word)
-      {
-        atomicOr(errorWord, kErrLayout);
-        continue;
-      }
+      atomicOr(errorWord, kErrLayout);
+      continue;
     }
     Slot slot[4];
     const int ns = node4_slots(lr, lrCount, runStarts, L, nTris, collapse, role, [&](uint32_t c) { return index[c]; },
                                i, tris, slot);
-    write_node4(format, nodes, outIdx, slot, ns, errorWord);
+    write_node4(format, nodes, o, slot, ns, errorWord);
   }
 }
 
@@ -602,31 +744,6 @@ __global__ void __launch_bounds__(kThreads) k_emit4(const BuildParams* __restric
 // The same collapse for the geometries of a segmented build at once: internal
 // node j of the batch is node j - intOffsets[s] of geometry s; each geometry's
 // 4-wide nodes are numbered from 0 (its root) and stored at node4Off[s].
-struct SegTree
-{
-  const BVHNode32* lr;
-  const uint32_t*  lrCount;
-  const uint32_t*  runStarts;
-  const uint32_t*  parent;
-  TriRec*          tris;
-  uint32_t         L, nTris, intBase, seg;
-};
-
-__device__ __forceinline__ SegTree seg_tree(const Bvh4Batch& b, uint32_t seg)
-{
-  SegTree t;
-  t.seg = seg;
-  t.lr = b.lr + b.nodeOffsets[seg];
-  t.lrCount = b.lrCount + b.nodeOffsets[seg];
-  t.parent = b.parent + b.nodeOffsets[seg];
-  t.runStarts = b.runStarts + b.leafOffsets[seg];
-  t.tris = b.tris + b.triOffsets[seg];
-  t.L = b.leafOffsets[seg + 1] - b.leafOffsets[seg];
-  t.nTris = b.triOffsets[seg + 1] - b.triOffsets[seg];
-  t.intBase = b.intOffsets[seg];
-  return t;
-}
-
 __global__ void __launch_bounds__(kThreads) k_seg4_depth_roles(Bvh4Batch b, uint32_t nInt, uint8_t* __restrict__ role)
 {
   for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < nInt; j += gridDim.x * kThreads)
@@ -634,63 +751,6 @@ __global__ void __launch_bounds__(kThreads) k_seg4_depth_roles(Bvh4Batch b, uint
     const SegTree t = seg_tree(b, bc::find_segment(b.intOffsets, b.G, j));
     const uint32_t i = j - t.intBase;
     role[j] = node_role(t.lr, t.runStarts, t.L, t.nTris, node_depth(t.parent, t.L, i), b.mergeMode, i);
-  }
-}
-
-// Largest-first roles of a batch: the geometries' roots as the first level
-// (batch-wide internal node indices), then one launch per level.
-__global__ void __launch_bounds__(kThreads) k_seg4_roles_init(Bvh4Batch b, uint32_t* __restrict__ front,
-                                                              uint32_t* counts, int levels, uint8_t* __restrict__ role)
-{
-  const uint32_t tid = blockIdx.x * kThreads + threadIdx.x;
-  if (tid == 0)
-    for (int k = 1; k <= levels; k++) counts[k] = 0u;
-  for (uint32_t seg = tid; seg < b.G; seg += gridDim.x * kThreads)
-    if (b.leafOffsets[seg + 1] - b.leafOffsets[seg] >= 2u)
-    {
-      const uint32_t j = b.intOffsets[seg];
-      role[j] = 1;
-      front[atomicAdd(counts, 1u)] = j;
-    }
-}
-
-__global__ void __launch_bounds__(kThreads)
-    k_seg4_roles_level(Bvh4Batch b, uint32_t nInt, const uint32_t* __restrict__ frontIn,
-                       const uint32_t* __restrict__ countIn, uint32_t* __restrict__ frontOut, uint32_t* countOut,
-                       uint8_t* __restrict__ role, uint32_t* errorWord)
-{
-  const uint32_t n = min(*countIn, nInt);
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warpBase = (blockIdx.x * kThreads + threadIdx.x) & ~31u;
-  for (uint32_t b0 = warpBase; b0 < n; b0 += gridDim.x * kThreads)
-  {
-    const uint32_t f = b0 + lane;
-    uint32_t next[4] = {0u, 0u, 0u, 0u};
-    int cnt = 0;
-    if (f < n)
-    {
-      const uint32_t j = frontIn[f];
-      const SegTree t = seg_tree(b, bc::find_segment(b.intOffsets, b.G, j));
-      uint32_t cand[4];
-      const int nc = collapse_slots(t.lr, t.lrCount, t.L, kCollapseLargestFirst, j - t.intBase, cand);
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-      {
-        if (k >= nc) break;
-        const uint32_t c = cand[k];
-        if (c + 1u >= t.L) continue;
-        const bool m = merges(t.lr, t.runStarts, t.L, t.nTris, b.mergeMode, c);
-        role[t.intBase + c] = m ? 2 : 1;
-        if (!m)
-        {
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            if (q == cnt) next[q] = t.intBase + c;
-          cnt++;
-        }
-      }
-    }
-    warp_append(next, cnt, frontOut, countOut, nInt, errorWord);
   }
 }
 
@@ -737,26 +797,35 @@ __global__ void __launch_bounds__(1024) k_seg4_counts(Bvh4Batch b, uint32_t nInt
   if (threadIdx.x == 0) node4Off[b.G] = s_carry;
 }
 
-// Threads j < nInt emit the role-1 internal nodes; threads nInt + s emit the
-// lone-leaf node of geometry s when it has exactly one leaf.
+// Threads o < *rankTotal emit the 4-wide nodes of `list`; threads
+// *rankTotal + s emit the lone-leaf node of geometry s when it has exactly one
+// leaf.
 __global__ void __launch_bounds__(kThreads) k_seg4_emit(Bvh4Batch b, uint32_t nInt, const uint8_t* __restrict__ role,
                                                         const uint32_t* __restrict__ rank,
+                                                        const uint32_t* __restrict__ list,
+                                                        const uint32_t* __restrict__ rankTotal,
                                                         const uint32_t* __restrict__ rootRank,
                                                         const uint32_t* __restrict__ node4Off, int format,
                                                         void* __restrict__ nodes, uint32_t* errorWord)
 {
-  for (uint32_t j = blockIdx.x * kThreads + threadIdx.x; j < nInt + b.G; j += gridDim.x * kThreads)
+  const uint32_t n4 = min(*rankTotal, nInt);
+  for (uint32_t o = blockIdx.x * kThreads + threadIdx.x; o < n4 + b.G; o += gridDim.x * kThreads)
   {
-    uint32_t seg, i;
-    if (j < nInt)
+    uint32_t seg, i, j = 0;
+    if (o < n4)
     {
-      if (role[j] != 1) continue;
+      j = list[o];
+      if (j >= nInt || role[j] != 1)
+      {
+        atomicOr(errorWord, kErrLayout);
+        continue;
+      }
       seg = bc::find_segment(b.intOffsets, b.G, j);
       i = j - b.intOffsets[seg];
     }
     else
     {
-      seg = j - nInt;
+      seg = o - n4;
       if (b.leafOffsets[seg + 1] - b.leafOffsets[seg] != 1u) continue;
       i = 0;
     }
@@ -786,39 +855,20 @@ inline uint32_t grid_for(uint64_t n, int numSMs)
   return g == 0 ? 1u : (uint32_t)g;
 }
 
-// Blocks for level `lvl` of the largest-first roles: the level holds at most
-// roots * 4^lvl entries (and never more than the internal nodes); the loop
-// strides over larger levels, so two blocks per SM suffice.
-inline uint32_t level_grid(int lvl, uint64_t roots, uint64_t nInternal, int numSMs)
-{
-  uint64_t most = roots;
-  for (int k = 0; k < lvl && most < nInternal; k++) most *= 4;
-  if (most > nInternal) most = nInternal;
-  uint64_t g = (most + kThreads - 1) / kThreads;
-  const uint64_t cap = (uint64_t)numSMs * 2;
-  if (g > cap) g = cap;
-  return g == 0 ? 1u : (uint32_t)g;
-}
-
 }  // namespace
 
-// Scratch: total (256 B), depth and role (N B each), index (4N B; also the
-// first frontier of the largest-first roles), scan tile status, the second
-// frontier (4N B) and the level counts.
-size_t bvh4_scratch_bytes(uint32_t nTris)
-{
-  const size_t n = nTris ? nTris : 1;
-  const size_t tiles = (n + kScanTile - 1) / kScanTile;
-  return 256 + ((2 * n + 255) / 256) * 256 + ((4 * n + 255) / 256) * 256 + ((4 * (tiles + 8) + 255) / 256) * 256 +
-         ((4 * n + 255) / 256) * 256 + 4 * (kCollapseLevels + 1);
-}
-
+// Scratch: what starts at zero first (total and frontier state, 256 B; scan
+// tile status; roles, N B), then the depths (N B), the node numbering (4N B;
+// also a frontier list of the largest-first roles) and the other list (4N B).
 namespace
 {
+constexpr size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
 struct SingleScratch
 {
-  uint32_t *total, *index, *tiles, *front2, *levelCounts;
-  uint8_t *depth, *role;
+  uint32_t *total, *state, *index, *tiles, *front2;
+  uint8_t  *depth, *role;
+  size_t    zeroBytes, bytes;
 };
 SingleScratch single_scratch(void* scratch, uint32_t N)
 {
@@ -826,48 +876,64 @@ SingleScratch single_scratch(void* scratch, uint32_t N)
   const size_t tiles = (n + kScanTile - 1) / kScanTile;
   char* p = (char*)scratch;
   SingleScratch q;
+  size_t at = 0;
   q.total = (uint32_t*)p;
-  q.depth = (uint8_t*)(p + 256);
-  q.role = q.depth + N;
-  q.index = (uint32_t*)(p + 256 + ((2 * n + 255) / 256) * 256);
-  q.tiles = (uint32_t*)((char*)q.index + ((4 * n + 255) / 256) * 256);
-  q.front2 = (uint32_t*)((char*)q.tiles + ((4 * (tiles + 8) + 255) / 256) * 256);
-  q.levelCounts = (uint32_t*)((char*)q.front2 + ((4 * n + 255) / 256) * 256);
+  q.state = q.total + 1;
+  at += 256;
+  q.tiles = (uint32_t*)(p + at);
+  at += up256(4 * (tiles + 8));
+  q.role = (uint8_t*)(p + at);
+  at += up256(n);
+  q.zeroBytes = at;
+  q.depth = (uint8_t*)(p + at);
+  at += up256(n);
+  q.index = (uint32_t*)(p + at);
+  at += up256(4 * n);
+  q.front2 = (uint32_t*)(p + at);
+  q.bytes = at + up256(4 * n);
   return q;
 }
+
+// The largest-first roles of r's trees (at most nMost internal nodes).
+cudaError_t largest_first_roles(const RoleTrees& r, uint32_t nMost, uint32_t* front0, uint32_t* front1, uint32_t* state,
+                                uint8_t* role, uint32_t* errorWord, int numSMs, cudaStream_t s)
+{
+  k_roles_top<<<1, kTopThreads, 0, s>>>(r, front0, front1, state, role, errorWord);
+  // a block per subtree: the level ends within four times the frontier's size
+  // (a batch's roots may be more)
+  const uint64_t most = std::min<uint64_t>(nMost, std::max<uint64_t>(4 * (uint64_t)kTopFrontier, r.params ? 0u : r.batch.G));
+  const uint64_t blocks = std::min<uint64_t>(most, (uint64_t)numSMs * 8);
+  k_roles_sub<<<(uint32_t)std::max<uint64_t>(blocks, 1), kSubThreads, 0, s>>>(r, front0, front1, state, role, errorWord);
+  return cudaGetLastError();
+}
 }  // namespace
+
+size_t bvh4_scratch_bytes(uint32_t nTris) { return single_scratch(nullptr, nTris).bytes; }
 
 cudaError_t bvh4_plan(const Bvh4Buffers& b, int numSMs, cudaStream_t s)
 {
   const uint32_t N = b.nTris;
   const SingleScratch q = single_scratch(b.scratch, N);
   const size_t nTiles = ((size_t)N + kScanTile - 1) / kScanTile;
-  cudaError_t e = cudaMemsetAsync(q.total, 0, 4, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(q.tiles, 0, 4 * (nTiles + 8), s);
+  cudaError_t e = cudaMemsetAsync(b.scratch, 0, q.zeroBytes, s);
   if (e != cudaSuccess) return e;
   const uint32_t g = grid_for(N, numSMs);
   if (b.collapse == kCollapseLargestFirst)
   {
-    e = cudaMemsetAsync(q.role, 0, N ? N : 1, s);
+    RoleTrees r = {};
+    r.params = b.params;
+    r.one = SegTree{b.lr, b.lrCount, b.runStarts, b.parent, b.tris, 0u, N, 0u, 0u};
+    r.visit = b.visit;
+    r.mergeMode = b.mergeMode;
+    e = largest_first_roles(r, N, q.index, q.front2, q.state, q.role, &b.params->error, numSMs, s);
     if (e != cudaSuccess) return e;
-    k_roles_level_init<<<1, 64, 0, s>>>(b.params, q.index, q.levelCounts, kCollapseLevels, q.role);
-    for (int lvl = 0; lvl < kCollapseLevels; lvl++)
-    {
-      uint32_t* in = (lvl & 1) ? q.front2 : q.index;
-      uint32_t* out = (lvl & 1) ? q.index : q.front2;
-      k_roles_level<<<level_grid(lvl, 1, N, numSMs), kThreads, 0, s>>>(
-          b.params, b.lr, b.lrCount, b.runStarts, N, b.mergeMode, in, q.levelCounts + lvl, out,
-          q.levelCounts + lvl + 1, q.role, &b.params->error);
-    }
-    k_roles_level_check<<<1, 1, 0, s>>>(q.levelCounts, kCollapseLevels, &b.params->error);
   }
   else
   {
-    k_depth<<<g, kThreads, 0, s>>>(b.params, b.parent, q.depth);
+    k_depth<<<g, kThreads, 0, s>>>(b.params, b.parent, b.visit, q.depth);
     k_roles<<<g, kThreads, 0, s>>>(b.params, b.lr, b.runStarts, N, q.depth, b.mergeMode, q.role);
   }
-  k_scan_roles<<<(uint32_t)(nTiles ? nTiles : 1), kThreads, 0, s>>>(b.params, 0u, q.role, q.index, q.tiles + 4,
+  k_scan_roles<<<(uint32_t)(nTiles ? nTiles : 1), kThreads, 0, s>>>(b.params, 0u, q.role, q.index, q.front2, q.tiles + 4,
                                                                       q.tiles, q.total, &b.params->error);
   return cudaMemcpyAsync(b.hostNodeCount, q.total, 4, cudaMemcpyDeviceToHost, s);
 }
@@ -876,29 +942,21 @@ cudaError_t bvh4_emit(const Bvh4Buffers& b, int format, void* nodes, uint32_t ma
 {
   const uint32_t N = b.nTris;
   const SingleScratch q = single_scratch(b.scratch, N);
-  k_emit4<<<grid_for(N, numSMs), kThreads, 0, s>>>(b.params, b.lr, b.lrCount, b.runStarts, N, b.collapse, q.role,
-                                                   q.index, format, nodes, maxNodes, b.tris, &b.params->error);
+  k_emit4<<<grid_for(maxNodes, numSMs), kThreads, 0, s>>>(b.params, b.lr, b.lrCount, b.runStarts, N, b.collapse, q.role,
+                                                   q.index, q.front2, format, nodes, maxNodes, b.tris, &b.params->error);
   return cudaGetLastError();
 }
 
-// Batch scratch: total (256 B), role (nInt B), rank (4 nInt B; also the
-// first frontier of the largest-first roles), per-geometry rootRank, count4,
-// node4Off (4 (3G + 1) B), scan tile status, the second frontier (4 nInt B)
-// and the level counts.
-size_t bvh4_batch_scratch_bytes(uint32_t nInt, uint32_t G)
-{
-  const size_t n = nInt ? nInt : 1;
-  const size_t tiles = (n + kScanTile - 1) / kScanTile;
-  return 256 + ((n + 255) / 256) * 256 + ((4 * n + 255) / 256) * 256 + ((4 * (3 * (size_t)G + 1) + 255) / 256) * 256 +
-         ((4 * (tiles + 8) + 255) / 256) * 256 + ((4 * n + 255) / 256) * 256 + 4 * (kCollapseLevels + 1);
-}
-
+// Batch scratch: what starts at zero first (total and frontier state, scan
+// tile status, roles), then the ranks (4 nInt B; also a frontier list),
+// per-geometry rootRank, count4, node4Off (4 (3G + 1) B) and the other list.
 namespace
 {
 struct BatchScratch
 {
-  uint32_t *total, *rank, *rootRank, *count4, *node4Off, *tiles, *front2, *levelCounts;
-  uint8_t* role;
+  uint32_t *total, *state, *rank, *rootRank, *count4, *node4Off, *tiles, *front2;
+  uint8_t*  role;
+  size_t    zeroBytes, bytes;
 };
 BatchScratch batch_scratch(void* scratch, uint32_t nInt, uint32_t G)
 {
@@ -906,49 +964,50 @@ BatchScratch batch_scratch(void* scratch, uint32_t nInt, uint32_t G)
   const size_t tiles = (n + kScanTile - 1) / kScanTile;
   char* p = (char*)scratch;
   BatchScratch q;
+  size_t at = 0;
   q.total = (uint32_t*)p;
-  q.role = (uint8_t*)(p + 256);
-  q.rank = (uint32_t*)(p + 256 + ((n + 255) / 256) * 256);
-  q.rootRank = (uint32_t*)((char*)q.rank + ((4 * n + 255) / 256) * 256);
+  q.state = q.total + 1;
+  at += 256;
+  q.tiles = (uint32_t*)(p + at);
+  at += up256(4 * (tiles + 8));
+  q.role = (uint8_t*)(p + at);
+  at += up256(n);
+  q.zeroBytes = at;
+  q.rank = (uint32_t*)(p + at);
+  at += up256(4 * n);
+  q.rootRank = (uint32_t*)(p + at);
   q.count4 = q.rootRank + G;
   q.node4Off = q.count4 + G;
-  q.tiles = (uint32_t*)((char*)q.rootRank + ((4 * (3 * (size_t)G + 1) + 255) / 256) * 256);
-  q.front2 = (uint32_t*)((char*)q.tiles + ((4 * (tiles + 8) + 255) / 256) * 256);
-  q.levelCounts = (uint32_t*)((char*)q.front2 + ((4 * n + 255) / 256) * 256);
+  at += up256(4 * (3 * (size_t)G + 1));
+  q.front2 = (uint32_t*)(p + at);
+  q.bytes = at + up256(4 * n);
   return q;
 }
 }  // namespace
+
+size_t bvh4_batch_scratch_bytes(uint32_t nInt, uint32_t G) { return batch_scratch(nullptr, nInt, G).bytes; }
 
 cudaError_t bvh4_plan_batch(const Bvh4Batch& b, uint32_t nInt, void* scratch, uint32_t* hostCount4,
                             uint32_t* hostNode4Off, uint32_t* errorWord, int numSMs, cudaStream_t s)
 {
   const BatchScratch q = batch_scratch(scratch, nInt, b.G);
   const size_t nTiles = ((size_t)(nInt ? nInt : 1) + kScanTile - 1) / kScanTile;
-  cudaError_t e = cudaMemsetAsync(q.total, 0, 4, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(q.tiles, 0, 4 * (nTiles + 8), s);
+  cudaError_t e = cudaMemsetAsync(scratch, 0, q.zeroBytes, s);
   if (e != cudaSuccess) return e;
   if (nInt)
   {
     if (b.collapse == kCollapseLargestFirst)
     {
-      e = cudaMemsetAsync(q.role, 0, nInt, s);
+      RoleTrees r = {};
+      r.batch = b;
+      r.nInt = nInt;
+      r.mergeMode = b.mergeMode;
+      e = largest_first_roles(r, nInt, q.rank, q.front2, q.state, q.role, errorWord, numSMs, s);
       if (e != cudaSuccess) return e;
-      e = cudaMemsetAsync(q.levelCounts, 0, 4, s);
-      if (e != cudaSuccess) return e;
-      k_seg4_roles_init<<<grid_for(b.G, numSMs), kThreads, 0, s>>>(b, q.rank, q.levelCounts, kCollapseLevels, q.role);
-      for (int lvl = 0; lvl < kCollapseLevels; lvl++)
-      {
-        uint32_t* in = (lvl & 1) ? q.front2 : q.rank;
-        uint32_t* out = (lvl & 1) ? q.rank : q.front2;
-        k_seg4_roles_level<<<level_grid(lvl, b.G, nInt, numSMs), kThreads, 0, s>>>(
-            b, nInt, in, q.levelCounts + lvl, out, q.levelCounts + lvl + 1, q.role, errorWord);
-      }
-      k_roles_level_check<<<1, 1, 0, s>>>(q.levelCounts, kCollapseLevels, errorWord);
     }
     else
       k_seg4_depth_roles<<<grid_for(nInt, numSMs), kThreads, 0, s>>>(b, nInt, q.role);
-    k_scan_roles<<<(uint32_t)nTiles, kThreads, 0, s>>>(nullptr, nInt, q.role, q.rank, q.tiles + 4, q.tiles, q.total,
+    k_scan_roles<<<(uint32_t)nTiles, kThreads, 0, s>>>(nullptr, nInt, q.role, q.rank, q.front2, q.tiles + 4, q.tiles, q.total,
                                                        errorWord);
   }
   k_seg4_counts<<<1, 1024, 0, s>>>(b, nInt, q.rank, q.total, q.rootRank, q.count4, q.node4Off);
@@ -961,7 +1020,7 @@ cudaError_t bvh4_emit_batch(const Bvh4Batch& b, uint32_t nInt, void* scratch, in
                             uint32_t* errorWord, int numSMs, cudaStream_t s)
 {
   const BatchScratch q = batch_scratch(scratch, nInt, b.G);
-  k_seg4_emit<<<grid_for((uint64_t)nInt + b.G, numSMs), kThreads, 0, s>>>(b, nInt, q.role, q.rank, q.rootRank,
+  k_seg4_emit<<<grid_for((uint64_t)nInt + b.G, numSMs), kThreads, 0, s>>>(b, nInt, q.role, q.rank, q.front2, q.total, q.rootRank,
                                                                            q.node4Off, format, nodes, errorWord);
   return cudaGetLastError();
 }

@@ -76,6 +76,17 @@ __global__ void k_pack_verts(const uint8_t* __restrict__ raw, uint64_t n, uint64
   }
 }
 
+// Vertices already on the device (stride bytes each, xyz first) to float4 (w = 1).
+int pack_verts(hrt_context* ctx, cudaStream_t st, float4* dst, const uint8_t* raw, uint64_t nVert, uint64_t stride)
+{
+  if (nVert == 0) return HRT_OK;
+  uint64_t blocks = (nVert + 255) / 256;
+  if (blocks > 65535) blocks = 65535;
+  k_pack_verts<<<(uint32_t)blocks, 256, 0, st>>>(raw, nVert, stride, dst);
+  HRT_CUDA(ctx, cudaGetLastError());
+  return HRT_OK;
+}
+
 // Inverse of a column-major 4x4 through the adjugate, in float, the same
 // evaluation as the reference checker's LiteMath stand-in.
 void inverse4x4(const float* mc, float* inv12)
@@ -137,26 +148,24 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   uint64_t* bytes = &g.bytes;
   HRT_CUDA(ctx, dalloc(&g.verts, nVert, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.params, 1, bytes, st));
-  HRT_CUDA(ctx, cudaMemsetAsync(g.params, 0, sizeof(BuildParams), st));
+  uint8_t* raw = nullptr;
   if (nVert)
   {
     if (stride == 16)
       HRT_CUDA(ctx, cudaMemcpyAsync(g.verts, vpos, 16 * nVert, cudaMemcpyDefault, st));
-    uint8_t* raw = nullptr;
-    if (stride != 16)
+    else
     {
       HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
       HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * nVert, cudaMemcpyDefault, st));
     }
-    const uint8_t* src = raw ? raw : reinterpret_cast<const uint8_t*>(g.verts);
-    uint64_t blocks = (nVert + 255) / 256;
-    if (blocks > 65535) blocks = 65535;
-    k_pack_verts<<<(uint32_t)blocks, 256, 0, st>>>(src, nVert, stride, g.verts);
-    HRT_CUDA(ctx, cudaGetLastError());
-    if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
   }
+  const uint8_t* src = raw ? raw : reinterpret_cast<const uint8_t*>(g.verts);
   if (N == 0)
   {
+    HRT_CUDA(ctx, cudaMemsetAsync(g.params, 0, sizeof(BuildParams), st));
+    const int rc = pack_verts(ctx, st, g.verts, src, nVert, stride);
+    if (rc != HRT_OK) return rc;
+    if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
     HRT_CUDA(ctx, cudaStreamSynchronize(st));
     for (int c = 0; c < 4; c++)
     {
@@ -190,6 +199,8 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   HRT_CUDA(ctx, cudaMallocAsync(&scratch, build_scratch_bytes(N), st));
 
   BuildBuffers b;
+  b.raw = src;
+  b.rawStride = stride;
   b.verts = g.verts;
   b.idx = dIdx;
   b.nVerts = g.nVerts;
@@ -232,6 +243,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
     b4.lr = g.lr;
     b4.runStarts = g.runStarts;
     b4.parent = parent;
+    b4.visit = visit;
     b4.tris = g.tris;
     b4.scratch = scratch4;
     b4.mergeMode = s->bvh4Merge;
@@ -252,6 +264,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   }
   HRT_CUDA(ctx, cudaEventRecord(e1, st));
   HRT_CUDA(ctx, cudaMemcpyAsync(&g.host, g.params, sizeof(BuildParams), cudaMemcpyDeviceToHost, st));
+  if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
   HRT_CUDA(ctx, cudaFreeAsync(dIdx, st));
   HRT_CUDA(ctx, cudaFreeAsync(keysAlt, st));
   HRT_CUDA(ctx, cudaFreeAsync(valsAlt, st));
@@ -321,11 +334,8 @@ int build_batch(hrt_scene* s, uint32_t G, const float* vpos, const uint64_t* vOf
       HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * V, st));
       HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * V, cudaMemcpyHostToDevice, st));
     }
-    const uint8_t* src = raw ? raw : reinterpret_cast<const uint8_t*>(verts);
-    uint64_t blocks = (V + 255) / 256;
-    if (blocks > 65535) blocks = 65535;
-    k_pack_verts<<<(uint32_t)blocks, 256, 0, st>>>(src, V, stride, verts);
-    HRT_CUDA(ctx, cudaGetLastError());
+    const int rc = pack_verts(ctx, st, verts, raw ? raw : reinterpret_cast<const uint8_t*>(verts), V, stride);
+    if (rc != HRT_OK) return rc;
     if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
   }
   BatchBuffers b{};
@@ -619,25 +629,6 @@ int build_tlas(hrt_scene* s)
   return HRT_OK;
 }
 
-// Copies nVert host vertices of `stride` bytes (xyz first) to float4 (w = 1) on the device.
-int upload_verts(hrt_context* ctx, cudaStream_t st, float4* dst, const float* vpos, uint64_t nVert, uint64_t stride)
-{
-  if (nVert == 0) return HRT_OK;
-  if (stride == 16) HRT_CUDA(ctx, cudaMemcpyAsync(dst, vpos, 16 * nVert, cudaMemcpyHostToDevice, st));
-  uint8_t* raw = nullptr;
-  if (stride != 16)
-  {
-    HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
-    HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * nVert, cudaMemcpyHostToDevice, st));
-  }
-  uint64_t blocks = (nVert + 255) / 256;
-  if (blocks > 65535) blocks = 65535;
-  k_pack_verts<<<(uint32_t)blocks, 256, 0, st>>>(raw ? raw : reinterpret_cast<const uint8_t*>(dst), nVert, stride, dst);
-  HRT_CUDA(ctx, cudaGetLastError());
-  if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
-  return HRT_OK;
-}
-
 // Refit of geometry g to new vertex positions (same vertex and index counts,
 // same index buffer): the build's tree topology and sorted order are kept,
 // every box, triangle record and traversal record is recomputed, and a 4-wide
@@ -647,10 +638,20 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   hrt_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   const uint32_t N = g.nTris;
-  int rc = upload_verts(ctx, st, g.verts, vpos, g.nVerts, stride);
-  if (rc != HRT_OK) return rc;
+  const uint64_t nVert = g.nVerts;
+  uint8_t* raw = nullptr;
+  if (nVert && stride == 16) HRT_CUDA(ctx, cudaMemcpyAsync(g.verts, vpos, 16 * nVert, cudaMemcpyHostToDevice, st));
+  if (nVert && stride != 16)
+  {
+    HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
+    HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * nVert, cudaMemcpyHostToDevice, st));
+  }
+  const uint8_t* src = raw ? raw : reinterpret_cast<const uint8_t*>(g.verts);
   if (N == 0)
   {
+    const int rc = pack_verts(ctx, st, g.verts, src, nVert, stride);
+    if (rc != HRT_OK) return rc;
+    if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
     HRT_CUDA(ctx, cudaStreamSynchronize(st));
     return HRT_OK;
   }
@@ -662,9 +663,11 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   HRT_CUDA(ctx, cudaMallocAsync((void**)&parent, sizeof(uint32_t) * (2 * (size_t)N - 1), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&visit, sizeof(uint32_t) * 2 * (size_t)N, st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&box, sizeof(BuildParams), st));
-  HRT_CUDA(ctx, cudaMallocAsync(&scratch, refit_scratch_bytes(), st));
+  HRT_CUDA(ctx, cudaMallocAsync(&scratch, refit_scratch_bytes(N), st));
   HRT_CUDA(ctx, cudaMemsetAsync(&g.params->error, 0, sizeof(uint32_t), st));
   BuildBuffers b{};
+  b.raw = src;
+  b.rawStride = stride;
   b.verts = g.verts;
   b.idx = dIdx;
   b.nVerts = g.nVerts;
@@ -700,6 +703,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
     b4.lr = g.lr;
     b4.runStarts = g.runStarts;
     b4.parent = parent;
+    b4.visit = visit;
     b4.tris = g.tris;
     b4.scratch = scratch4;
     b4.mergeMode = g.bvh4Merge;
@@ -717,6 +721,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   BuildParams hb{}, hp{};
   HRT_CUDA(ctx, cudaMemcpyAsync(&hb, box, sizeof(BuildParams), cudaMemcpyDeviceToHost, st));
   HRT_CUDA(ctx, cudaMemcpyAsync(&hp, g.params, sizeof(BuildParams), cudaMemcpyDeviceToHost, st));
+  if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
   HRT_CUDA(ctx, cudaFreeAsync(dIdx, st));
   HRT_CUDA(ctx, cudaFreeAsync(parent, st));
   HRT_CUDA(ctx, cudaFreeAsync(visit, st));

@@ -13,11 +13,13 @@ namespace hrt
 // Stable LSD onesweep radix sort of (key, value) pairs by 32-bit key, four
 // 8-bit digit passes.  keys/vals hold the input and receive the output;
 // keysAlt/valsAlt are ping-pong buffers of n entries.  scratch must hold
-// radix_sort_scratch_bytes(n) bytes; it is cleared by the call.
+// radix_sort_scratch_bytes(n) bytes; it is cleared by the call, unless `counted`:
+// then it was cleared before and its first 4 x 256 words already hold the
+// counts of the keys' four digits.
 constexpr uint32_t kTileSize = 4096;  // pairs per onesweep tile
 size_t radix_sort_scratch_bytes(uint32_t n);
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keysAlt, uint32_t* valsAlt, uint32_t n,
-                             void* scratch, uint32_t* errorWord, int numSMs, cudaStream_t stream);
+                             void* scratch, uint32_t* errorWord, int numSMs, cudaStream_t stream, bool counted = false);
 // Stable sort by (segment, key) where the segment of a pair is the segment of
 // its value in segOffsets[0..segCount] (device, ascending, offsets[0] = 0):
 // each segment ends up sorted by key in place of its input range.
@@ -30,7 +32,9 @@ cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t*
 struct BuildBuffers
 {
   // inputs (device)
-  const float4*   verts;      // nVerts, w = 1
+  const uint8_t*  raw;        // nVerts vertices of rawStride bytes, xyz first (may be verts itself)
+  uint64_t        rawStride;
+  float4*         verts;      // nVerts, packed from raw with w = 1
   const uint32_t* idx;        // 3 * nTris
   uint32_t        nVerts;
   uint32_t        nTris;
@@ -64,7 +68,7 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t stream);
 // b.nTris, b.vals, b.compressed, b.runStarts, b.lr, b.lrCount, b.parent,
 // b.visit, b.recs, b.tris, b.sortedIdx, b.params and b.scratch
 // (refit_scratch_bytes()); the new vertex box is written to boxOut.
-size_t refit_scratch_bytes();
+size_t refit_scratch_bytes(uint32_t nTris);
 cudaError_t refit_lbvh(const BuildBuffers& b, BuildParams* boxOut, int numSMs, cudaStream_t stream);
 
 // ---------------------------------------------------------------- build_batch.cu
@@ -129,6 +133,7 @@ struct Bvh4Buffers
   const uint32_t*  parent;          // 2L-1
   TriRec*          tris;            // N; bit 1 of a.w marks 4-wide leaf ends
   const uint32_t*  lrCount;         // 2L-1 descendant node counts (the largest-first collapse opens by them)
+  const uint32_t*  visit;           // [0]: arrivals at the root of the box refit (2: it is done)
   int              mergeMode;       // 0: merge two leaf children (reference rule); M > 0: merge subtrees of <= M triangles
   int              collapse;        // HRT_BVH4_COLLAPSE_*
   void*            scratch;         // bvh4_scratch_bytes(nTris)

@@ -4,7 +4,8 @@
 // with a stable GPU sort (Adinets & Merrill, "Onesweep: A Faster Least
 // Significant Digit Radix Sort for GPUs", 2022):
 //   1. one histogram pass counts all four 8-bit digits of every key;
-//   2. a one-block kernel turns the four histograms into exclusive digit bases;
+//   2. every block of a pass turns the pass's histogram into exclusive digit
+//      bases itself (256 values; a launch of its own took 3 us);
 //   3. four digit passes, each ONE kernel: a tile of 4096 pairs is ranked in
 //      shared memory (warp-level __match_any_sync ranking, stable), the tile's
 //      per-digit counts are published and the exclusive prefix over earlier
@@ -54,10 +55,11 @@ __device__ __forceinline__ uint32_t load_relaxed(const uint32_t* p)
 // passes of the segmented sort - a byte of the index of the segment that holds
 // the element's value (ascending offsets[0..segCount]; value = global
 // triangle index).
+template <bool SEG>
 __device__ __forceinline__ uint32_t pass_digit(uint32_t key, uint32_t val, uint32_t shift,
                                                const uint32_t* __restrict__ segOffsets, uint32_t segCount)
 {
-  if (segOffsets == nullptr) return (key >> shift) & 0xFFu;
+  if (!SEG) return (key >> shift) & 0xFFu;
   return (bc::find_segment(segOffsets, segCount, val) >> shift) & 0xFFu;
 }
 
@@ -124,22 +126,11 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* w
   return r;
 }
 
-__global__ void __launch_bounds__(kThreads) k_scan_histograms(uint32_t* __restrict__ hist, int nHist)
-{
-  __shared__ uint32_t warpSums[kWarps + 1];
-  for (int p = 0; p < nHist; p++)
-  {
-    uint32_t total;
-    const uint32_t v = hist[p * kRadix + threadIdx.x];
-    const uint32_t e = block_exclusive_scan(v, warpSums, &total);
-    hist[p * kRadix + threadIdx.x] = e;
-  }
-}
-
+template <bool SEG>
 __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __restrict__ keysIn,
                                                        const uint32_t* __restrict__ valsIn,
                                                        uint32_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut,
-                                                       uint32_t n, uint32_t shift, const uint32_t* __restrict__ digitBase,
+                                                       uint32_t n, uint32_t shift, const uint32_t* __restrict__ hist,
                                                        uint32_t* tileStatus, uint32_t* tileCounter, uint32_t* errorWord,
                                                        const uint32_t* __restrict__ segOffsets, uint32_t segCount)
 {
@@ -161,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
 
   // Warp-striped load: item k of lane l is element warpBase + 32k + l, so the
   // (warp, k, lane) order is the input order and the ranking below is stable.
-  uint32_t key[kItems], val[kItems], rank[kItems];
+  uint32_t key[kItems], val[kItems], rank[kItems / 2];  // two 16-bit ranks a word
 #pragma unroll
   for (int k = 0; k < kItems; k++)
   {
@@ -175,10 +166,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
   for (int k = 0; k < kItems; k++)
   {
     const bool valid = (warpBase + k * 32 + lane) < n;
-    const uint32_t digit = valid ? pass_digit(key[k], val[k], shift, segOffsets, segCount) : 0xFFu;
+    const uint32_t digit = valid ? pass_digit<SEG>(key[k], val[k], shift, segOffsets, segCount) : 0xFFu;
+    // (eight ballots and selects instead of the match took 43 us a pass against
+    // 22: a mesh's neighbours share digits, which the match is quick on)
     const uint32_t peers = __match_any_sync(0xFFFFFFFFu, valid ? digit : (0x100u + lane));
     const uint32_t before = s_warpHist[warp][digit];
-    rank[k] = before + __popc(peers & ltMask);
+    const uint32_t r = before + __popc(peers & ltMask);
+    rank[k / 2] = (k & 1) ? rank[k / 2] | (r << 16) : r;
     __syncwarp();
     if (valid && lane == __ffs(peers) - 1) s_warpHist[warp][digit] = before + __popc(peers);
     __syncwarp();
@@ -199,17 +193,40 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
   store_relaxed(myStatus, (tile == 0 ? kFlagPrefix : kFlagAgg) | total);
   uint32_t blockTotal;
   s_digitStart[d] = block_exclusive_scan(total, s_warpSums, &blockTotal);
+  const uint32_t digitBase = block_exclusive_scan(hist[d], s_warpSums, &blockTotal);
 
+  // Look back eight tiles a time (their words are independent loads): tiles
+  // start together, so a tile first meets sums and only then a prefix, and one
+  // load's latency per tile adds up (2M pairs: 24.5 us a pass, now 21).
   uint32_t excl = 0;
   if (tile > 0)
   {
-    int64_t t = (int64_t)tile - 1;
+    constexpr int kBack = 8;
+    int t = (int)tile - 1;
     uint32_t spins = 0;
-    while (t >= 0)
+    bool done = false;
+    while (!done)
     {
-      const uint32_t s = load_relaxed(tileStatus + (size_t)t * kRadix + d);
-      const uint32_t flag = s & ~kValueMask;
-      if (flag == 0u)
+      uint32_t w[kBack];
+      const uint32_t* at = tileStatus + (size_t)t * kRadix + d;  // read where t - q >= 0
+#pragma unroll
+      for (int q = 0; q < kBack; q++) w[q] = t - q >= 0 ? load_relaxed(at - q * kRadix) : kFlagPrefix;
+      int used = 0;
+      bool open = true;
+#pragma unroll
+      for (int q = 0; q < kBack; q++)
+      {
+        const uint32_t flag = w[q] & ~kValueMask;
+        open = open && !done && flag != 0u;
+        if (open)
+        {
+          excl += w[q] & kValueMask;
+          used++;
+          done = flag == kFlagPrefix;
+        }
+      }
+      t -= used;
+      if (used == 0)
       {
         if (++spins > kSpinLimit)
         {
@@ -217,15 +234,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
           break;
         }
         if (spins > 64) __nanosleep(32);
-        continue;
       }
-      excl += s & kValueMask;
-      if (flag == kFlagPrefix) break;
-      t--;
     }
     store_relaxed(myStatus, kFlagPrefix | (excl + total));
   }
-  s_dst[d] = digitBase[d] + excl - s_digitStart[d];
+  s_dst[d] = digitBase + excl - s_digitStart[d];
   __syncthreads();
 
 #pragma unroll
@@ -233,8 +246,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
   {
     if ((warpBase + k * 32 + lane) < n)
     {
-      const uint32_t digit = pass_digit(key[k], val[k], shift, segOffsets, segCount);
-      const uint32_t pos = s_digitStart[digit] + s_warpHist[warp][digit] + rank[k];
+      const uint32_t digit = pass_digit<SEG>(key[k], val[k], shift, segOffsets, segCount);
+      const uint32_t pos = s_digitStart[digit] + s_warpHist[warp][digit] + ((rank[k / 2] >> (16 * (k & 1))) & 0xFFFFu);
       s_keys[pos] = key[k];
       s_vals[pos] = val[k];
     }
@@ -245,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep(const uint32_t* __rest
   for (uint32_t i = tid; i < count; i += kThreads)
   {
     const uint32_t k = s_keys[i];
-    const uint32_t dst = s_dst[pass_digit(k, s_vals[i], shift, segOffsets, segCount)] + i;
+    const uint32_t dst = s_dst[pass_digit<SEG>(k, s_vals[i], shift, segOffsets, segCount)] + i;
     if (dst < n)  // always true unless a look-back wait gave up (reported through errorWord)
     {
       keysOut[dst] = k;
@@ -267,27 +280,29 @@ constexpr size_t sort_scratch_bytes(size_t n)
 size_t radix_sort_scratch_bytes(uint32_t n) { return sort_scratch_bytes(n); }
 
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keysAlt, uint32_t* valsAlt, uint32_t n,
-                             void* scratch, uint32_t* errorWord, int numSMs, cudaStream_t stream)
+                             void* scratch, uint32_t* errorWord, int numSMs, cudaStream_t stream, bool counted)
 {
   if (n <= 1) return cudaSuccess;
   const uint32_t tiles = (n + kTile - 1) / kTile;
   uint32_t* hist = (uint32_t*)scratch;
   uint32_t* counters = hist + kPasses * kRadix;
   uint32_t* status = counters + kPasses + 4;
-  cudaError_t e = cudaMemsetAsync(scratch, 0, radix_sort_scratch_bytes(n), stream);
-  if (e != cudaSuccess) return e;
-  uint32_t hb = (n + kThreads - 1) / kThreads;
-  const uint32_t maxHb = (uint32_t)numSMs * 4u;
-  if (hb > maxHb) hb = maxHb;
-  k_histogram<<<hb, kThreads, 0, stream>>>(keys, n, hist);
-  k_scan_histograms<<<1, kThreads, 0, stream>>>(hist, kPasses);
+  if (!counted)
+  {
+    cudaError_t e = cudaMemsetAsync(scratch, 0, radix_sort_scratch_bytes(n), stream);
+    if (e != cudaSuccess) return e;
+    uint32_t hb = (n + kThreads - 1) / kThreads;
+    const uint32_t maxHb = (uint32_t)numSMs * 4u;
+    if (hb > maxHb) hb = maxHb;
+    k_histogram<<<hb, kThreads, 0, stream>>>(keys, n, hist);
+  }
   uint32_t* srcK = keys;
   uint32_t* srcV = vals;
   uint32_t* dstK = keysAlt;
   uint32_t* dstV = valsAlt;
   for (int p = 0; p < kPasses; p++)
   {
-    k_onesweep<<<tiles, kThreads, 0, stream>>>(srcK, srcV, dstK, dstV, n, 8u * p, hist + p * kRadix,
+    k_onesweep<false><<<tiles, kThreads, 0, stream>>>(srcK, srcV, dstK, dstV, n, 8u * p, hist + p * kRadix,
                                                status + (size_t)p * tiles * kRadix, counters + p, errorWord, nullptr, 0u);
     uint32_t* t = srcK; srcK = dstK; dstK = t;
     t = srcV; srcV = dstV; dstV = t;
@@ -330,7 +345,6 @@ cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t*
   for (int q = 0; q < segPasses; q++)
     k_segment_histogram<<<(segCount + 255) / 256, 256, 0, stream>>>(segOffsets, segCount, 8u * q,
                                                                      hist + (kPasses + q) * kRadix);
-  k_scan_histograms<<<1, kThreads, 0, stream>>>(hist, passes);
   uint32_t* srcK = keys;
   uint32_t* srcV = vals;
   uint32_t* dstK = keysAlt;
@@ -340,9 +354,10 @@ cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t*
   for (int p = 0; p < passes; p++)
   {
     const bool seg = p >= kPasses;
-    k_onesweep<<<tiles, kThreads, 0, stream>>>(srcK, srcV, dstK, dstV, n, seg ? 8u * (p - kPasses) : 8u * p,
-                                               hist + p * kRadix, status + (size_t)p * tiles * kRadix, counters + p,
-                                               errorWord, seg ? segOffsets : nullptr, segCount);
+    auto pass = seg ? k_onesweep<true> : k_onesweep<false>;
+    pass<<<tiles, kThreads, 0, stream>>>(srcK, srcV, dstK, dstV, n, seg ? 8u * (p - kPasses) : 8u * p,
+                                         hist + p * kRadix, status + (size_t)p * tiles * kRadix, counters + p,
+                                         errorWord, segOffsets, segCount);
     uint32_t* t = srcK; srcK = dstK; dstK = t;
     t = srcV; srcV = dstV; dstV = t;
   }
