@@ -3,6 +3,8 @@
 // records.  Every stage reproduces the integer and float results of HeavyRT's
 // LBVHBuilder (core/builders/lbvh.cpp) bit for bit; float arithmetic is written
 // with explicit round-to-nearest intrinsics so that no multiply-add is fused.
+#include <algorithm>
+
 #include "build_common.cuh"
 #include "hrt_kernels.cuh"
 #include "leaf_tree.cuh"
@@ -15,30 +17,87 @@ namespace
 constexpr int kThreads = 256;
 
 // ---------------------------------------------------------------- vertices and scene box
-// The vertices packed to float4 (w = 1), and in the same pass their box and the
-// Morton scale (kernel1D_RedunctionFromVertices, core/builders/lbvh.cpp:228-239;
+// The build's inputs read once: the indices copied, the vertices packed to
+// float4 (w = 1), and in the same pass their box and the Morton scale
+// (kernel1D_RedunctionFromVertices, core/builders/lbvh.cpp:228-239;
 // ZIndexMultCoeff on the box widened by 1e-4, :41-51,263): each block leaves its
 // part's bounds, the last block to finish (counted in *done, zero before)
 // combines them.  min/max are exact, so only the sign of a zero bound can
 // depend on the order; it never reaches a Morton code (+0 and -0 give the same
 // quantised offset).  `reset` also clears the build's counters in params.
-// Three launches before (pack, parts, final): 12 us of a 2M-triangle build.
+//
+// The sources may be host memory read over the host link (page-locked, or
+// pageable where the GPU translates through the host's page tables): reads are
+// whole lines, tightly packed vertices by way of shared memory.  Bound by the
+// link: 38 MB of numpy arrays in 186 us (205 GB/s); copied to the device first
+// 210 + 10 us, and the load 890 us instead of 824.
+constexpr uint32_t kPackTile = 4 * kThreads;  // vertices of a block's step (12-byte stride)
+
 __global__ void __launch_bounds__(kThreads)
-    k_pack_box(const uint8_t* raw, uint64_t stride, uint32_t n, float4* out, float4* partial,
-               uint32_t* done, BuildParams* params, int cubic, int reset)
+    k_read_inputs(const uint8_t* raw, uint64_t stride, uint32_t n, float4* out, const uint32_t* idxSrc, uint32_t* idx,
+                  uint64_t nIdx, float4* partial, uint32_t* done, BuildParams* params, int cubic, int reset)
 {
   float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
-  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
-  {
-    const float* p = reinterpret_cast<const float*>(raw + (size_t)i * stride);
-    const float v[4] = {p[0], p[1], p[2], 1.0f};
-    out[i] = make_float4(v[0], v[1], v[2], 1.0f);
+  auto take = [&](uint32_t i, float x, float y, float z) {
+    const float v[4] = {x, y, z, 1.0f};
+    out[i] = make_float4(x, y, z, 1.0f);
 #pragma unroll
     for (int k = 0; k < 4; k++)
     {
       mn[k] = lm_min(mn[k], v[k]);
       mx[k] = lm_max(mx[k], v[k]);
     }
+  };
+  const bool aligned = (reinterpret_cast<uintptr_t>(raw) & 15u) == 0u;
+  if (stride == 12 && aligned)
+  {
+    __shared__ float4 s_raw[3 * kThreads];
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kPackTile; v0 < n; v0 += (uint64_t)gridDim.x * kPackTile)
+    {
+      const uint32_t count = (uint32_t)min((uint64_t)kPackTile, n - v0);
+      const uint32_t pieces = 3 * count / 4;  // whole 16-byte pieces
+      const float4* src = reinterpret_cast<const float4*>(raw + 12 * v0);
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+      {
+        const uint32_t k = q * kThreads + threadIdx.x;
+        if (k < pieces) s_raw[k] = src[k];
+      }
+      float* words = reinterpret_cast<float*>(s_raw);
+      if (threadIdx.x < 3 * count - 4 * pieces)
+        words[4 * pieces + threadIdx.x] = reinterpret_cast<const float*>(src)[4 * pieces + threadIdx.x];
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+      {
+        const uint32_t k = q * kThreads + threadIdx.x;
+        if (k < count) take((uint32_t)(v0 + k), words[3 * k], words[3 * k + 1], words[3 * k + 2]);
+      }
+      __syncthreads();
+    }
+  }
+  else if (stride == 16 && aligned)
+  {
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+    {
+      const float4 p = reinterpret_cast<const float4*>(raw)[i];
+      take(i, p.x, p.y, p.z);
+    }
+  }
+  else
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+    {
+      const float* p = reinterpret_cast<const float*>(raw + (size_t)i * stride);
+      take(i, p[0], p[1], p[2]);
+    }
+  if (idxSrc != idx)
+  {
+    const uint64_t step = (uint64_t)gridDim.x * kThreads, first = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    const uint64_t whole = (reinterpret_cast<uintptr_t>(idxSrc) & 15u) == 0u ? nIdx / 4 : 0;  // idx starts an allocation
+#pragma unroll 4
+    for (uint64_t k = first; k < whole; k += step)
+      reinterpret_cast<uint4*>(idx)[k] = reinterpret_cast<const uint4*>(idxSrc)[k];
+    for (uint64_t k = 4 * whole + first; k < nIdx; k += step) idx[k] = idxSrc[k];
   }
   __shared__ float smn[kThreads / 32][4], smx[kThreads / 32][4];
   __shared__ bool  s_last;
@@ -258,7 +317,7 @@ inline uint32_t grid_for(uint64_t n, int numSMs, int perSM = 8)
 namespace
 {
 constexpr size_t up256(size_t b) { return (b + 255) / 256 * 256; }
-constexpr uint32_t kBoxBlocks = 1024;  // most blocks of k_pack_box
+constexpr uint32_t kBoxBlocks = 1024;  // most blocks of k_read_inputs
 
 // Build scratch: what starts at zero first (box and scan counters, scan tile
 // status, the sort's scratch), then the box parts.
@@ -287,10 +346,15 @@ BuildScratch build_scratch(void* scratch, uint32_t nTris)
   return q;
 }
 
-uint32_t box_blocks(uint32_t nVerts, int numSMs)
+cudaError_t read_inputs(const BuildBuffers& b, float4* partial, uint32_t* done, BuildParams* params, int reset,
+                        int numSMs, cudaStream_t s)
 {
-  const uint32_t g = grid_for(nVerts, numSMs, 4);
-  return g > kBoxBlocks ? kBoxBlocks : g;
+  const uint64_t nIdx = 3 * (uint64_t)b.nTris;
+  uint32_t g = grid_for(std::max<uint64_t>(b.nVerts, nIdx / 4), numSMs, 4);
+  if (g > kBoxBlocks) g = kBoxBlocks;
+  k_read_inputs<<<g, kThreads, 0, s>>>(b.raw, b.rawStride, b.nVerts, b.verts, b.idxSrc, b.idx, nIdx, partial, done,
+                                       params, b.mortonCubic, reset);
+  return cudaGetLastError();
 }
 
 // Leaves, hierarchy, boxes and (binary layout) pair records, from the sorted
@@ -337,9 +401,9 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   uint32_t* err = &b.params->error;
   cudaError_t e = cudaMemsetAsync(b.scratch, 0, q.zeroBytes, s);
   if (e != cudaSuccess) return e;
-  // 1. vertices, scene box and Morton scale
-  k_pack_box<<<box_blocks(b.nVerts, numSMs), kThreads, 0, s>>>(b.raw, b.rawStride, b.nVerts, b.verts, q.partial,
-                                                               q.boxDone, b.params, b.mortonCubic, 1);
+  // 1. inputs, scene box and Morton scale
+  e = read_inputs(b, q.partial, q.boxDone, b.params, 1, numSMs, s);
+  if (e != cudaSuccess) return e;
   // 2. Morton codes and their digits' counts
   constexpr uint32_t kPerBlock = kThreads * kMortonItems;
   k_morton<<<(N + kPerBlock - 1) / kPerBlock, kThreads, 0, s>>>(b.verts, b.idx, N, b.nVerts, b.params, b.keys,
@@ -366,10 +430,9 @@ cudaError_t refit_lbvh(const BuildBuffers& b, BuildParams* boxOut, int numSMs, c
   uint32_t* done = (uint32_t*)b.scratch;  // refit_scratch_bytes(): counters, box parts, open walks
   float4* partial = (float4*)((char*)b.scratch + 256);
   uint32_t* open = (uint32_t*)(partial + 2 * kBoxBlocks);
-  const cudaError_t e = cudaMemsetAsync(done, 0, 2 * sizeof(uint32_t), s);
+  cudaError_t e = cudaMemsetAsync(done, 0, 2 * sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = read_inputs(b, partial, done, boxOut, 0, numSMs, s);
   if (e != cudaSuccess) return e;
-  k_pack_box<<<box_blocks(b.nVerts, numSMs), kThreads, 0, s>>>(b.raw, b.rawStride, b.nVerts, b.verts, partial, done,
-                                                               boxOut, b.mortonCubic, 0);
   return build_tree(b, open, done + 1, numSMs, s);
 }
 

@@ -23,30 +23,90 @@ namespace
 constexpr int kThreads = 256;
 using bc::find_segment;
 
-// Scene box and Morton scale of each geometry, in two passes: every geometry's
-// vertices in chunks of kBoxChunk, one block per chunk (geometry s owns chunks
-// [chunkOffsets[s], chunkOffsets[s + 1])), then the chunks of each geometry
-// combined in order.  Min / max are exact, so the box is the reference's
-// (core/builders/lbvh.cpp:228-239; init +-1e10, :53).
-constexpr uint32_t kBoxChunk = kBatchBoxChunk;
-
-__global__ void __launch_bounds__(kThreads) k_seg_box_partial(const float4* __restrict__ v,
-                                                              const uint32_t* __restrict__ vertOffsets,
-                                                              const uint32_t* __restrict__ chunkOffsets, uint32_t G,
-                                                              float4* __restrict__ partial)
+// The inputs of all geometries read once, a block per chunk: vertices packed to
+// float4 (w = 1) with the chunk's bounds (geometry s owns chunks
+// [boxChunkOffsets[s], boxChunkOffsets[s + 1])), and indices copied.  The sources
+// are the caller's arrays, one per geometry, wherever the kernel reaches them:
+// reads over the host link are whole lines, tightly packed vertices by way of
+// shared memory (as k_read_inputs in build.cu).  Min / max are exact, so the box
+// is the reference's (core/builders/lbvh.cpp:228-239; init +-1e10, :53).
+// 48 soups, 26 MB: copied by the host into one array and to the device 1,550 us,
+// so 130 us.
+__global__ void __launch_bounds__(kThreads) k_seg_read_inputs(BatchBuffers b)
 {
-  const uint32_t k = blockIdx.x;
-  const uint32_t s = find_segment(chunkOffsets, G, k);
-  const uint32_t c = k - chunkOffsets[s];
-  const uint32_t b = vertOffsets[s] + c * kBoxChunk;
-  const uint32_t e = min(b + kBoxChunk, vertOffsets[s + 1]);
-  float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
-  for (uint32_t i = b + threadIdx.x; i < e; i += kThreads)
+  if (blockIdx.x >= b.nBoxChunks)
   {
-    const float4 p = v[i];
-    mn[0] = lm_min(mn[0], p.x); mn[1] = lm_min(mn[1], p.y); mn[2] = lm_min(mn[2], p.z); mn[3] = lm_min(mn[3], p.w);
-    mx[0] = lm_max(mx[0], p.x); mx[1] = lm_max(mx[1], p.y); mx[2] = lm_max(mx[2], p.z); mx[3] = lm_max(mx[3], p.w);
+    const uint32_t k = blockIdx.x - b.nBoxChunks;
+    const uint32_t s = find_segment(b.idxChunkOffsets, b.G, k);
+    const uint32_t first = (k - b.idxChunkOffsets[s]) * kBatchIdxChunk, t0 = b.triOffsets[s];
+    const uint32_t n = 3u * (b.triOffsets[s + 1] - t0);  // at most 3 * 2^24 words
+    const uint32_t end = min(first + kBatchIdxChunk, n);
+    const uint32_t* src = b.rawIdx[s];
+    uint32_t* dst = b.idx + 3 * (size_t)t0;
+    uint32_t at = first;
+    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0u)
+    {
+      const uint32_t pieces = (end - first) / 4;
+#pragma unroll 4
+      for (uint32_t q = threadIdx.x; q < pieces; q += kThreads)
+      {
+        const uint4 v = reinterpret_cast<const uint4*>(src + first)[q];
+        uint32_t* o = dst + first + 4 * q;
+        o[0] = v.x;
+        o[1] = v.y;
+        o[2] = v.z;
+        o[3] = v.w;
+      }
+      at = first + 4 * pieces;
+    }
+    for (uint32_t i = at + threadIdx.x; i < end; i += kThreads) dst[i] = src[i];
+    return;
   }
+  const uint32_t k = blockIdx.x;
+  const uint32_t s = find_segment(b.boxChunkOffsets, b.G, k);
+  const uint32_t v0 = b.vertOffsets[s], first = (k - b.boxChunkOffsets[s]) * kBatchBoxChunk;
+  const uint32_t end = min(first + kBatchBoxChunk, b.vertOffsets[s + 1] - v0);
+  const uint8_t* raw = b.rawVerts[s] + (size_t)first * b.rawStride;  // first vertex of the chunk
+  float4* out = b.verts + (size_t)v0 + first;
+  const uint32_t n = end - first;
+  float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
+  auto take = [&](uint32_t i, float x, float y, float z) {
+    const float v[4] = {x, y, z, 1.0f};
+    out[i] = make_float4(x, y, z, 1.0f);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+      mn[q] = lm_min(mn[q], v[q]);
+      mx[q] = lm_max(mx[q], v[q]);
+    }
+  };
+  const bool aligned = (reinterpret_cast<uintptr_t>(raw) & 15u) == 0u;
+  if (b.rawStride == 12 && aligned)
+  {
+    __shared__ float s_raw[3 * kBatchBoxChunk];
+    const uint32_t pieces = 3 * n / 4;  // whole 16-byte pieces
+#pragma unroll 6
+    for (uint32_t q = threadIdx.x; q < pieces; q += kThreads)
+      reinterpret_cast<float4*>(s_raw)[q] = reinterpret_cast<const float4*>(raw)[q];
+    for (uint32_t q = 4 * pieces + threadIdx.x; q < 3 * n; q += kThreads) s_raw[q] = reinterpret_cast<const float*>(raw)[q];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads) take(i, s_raw[3 * i], s_raw[3 * i + 1], s_raw[3 * i + 2]);
+  }
+  else if (b.rawStride == 16 && aligned)
+  {
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads)
+    {
+      const float4 p = reinterpret_cast<const float4*>(raw)[i];
+      take(i, p.x, p.y, p.z);
+    }
+  }
+  else
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads)
+    {
+      const float* p = reinterpret_cast<const float*>(raw + (size_t)i * b.rawStride);
+      take(i, p[0], p[1], p[2]);
+    }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -64,27 +124,40 @@ __global__ void __launch_bounds__(kThreads) k_seg_box_partial(const float4* __re
   {
     for (int w = 1; w < kThreads / 32; w++)
       for (int q = 0; q < 4; q++) { mn[q] = lm_min(mn[q], smn[w][q]); mx[q] = lm_max(mx[q], smx[w][q]); }
-    partial[2 * k] = make_float4(mn[0], mn[1], mn[2], mn[3]);
-    partial[2 * k + 1] = make_float4(mx[0], mx[1], mx[2], mx[3]);
+    b.boxPartial[2 * k] = make_float4(mn[0], mn[1], mn[2], mn[3]);
+    b.boxPartial[2 * k + 1] = make_float4(mx[0], mx[1], mx[2], mx[3]);
   }
 }
 
+// The chunks of each geometry combined, a warp each.
 __global__ void __launch_bounds__(kThreads) k_seg_box_final(const uint32_t* __restrict__ chunkOffsets, uint32_t G,
                                                             const float4* __restrict__ partial, BuildParams* params,
                                                             int cubic)
 {
-  for (uint32_t s = blockIdx.x * kThreads + threadIdx.x; s < G; s += gridDim.x * kThreads)
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t s = (blockIdx.x * kThreads + threadIdx.x) >> 5; s < G; s += (gridDim.x * kThreads) >> 5)
   {
     float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
-    for (uint32_t k = chunkOffsets[s]; k < chunkOffsets[s + 1]; k++)
+    for (uint32_t k = chunkOffsets[s] + lane; k < chunkOffsets[s + 1]; k += 32)
     {
-      const float4 a = partial[2 * k], b = partial[2 * k + 1];
+      const float4 a = partial[2 * k], c = partial[2 * k + 1];
       mn[0] = lm_min(mn[0], a.x); mn[1] = lm_min(mn[1], a.y); mn[2] = lm_min(mn[2], a.z); mn[3] = lm_min(mn[3], a.w);
-      mx[0] = lm_max(mx[0], b.x); mx[1] = lm_max(mx[1], b.y); mx[2] = lm_max(mx[2], b.z); mx[3] = lm_max(mx[3], b.w);
+      mx[0] = lm_max(mx[0], c.x); mx[1] = lm_max(mx[1], c.y); mx[2] = lm_max(mx[2], c.z); mx[3] = lm_max(mx[3], c.w);
     }
-    bc::zindex_scale(mn, mx, &params[s], cubic);
-    params[s].nLeaves = 0;
-    params[s].error = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+      {
+        mn[q] = lm_min(mn[q], __shfl_down_sync(0xFFFFFFFFu, mn[q], o));
+        mx[q] = lm_max(mx[q], __shfl_down_sync(0xFFFFFFFFu, mx[q], o));
+      }
+    if (lane == 0)
+    {
+      bc::zindex_scale(mn, mx, &params[s], cubic);
+      params[s].nLeaves = 0;
+      params[s].error = 0;
+    }
   }
 }
 
@@ -334,10 +407,9 @@ cudaError_t build_lbvh_batch(const BatchBuffers& b, int numSMs, cudaStream_t s)
   uint32_t* scanStatus = scanCounter + 4;
   void* sortScratch = scratch + scanBytes;
 
-  if (b.nBoxChunks) k_seg_box_partial<<<b.nBoxChunks, kThreads, 0, s>>>(b.verts, b.vertOffsets, b.boxChunkOffsets, G,
-                                                                         b.boxPartial);
-  k_seg_box_final<<<(G + kThreads - 1) / kThreads, kThreads, 0, s>>>(b.boxChunkOffsets, G, b.boxPartial, b.params,
-                                                                      b.mortonCubic);
+  if (b.nBoxChunks + b.nIdxChunks) k_seg_read_inputs<<<b.nBoxChunks + b.nIdxChunks, kThreads, 0, s>>>(b);
+  k_seg_box_final<<<(G + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, s>>>(b.boxChunkOffsets, G, b.boxPartial,
+                                                                                  b.params, b.mortonCubic);
   k_seg_morton<<<(N + kThreads - 1) / kThreads, kThreads, 0, s>>>(b.verts, b.idx, b.vertOffsets, b.triOffsets, G, N,
                                                                    b.params, b.keys, b.vals, b.errorWord);
   cudaError_t e = cudaMemcpyAsync(b.keysUnsorted, b.keys, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, s);

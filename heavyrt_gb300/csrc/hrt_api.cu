@@ -148,18 +148,16 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   uint64_t* bytes = &g.bytes;
   HRT_CUDA(ctx, dalloc(&g.verts, nVert, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.params, 1, bytes, st));
+  // inputs are read where they are when the kernels reach them, else copied
+  const uint8_t* src = nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos)) : nullptr;
   uint8_t* raw = nullptr;
-  if (nVert)
+  if (nVert && !src)
   {
-    if (stride == 16)
-      HRT_CUDA(ctx, cudaMemcpyAsync(g.verts, vpos, 16 * nVert, cudaMemcpyDefault, st));
-    else
-    {
-      HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
-      HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * nVert, cudaMemcpyDefault, st));
-    }
+    if (stride != 16) HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
+    void* to = raw ? raw : reinterpret_cast<uint8_t*>(g.verts);
+    HRT_CUDA(ctx, cudaMemcpyAsync(to, vpos, stride * nVert, cudaMemcpyDefault, st));
+    src = static_cast<const uint8_t*>(to);
   }
-  const uint8_t* src = raw ? raw : reinterpret_cast<const uint8_t*>(g.verts);
   if (N == 0)
   {
     HRT_CUDA(ctx, cudaMemsetAsync(g.params, 0, sizeof(BuildParams), st));
@@ -179,7 +177,12 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   uint32_t *keysAlt = nullptr, *valsAlt = nullptr, *parent = nullptr, *visit = nullptr;
   void* scratch = nullptr;
   HRT_CUDA(ctx, cudaMallocAsync((void**)&dIdx, sizeof(uint32_t) * nIdx, st));
-  HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * nIdx, cudaMemcpyDefault, st));
+  const uint32_t* idxSrc = static_cast<const uint32_t*>(input_in_place(ctx, idx));
+  if (!idxSrc)
+  {
+    HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * nIdx, cudaMemcpyDefault, st));
+    idxSrc = dIdx;
+  }
   HRT_CUDA(ctx, dalloc(&g.keys, N, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.vals, N, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.keysUnsorted, N, bytes, st));
@@ -202,6 +205,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   b.raw = src;
   b.rawStride = stride;
   b.verts = g.verts;
+  b.idxSrc = idxSrc;
   b.idx = dIdx;
   b.nVerts = g.nVerts;
   b.nTris = N;
@@ -291,88 +295,129 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   return HRT_OK;
 }
 
-// Device allocation owned by a batch: recorded in `owned` (freed together).
-template <typename T> cudaError_t balloc(T** p, size_t count, std::vector<void*>& owned)
+// Device allocation owned by a batch: recorded in `owned` (freed together,
+// free_batch), from the device's stream-ordered pool like a geometry's.
+template <typename T> cudaError_t balloc(T** p, size_t count, std::vector<void*>& owned, cudaStream_t st)
 {
-  const cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
+  const cudaError_t e = cudaMallocAsync((void**)p, sizeof(T) * (count ? count : 1), st);
   if (e == cudaSuccess) owned.push_back(*p);
   return e;
 }
 
+// Frees batch allocations, after the queries that may still read them.
+void free_batch(std::vector<void*>& owned)
+{
+  if (!owned.empty()) cudaDeviceSynchronize();
+  for (void* p : owned) cudaFree(p);
+  owned.clear();
+}
+
 inline size_t align_up(size_t b, size_t a) { return (b + a - 1) / a * a; }
+
+// The inputs of a batch: geometry i has vertices vOff[i] .. vOff[i+1]-1 and
+// indices iOff[i] .. iOff[i+1]-1 of the batch, in arrays of its own.  `joined`:
+// the arrays of all geometries follow one another (vpos[0], idx[0] their start).
+struct BatchInputs
+{
+  const float* const*    vpos;
+  const uint32_t* const* idx;
+  const uint64_t*        vOff;
+  const uint64_t*        iOff;
+  uint64_t               stride;
+  bool                   joined;
+};
 
 // Builds G geometries with one segmented LBVH build (build_batch.cu) and, for
 // a 4-wide layout, collapses each.  On success appends G geometries whose
 // arrays point into allocations recorded in `owned`.
-int build_batch(hrt_scene* s, uint32_t G, const float* vpos, const uint64_t* vOff, const uint32_t* idx,
-                const uint64_t* iOff, uint64_t stride, std::vector<Geom>& out, std::vector<void*>& owned)
+int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geom>& out, std::vector<void*>& owned)
 {
   hrt_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
+  const uint64_t *vOff = in.vOff, *iOff = in.iOff, stride = in.stride;
   const uint64_t V = vOff[G], N = iOff[G] / 3;
-  std::vector<uint32_t> hv(G + 1), ht(G + 1);
-  for (uint32_t i = 0; i <= G; i++)
+  // one table for the device: source addresses, then the offsets of vertices,
+  // triangles, vertex chunks and index chunks
+  std::vector<uint64_t> table(2 * (size_t)G + 2 * ((size_t)G + 1));
+  uint64_t* srcV = table.data();
+  uint64_t* srcI = srcV + G;
+  uint32_t* hv = reinterpret_cast<uint32_t*>(srcI + G);
+  uint32_t *ht = hv + (G + 1), *hBox = ht + (G + 1), *hIdx = hBox + (G + 1);
+  hv[0] = ht[0] = hBox[0] = hIdx[0] = 0;
+  for (uint32_t i = 1; i <= G; i++)
   {
     hv[i] = (uint32_t)vOff[i];
     ht[i] = (uint32_t)(iOff[i] / 3);
+    hBox[i] = hBox[i - 1] + (hv[i] - hv[i - 1] + kBatchBoxChunk - 1) / kBatchBoxChunk;
+    hIdx[i] = hIdx[i - 1] + (uint32_t)((iOff[i] - iOff[i - 1] + kBatchIdxChunk - 1) / kBatchIdxChunk);
   }
-  // inputs
-  float4* verts = nullptr;
-  uint32_t *dVOff = nullptr, *dTOff = nullptr, *dIdx = nullptr;
-  HRT_CUDA(ctx, balloc(&verts, V, owned));
-  HRT_CUDA(ctx, cudaMallocAsync((void**)&dVOff, sizeof(uint32_t) * (G + 1), st));
-  HRT_CUDA(ctx, cudaMallocAsync((void**)&dTOff, sizeof(uint32_t) * (G + 1), st));
-  HRT_CUDA(ctx, cudaMemcpyAsync(dVOff, hv.data(), sizeof(uint32_t) * (G + 1), cudaMemcpyHostToDevice, st));
-  HRT_CUDA(ctx, cudaMemcpyAsync(dTOff, ht.data(), sizeof(uint32_t) * (G + 1), cudaMemcpyHostToDevice, st));
-  if (V)
+  // Inputs are read where they are when the kernels reach them, else copied
+  // first.  Arrays that follow one another are asked for once.
+  uint8_t *stageV = nullptr, *stageI = nullptr;
+  for (uint32_t i = 0; i < G; i++)
   {
-    uint8_t* raw = nullptr;
-    if (stride == 16)
-      HRT_CUDA(ctx, cudaMemcpyAsync(verts, vpos, 16 * V, cudaMemcpyHostToDevice, st));
-    else
+    const uint64_t nv = vOff[i + 1] - vOff[i], ni = iOff[i + 1] - iOff[i];
+    const bool derive = in.joined && i > 0;
+    srcV[i] = derive ? (srcV[0] ? srcV[0] + stride * vOff[i] : 0)
+                     : (uint64_t)(uintptr_t)((nv || in.joined) && V ? input_in_place(ctx, in.vpos[i]) : nullptr);
+    srcI[i] = derive ? (srcI[0] ? srcI[0] + 4 * iOff[i] : 0)
+                     : (uint64_t)(uintptr_t)((ni || in.joined) && N ? input_in_place(ctx, in.idx[i]) : nullptr);
+    const bool copyV = !srcV[i] && (derive ? false : (in.joined ? V : nv) > 0);
+    const bool copyI = !srcI[i] && (derive ? false : (in.joined ? N : ni) > 0);
+    if (copyV)
     {
-      HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * V, st));
-      HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * V, cudaMemcpyHostToDevice, st));
+      if (!stageV) HRT_CUDA(ctx, cudaMallocAsync((void**)&stageV, stride * V, st));
+      HRT_CUDA(ctx, cudaMemcpyAsync(stageV + stride * vOff[i], in.vpos[i], stride * (in.joined ? V : nv),
+                                    cudaMemcpyDefault, st));
+      srcV[i] = (uint64_t)(uintptr_t)(stageV + stride * vOff[i]);
     }
-    const int rc = pack_verts(ctx, st, verts, raw ? raw : reinterpret_cast<const uint8_t*>(verts), V, stride);
-    if (rc != HRT_OK) return rc;
-    if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
+    if (copyI)
+    {
+      if (!stageI) HRT_CUDA(ctx, cudaMallocAsync((void**)&stageI, 12 * N, st));
+      HRT_CUDA(ctx, cudaMemcpyAsync(stageI + 4 * iOff[i], in.idx[i], 4 * (in.joined ? 3 * N : ni), cudaMemcpyDefault, st));
+      srcI[i] = (uint64_t)(uintptr_t)(stageI + 4 * iOff[i]);
+    }
   }
+  uint64_t* dTable = nullptr;
+  HRT_CUDA(ctx, cudaMallocAsync((void**)&dTable, sizeof(uint64_t) * table.size(), st));
+  HRT_CUDA(ctx, cudaMemcpyAsync(dTable, table.data(), sizeof(uint64_t) * table.size(), cudaMemcpyHostToDevice, st));
+  const uint32_t* dOff = reinterpret_cast<const uint32_t*>(dTable + 2 * (size_t)G);
   BatchBuffers b{};
-  b.verts = verts;
-  b.vertOffsets = dVOff;
-  b.triOffsets = dTOff;
+  b.rawVerts = reinterpret_cast<const uint8_t* const*>(dTable);
+  b.rawIdx = reinterpret_cast<const uint32_t* const*>(dTable + G);
+  b.rawStride = stride;
+  b.vertOffsets = dOff;
+  b.triOffsets = dOff + (G + 1);
+  b.boxChunkOffsets = dOff + 2 * ((size_t)G + 1);
+  b.idxChunkOffsets = dOff + 3 * ((size_t)G + 1);
+  b.nBoxChunks = hBox[G];
+  b.nIdxChunks = hIdx[G];
   b.G = G;
   b.nTris = (uint32_t)N;
   b.vertexRecords = s->triTest == HRT_TRI_WATERTIGHT;
   b.mortonCubic = s->mortonFrame == HRT_MORTON_CUBIC;
-  // scene-box chunks of each geometry's vertices
-  std::vector<uint32_t> hChunk(G + 1, 0);
-  for (uint32_t i = 0; i < G; i++) hChunk[i + 1] = hChunk[i] + (hv[i + 1] - hv[i] + kBatchBoxChunk - 1) / kBatchBoxChunk;
-  uint32_t* dChunk = nullptr;
-  float4* boxPartial = nullptr;
-  HRT_CUDA(ctx, cudaMallocAsync((void**)&dChunk, sizeof(uint32_t) * (G + 1), st));
-  HRT_CUDA(ctx, cudaMallocAsync((void**)&boxPartial, 2 * sizeof(float4) * (hChunk[G] ? hChunk[G] : 1), st));
-  HRT_CUDA(ctx, cudaMemcpyAsync(dChunk, hChunk.data(), sizeof(uint32_t) * (G + 1), cudaMemcpyHostToDevice, st));
-  b.boxChunkOffsets = dChunk;
-  b.nBoxChunks = hChunk[G];
+  float4 *verts = nullptr, *boxPartial = nullptr;
+  uint32_t* dIdx = nullptr;
+  HRT_CUDA(ctx, balloc(&verts, V, owned, st));
+  b.verts = verts;
+  HRT_CUDA(ctx, cudaMallocAsync((void**)&boxPartial, 2 * sizeof(float4) * (hBox[G] ? hBox[G] : 1), st));
   b.boxPartial = boxPartial;
   uint32_t *keysAlt = nullptr, *valsAlt = nullptr, *parent = nullptr, *visit = nullptr;
   void* scratch = nullptr;
-  HRT_CUDA(ctx, balloc(&b.keys, N, owned));
-  HRT_CUDA(ctx, balloc(&b.vals, N, owned));
-  HRT_CUDA(ctx, balloc(&b.keysUnsorted, N, owned));
-  HRT_CUDA(ctx, balloc(&b.compressed, N, owned));
-  HRT_CUDA(ctx, balloc(&b.runStarts, N, owned));
-  HRT_CUDA(ctx, balloc(&b.lr, 2 * N, owned));
-  HRT_CUDA(ctx, balloc(&b.lrCount, 2 * N, owned));
-  if (s->layout == HRT_LAYOUT_BVH2) HRT_CUDA(ctx, balloc(&b.recs, N, owned));
-  HRT_CUDA(ctx, balloc(&b.tris, N, owned));
-  HRT_CUDA(ctx, balloc(&b.sortedIdx, 3 * N, owned));
-  HRT_CUDA(ctx, balloc(&b.params, G, owned));
+  HRT_CUDA(ctx, balloc(&b.keys, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.vals, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.keysUnsorted, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.compressed, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.runStarts, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.lr, 2 * N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.lrCount, 2 * N, owned, st));
+  if (s->layout == HRT_LAYOUT_BVH2) HRT_CUDA(ctx, balloc(&b.recs, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.tris, N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.sortedIdx, 3 * N, owned, st));
+  HRT_CUDA(ctx, balloc(&b.params, G, owned, st));
   // offsets (4 x (G+1)), counts (4) and the error word in one array
   uint32_t* offs = nullptr;
-  HRT_CUDA(ctx, balloc(&offs, 4 * ((size_t)G + 1) + 8, owned));
+  HRT_CUDA(ctx, balloc(&offs, 4 * ((size_t)G + 1) + 8, owned, st));
   b.leafOffsets = offs;
   b.intOffsets = offs + (G + 1);
   b.nodeOffsets = offs + 2 * (G + 1);
@@ -381,7 +426,6 @@ int build_batch(hrt_scene* s, uint32_t G, const float* vpos, const uint64_t* vOf
   b.errorWord = b.counts + 4;
   HRT_CUDA(ctx, cudaMemsetAsync(offs, 0, sizeof(uint32_t) * (4 * ((size_t)G + 1) + 8), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&dIdx, sizeof(uint32_t) * 3 * (N ? N : 1), st));
-  if (N) HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * 3 * N, cudaMemcpyHostToDevice, st));
   b.idx = dIdx;
   HRT_CUDA(ctx, cudaMallocAsync((void**)&keysAlt, sizeof(uint32_t) * (N ? N : 1), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&valsAlt, sizeof(uint32_t) * (N ? N : 1), st));
@@ -438,23 +482,16 @@ int build_batch(hrt_scene* s, uint32_t G, const float* vpos, const uint64_t* vOf
     q.mergeMode = s->bvh4Merge;
     q.collapse = s->bvh4Collapse;
     HRT_CUDA(ctx, cudaMallocAsync(&scratch4, bvh4_batch_scratch_bytes(nInt, G), st));
-    uint32_t* hostCounts = nullptr;
-    HRT_CUDA(ctx, cudaMallocHost((void**)&hostCounts, sizeof(uint32_t) * (2 * (size_t)G + 1)));
-    cudaError_t pe = bvh4_plan_batch(q, nInt, scratch4, hostCounts, hostCounts + G, b.errorWord, ctx->numSMs, st);
-    if (pe == cudaSuccess) pe = cudaStreamSynchronize(st);
-    if (pe != cudaSuccess)
-    {
-      cudaFreeHost(hostCounts);
-      return cuda_fail(ctx, pe, "bvh4_plan_batch");
-    }
+    std::vector<uint32_t> hostCounts(2 * (size_t)G + 1);
+    HRT_CUDA(ctx, bvh4_plan_batch(q, nInt, scratch4, hostCounts.data(), hostCounts.data() + G, b.errorWord, ctx->numSMs, st));
+    HRT_CUDA(ctx, cudaStreamSynchronize(st));
     for (uint32_t i = 0; i < G; i++)
     {
       count4[i] = hostCounts[i];
       node4Off[i] = hostCounts[G + i];
     }
     const size_t total = hostCounts[2 * (size_t)G];
-    cudaFreeHost(hostCounts);
-    HRT_CUDA(ctx, balloc((char**)&nodes4, nodeBytes * (total ? total : 1), owned));
+    HRT_CUDA(ctx, balloc((char**)&nodes4, nodeBytes * (total ? total : 1), owned, st));
     HRT_CUDA(ctx, bvh4_emit_batch(q, nInt, scratch4, s->layout - 1, nodes4, b.errorWord, ctx->numSMs, st));
   }
   HRT_CUDA(ctx, cudaEventRecord(e1, st));
@@ -470,9 +507,9 @@ int build_batch(hrt_scene* s, uint32_t G, const float* vpos, const uint64_t* vOf
   HRT_CUDA(ctx, cudaFreeAsync(parent, st));
   HRT_CUDA(ctx, cudaFreeAsync(visit, st));
   HRT_CUDA(ctx, cudaFreeAsync(scratch, st));
-  HRT_CUDA(ctx, cudaFreeAsync(dVOff, st));
-  HRT_CUDA(ctx, cudaFreeAsync(dTOff, st));
-  HRT_CUDA(ctx, cudaFreeAsync(dChunk, st));
+  HRT_CUDA(ctx, cudaFreeAsync(dTable, st));
+  if (stageV) HRT_CUDA(ctx, cudaFreeAsync(stageV, st));
+  if (stageI) HRT_CUDA(ctx, cudaFreeAsync(stageI, st));
   HRT_CUDA(ctx, cudaFreeAsync(boxPartial, st));
   if (scratch4) HRT_CUDA(ctx, cudaFreeAsync(scratch4, st));
   HRT_CUDA(ctx, cudaStreamSynchronize(st));
@@ -639,14 +676,15 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   cudaStream_t st = ctx->stream;
   const uint32_t N = g.nTris;
   const uint64_t nVert = g.nVerts;
+  const uint8_t* src = nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos)) : nullptr;
   uint8_t* raw = nullptr;
-  if (nVert && stride == 16) HRT_CUDA(ctx, cudaMemcpyAsync(g.verts, vpos, 16 * nVert, cudaMemcpyHostToDevice, st));
-  if (nVert && stride != 16)
+  if (nVert && !src)
   {
-    HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
-    HRT_CUDA(ctx, cudaMemcpyAsync(raw, vpos, stride * nVert, cudaMemcpyHostToDevice, st));
+    if (stride != 16) HRT_CUDA(ctx, cudaMallocAsync((void**)&raw, stride * nVert, st));
+    void* to = raw ? raw : reinterpret_cast<uint8_t*>(g.verts);
+    HRT_CUDA(ctx, cudaMemcpyAsync(to, vpos, stride * nVert, cudaMemcpyDefault, st));
+    src = static_cast<const uint8_t*>(to);
   }
-  const uint8_t* src = raw ? raw : reinterpret_cast<const uint8_t*>(g.verts);
   if (N == 0)
   {
     const int rc = pack_verts(ctx, st, g.verts, src, nVert, stride);
@@ -659,7 +697,12 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   BuildParams* box = nullptr;
   void* scratch = nullptr;
   HRT_CUDA(ctx, cudaMallocAsync((void**)&dIdx, sizeof(uint32_t) * 3 * (size_t)N, st));
-  HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * 3 * (size_t)N, cudaMemcpyHostToDevice, st));
+  const uint32_t* idxSrc = static_cast<const uint32_t*>(input_in_place(ctx, idx));
+  if (!idxSrc)
+  {
+    HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * 3 * (size_t)N, cudaMemcpyDefault, st));
+    idxSrc = dIdx;
+  }
   HRT_CUDA(ctx, cudaMallocAsync((void**)&parent, sizeof(uint32_t) * (2 * (size_t)N - 1), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&visit, sizeof(uint32_t) * 2 * (size_t)N, st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&box, sizeof(BuildParams), st));
@@ -669,6 +712,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   b.raw = src;
   b.rawStride = stride;
   b.verts = g.verts;
+  b.idxSrc = idxSrc;
   b.idx = dIdx;
   b.nVerts = g.nVerts;
   b.nTris = N;
@@ -787,6 +831,20 @@ void* mapped_host(const void* p, bool pageable)
   if (a.type == cudaMemoryTypeHost) return a.devicePointer;
   if (pageable && a.type == cudaMemoryTypeUnregistered && pageable_access()) return const_cast<void*>(p);
   return nullptr;
+}
+
+const void* input_in_place(const hrt_context* ctx, const void* p)
+{
+  cudaPointerAttributes a;
+  if (!aligned_to(p, 4)) return nullptr;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess)
+  {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type == cudaMemoryTypeDevice) return a.device == ctx->device ? p : nullptr;
+  if (a.type == cudaMemoryTypeHost) return a.devicePointer;
+  return a.type == cudaMemoryTypeUnregistered && pageable_access() ? p : nullptr;
 }
 
 int ensure_stage(hrt_scene* s, uint64_t n)
@@ -984,8 +1042,7 @@ int hrt_clear_geom(hrt_scene* s)
   cudaStreamSynchronize(s->ctx->stream);
   for (Geom& gm : s->geoms) free_geom(gm);
   free_geom(s->tlas);
-  for (void* p : s->batchAllocs) cudaFree(p);
-  s->batchAllocs.clear();
+  free_batch(s->batchAllocs);
   s->geoms.clear();
   s->insts.clear();
   s->committed = false;
@@ -1036,41 +1093,42 @@ int hrt_add_geom_triangles3f(hrt_scene* s, const float* vpos, uint64_t nVert, co
   return HRT_OK;
 }
 
-int hrt_add_geoms_triangles3f_batched(hrt_scene* s, uint32_t count, const float* vpos, const uint64_t* vertOffsets,
-                                      const uint32_t* idx, const uint64_t* idxOffsets, int quality,
-                                      uint64_t vByteStride, uint32_t* firstGeomId)
+// The two batch entry points: checks, build, registration.  Null arrays are
+// refused where they should hold something.
+static int add_batch(hrt_scene* s, uint32_t count, BatchInputs in, uint32_t* firstGeomId)
 {
-  (void)quality;
-  if (!s) return HRT_ERR_INVALID_ARGUMENT;
   hrt_context* ctx = s->ctx;
-  if (count == 0) return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "empty batch");
-  if (!vertOffsets || !idxOffsets) return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "null offset array");
-  if (vByteStride == 0) vByteStride = 12;
-  if (vByteStride < 12 || vByteStride % 4 != 0)
+  if (in.stride == 0) in.stride = 12;
+  if (in.stride < 12 || in.stride % 4 != 0)
     return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "vByteStride must be >= 12 and a multiple of 4");
-  if (vertOffsets[0] != 0 || idxOffsets[0] != 0) return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "offsets must start at 0");
+  if (in.vOff[0] != 0 || in.iOff[0] != 0) return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "offsets must start at 0");
   for (uint32_t i = 0; i < count; i++)
   {
-    if (vertOffsets[i + 1] < vertOffsets[i] || idxOffsets[i + 1] < idxOffsets[i])
+    if (in.vOff[i + 1] < in.vOff[i] || in.iOff[i + 1] < in.iOff[i])
       return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "offsets must be ascending");
-    if ((idxOffsets[i + 1] - idxOffsets[i]) % 3 != 0)
+    if ((in.iOff[i + 1] - in.iOff[i]) % 3 != 0)
       return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "a geometry's index count is not a multiple of 3");
-    if ((idxOffsets[i + 1] - idxOffsets[i]) / 3 > HRT_MAX_TRIS_PER_GEOM)
+    if ((in.iOff[i + 1] - in.iOff[i]) / 3 > HRT_MAX_TRIS_PER_GEOM)
       return fail(ctx, HRT_ERR_CAPACITY, "more than 2^24-1 triangles in one geometry");
   }
-  const uint64_t V = vertOffsets[count], nIdx = idxOffsets[count];
-  if ((V && !vpos) || (nIdx && !idx)) return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "null vertex or index pointer");
+  const uint64_t V = in.vOff[count], nIdx = in.iOff[count];
+  for (uint32_t i = 0; i < (in.joined ? 1u : count); i++)
+  {
+    const uint64_t nv = in.joined ? V : in.vOff[i + 1] - in.vOff[i], ni = in.joined ? nIdx : in.iOff[i + 1] - in.iOff[i];
+    if ((nv && !in.vpos[i]) || (ni && !in.idx[i]))
+      return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "null vertex or index pointer");
+  }
   if (nIdx / 3 > HRT_MAX_TRIS_PER_BATCH) return fail(ctx, HRT_ERR_CAPACITY, "more than 2^30-1 triangles in one batch");
   if (V > 0xFFFFFFFFull) return fail(ctx, HRT_ERR_CAPACITY, "more than 2^32-1 vertices in one batch");
   std::lock_guard<std::mutex> lk(s->mu);
   cudaSetDevice(ctx->device);
   std::vector<Geom> built;
   std::vector<void*> owned;
-  const int st = build_batch(s, count, vpos, vertOffsets, idx, idxOffsets, vByteStride, built, owned);
+  const int st = build_batch(s, count, in, built, owned);
   if (st != HRT_OK)
   {
     cudaStreamSynchronize(ctx->stream);
-    for (void* p : owned) cudaFree(p);
+    free_batch(owned);
     return st;
   }
   const uint32_t first = (uint32_t)s->geoms.size();
@@ -1079,6 +1137,37 @@ int hrt_add_geoms_triangles3f_batched(hrt_scene* s, uint32_t count, const float*
   s->committed = false;
   if (firstGeomId) *firstGeomId = first;
   return HRT_OK;
+}
+
+int hrt_add_geoms_triangles3f_batched(hrt_scene* s, uint32_t count, const float* vpos, const uint64_t* vertOffsets,
+                                      const uint32_t* idx, const uint64_t* idxOffsets, int quality,
+                                      uint64_t vByteStride, uint32_t* firstGeomId)
+{
+  (void)quality;
+  if (!s) return HRT_ERR_INVALID_ARGUMENT;
+  if (count == 0) return fail(s->ctx, HRT_ERR_INVALID_ARGUMENT, "empty batch");
+  if (!vertOffsets || !idxOffsets) return fail(s->ctx, HRT_ERR_INVALID_ARGUMENT, "null offset array");
+  return add_batch(s, count, BatchInputs{&vpos, &idx, vertOffsets, idxOffsets, vByteStride, true}, firstGeomId);
+}
+
+int hrt_add_geoms_triangles3f_arrays(hrt_scene* s, uint32_t count, const float* const* vpos, const uint64_t* nVert,
+                                     const uint32_t* const* idx, const uint64_t* nIdx, int quality,
+                                     uint64_t vByteStride, uint32_t* firstGeomId)
+{
+  (void)quality;
+  if (!s) return HRT_ERR_INVALID_ARGUMENT;
+  if (count == 0) return fail(s->ctx, HRT_ERR_INVALID_ARGUMENT, "empty batch");
+  if (!vpos || !nVert || !idx || !nIdx) return fail(s->ctx, HRT_ERR_INVALID_ARGUMENT, "null array of arrays or counts");
+  std::vector<uint64_t> vOff(count + 1, 0), iOff(count + 1, 0);
+  for (uint32_t i = 0; i < count; i++)
+  {
+    if (nVert[i] > 0xFFFFFFFFull) return fail(s->ctx, HRT_ERR_CAPACITY, "more than 2^32-1 vertices in one batch");
+    if (nIdx[i] / 3 > HRT_MAX_TRIS_PER_GEOM)
+      return fail(s->ctx, HRT_ERR_CAPACITY, "more than 2^24-1 triangles in one geometry");
+    vOff[i + 1] = vOff[i] + nVert[i];
+    iOff[i + 1] = iOff[i] + nIdx[i];
+  }
+  return add_batch(s, count, BatchInputs{vpos, idx, vOff.data(), iOff.data(), vByteStride, false}, firstGeomId);
 }
 
 int hrt_update_geom_triangles3f(hrt_scene* s, uint32_t geomId, const float* vpos, uint64_t nVert, const uint32_t* idx,

@@ -139,6 +139,10 @@ bool is_identity(const float* m);
 // (pageable_access); null otherwise.
 void* mapped_host(const void* p, bool pageable = false);
 bool pageable_access();
+// The address at which this device's kernels read a build's input in place:
+// device memory of the context's device, or host memory as mapped_host with
+// pageable; null where it has to be copied first.
+const void* input_in_place(const hrt_context* ctx, const void* p);
 // True when p is a multiple of `bytes` (a power of two).  Kernels read rays
 // and write hits as 16-byte vectors, so arrays they access in place must be
 // 16-byte aligned; the entry points check this before any launch.

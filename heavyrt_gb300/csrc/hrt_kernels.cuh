@@ -32,10 +32,11 @@ cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t*
 struct BuildBuffers
 {
   // inputs (device)
-  const uint8_t*  raw;        // nVerts vertices of rawStride bytes, xyz first (may be verts itself)
-  uint64_t        rawStride;
+  const uint8_t*  raw;        // nVerts vertices of rawStride bytes, xyz first (may be verts itself);
+  uint64_t        rawStride;  // device memory or host memory that kernels reach
+  const uint32_t* idxSrc;     // 3 * nTris, likewise (may be idx itself)
   float4*         verts;      // nVerts, packed from raw with w = 1
-  const uint32_t* idx;        // 3 * nTris
+  uint32_t*       idx;        // 3 * nTris, copied from idxSrc
   uint32_t        nVerts;
   uint32_t        nTris;
   // stage arrays (device)
@@ -82,8 +83,14 @@ cudaError_t refit_lbvh(const BuildBuffers& b, BuildParams* boxOut, int numSMs, c
 // are computed on the device.
 struct BatchBuffers
 {
-  const float4*   verts;        // total vertices, w = 1
-  const uint32_t* idx;          // 3 * nTris, local to each geometry
+  // inputs: geometry s's vertices (rawStride bytes each, xyz first) and indices
+  // (local to its vertices) at rawVerts[s] and rawIdx[s], device memory or host
+  // memory that kernels reach; packed and copied to verts and idx
+  const uint8_t* const*  rawVerts;  // G (device table)
+  const uint32_t* const* rawIdx;    // G (device table)
+  uint64_t        rawStride;
+  float4*         verts;        // total vertices, w = 1
+  uint32_t*       idx;          // 3 * nTris
   const uint32_t* vertOffsets;  // G+1 (device)
   const uint32_t* triOffsets;   // G+1 (device)
   uint32_t        G;
@@ -110,15 +117,17 @@ struct BatchBuffers
   uint32_t*  counts;            // 4
   uint32_t*  errorWord;         // device word shared by the batch
   void*      scratch;           // build_batch_scratch_bytes(nTris, G)
-  // scene boxes: geometry s's vertices in chunks [boxChunkOffsets[s], boxChunkOffsets[s+1])
-  // of kBatchBoxChunk vertices, one (min, max) float4 pair per chunk in boxPartial
+  // reading the inputs: geometry s's vertices in chunks [boxChunkOffsets[s], boxChunkOffsets[s+1])
+  // of kBatchBoxChunk vertices, one (min, max) float4 pair per chunk in boxPartial, its
+  // indices in chunks [idxChunkOffsets[s], idxChunkOffsets[s+1]) of kBatchIdxChunk words
   const uint32_t* boxChunkOffsets;  // G+1 (device)
-  uint32_t        nBoxChunks;
+  const uint32_t* idxChunkOffsets;  // G+1 (device)
+  uint32_t        nBoxChunks, nIdxChunks;
   float4*         boxPartial;       // 2 * nBoxChunks
   int             vertexRecords = 0;  // as BuildBuffers::vertexRecords
   int             mortonCubic = 0;    // as BuildBuffers::mortonCubic
 };
-constexpr uint32_t kBatchBoxChunk = 8192;
+constexpr uint32_t kBatchBoxChunk = 2048, kBatchIdxChunk = 8192;
 size_t build_batch_scratch_bytes(uint32_t nTris, uint32_t G);
 cudaError_t build_lbvh_batch(const BatchBuffers& b, int numSMs, cudaStream_t stream);
 

@@ -194,6 +194,7 @@ def lib() -> C.CDLL:
         "hrt_scene_set_trace_config": (i32, [vp, i32, C.POINTER(TraceConfig)]),
         "hrt_scene_get_trace_config": (i32, [vp, i32, C.POINTER(TraceConfig)]),
         "hrt_add_geoms_triangles3f_batched": (i32, [vp, u32, vp, vp, vp, vp, i32, u64, C.POINTER(u32)]),
+        "hrt_add_geoms_triangles3f_arrays": (i32, [vp, u32, vp, vp, vp, vp, i32, u64, C.POINTER(u32)]),
         "hrt_query_multi": (i32, [vp, C.POINTER(QueryDesc), vp]),
         "hrt_graph_create": (i32, [vp, C.POINTER(QueryDesc), u32, C.POINTER(vp)]),
         "hrt_graph_launch": (i32, [vp, vp]),
@@ -237,6 +238,13 @@ def lib() -> C.CDLL:
 
 def _ptr(a: np.ndarray) -> C.c_void_p:
     return C.c_void_p(a.ctypes.data)
+
+
+def _addresses(arrays) -> C.Array:
+    return (C.c_void_p * len(arrays))(*(a.__array_interface__["data"][0] for a in arrays))
+
+
+_IDENTITY = np.eye(4, dtype=np.float32)
 
 
 class Context:
@@ -381,6 +389,8 @@ class SceneRT:
             a_indNumber = idx.size
         if v.size * 4 < a_vertNumber * stride - (stride - 12):
             raise ValueError("vertex array smaller than a_vertNumber * vByteStride")
+        if idx.size < a_indNumber:
+            raise ValueError("index array smaller than a_indNumber")
         gid = C.c_uint32()
         self.ctx.check(lib().hrt_add_geom_triangles3f(self._h, _ptr(v), int(a_vertNumber), _ptr(idx), int(a_indNumber),
                                                       int(a_qualityLevel), stride, C.byref(gid)),
@@ -391,6 +401,9 @@ class SceneRT:
                                a_qualityLevel=BUILD_HIGH, vByteStride=12):  # core/CrossRT.h:105
         v = np.ascontiguousarray(a_vpos3f, dtype=np.float32)
         idx = np.ascontiguousarray(a_triIndices, dtype=np.uint32)
+        stride = int(vByteStride) if vByteStride else 12
+        if v.size * 4 < a_vertNumber * stride - (stride - 12) or idx.size < a_indNumber:
+            raise ValueError("vertex or index array smaller than its count")
         self.ctx.check(lib().hrt_update_geom_triangles3f(self._h, a_geomId, _ptr(v), a_vertNumber, _ptr(idx), a_indNumber,
                                                          a_qualityLevel, vByteStride), "UpdateGeom_Triangles3f")
 
@@ -401,8 +414,10 @@ class SceneRT:
         self.ctx.check(lib().hrt_commit_scene(self._h, int(a_qualityLevel)), "CommitScene")
 
     def AddInstance(self, a_geomId: int, a_matrix=None) -> int:  # core/CrossRT.h:123
-        m = np.eye(4, dtype=np.float32) if a_matrix is None else np.asarray(a_matrix, dtype=np.float32).reshape(4, 4)
-        col = np.ascontiguousarray(m.T)  # column-major storage
+        if a_matrix is None:
+            col = _IDENTITY
+        else:
+            col = np.ascontiguousarray(np.asarray(a_matrix, dtype=np.float32).reshape(4, 4).T)  # column-major storage
         iid = C.c_uint32()
         self.ctx.check(lib().hrt_add_instance(self._h, a_geomId, _ptr(col), C.byref(iid)), "AddInstance")
         return iid.value
@@ -447,26 +462,24 @@ class SceneRT:
         verts_list[i]."""
         if len(verts_list) != len(idx_list) or not verts_list:
             raise ValueError("verts_list and idx_list must be non-empty and of equal length")
+        # each array is read where it is; one stride for all (xyz read at 12 or
+        # 16 bytes, the engine does not use w)
         vs = []
         for v in verts_list:
             a = np.asarray(v, dtype=np.float32)
-            a = a.reshape(len(a), -1) if a.size else np.zeros((0, 4), np.float32)
-            if a.shape[1] != 4:  # the engine reads xyz at a 16-byte stride; w is not used
-                p4 = np.ones((len(a), 4), np.float32)
+            vs.append(np.ascontiguousarray(a.reshape(len(a), -1)) if a.size else np.zeros((0, 4), np.float32))
+        width = 3 if all(a.shape[1] == 3 for a in vs if len(a)) else 4
+        for k, a in enumerate(vs):
+            if a.shape[1] != width:
+                p4 = np.ones((len(a), width), np.float32)
                 p4[:, :3] = a[:, :3]
-                a = p4
-            vs.append(a)
-        v = np.concatenate(vs, axis=0) if len(vs) > 1 else np.ascontiguousarray(vs[0])
-        ids = [np.asarray(i, dtype=np.uint32).reshape(-1) for i in idx_list]
-        idx = np.ascontiguousarray(np.concatenate(ids))
-        voff = np.zeros(len(vs) + 1, dtype=np.uint64)
-        voff[1:] = np.cumsum([len(x) for x in vs])
-        ioff = np.zeros(len(ids) + 1, dtype=np.uint64)
-        ioff[1:] = np.cumsum([len(x) for x in ids])
+                vs[k] = p4
+        ids = [np.ascontiguousarray(i, dtype=np.uint32).reshape(-1) for i in idx_list]
+        n = len(vs)
         first = C.c_uint32()
-        self.ctx.check(lib().hrt_add_geoms_triangles3f_batched(self._h, len(vs), _ptr(v), _ptr(voff), _ptr(idx),
-                                                               _ptr(ioff), int(a_qualityLevel), 16, C.byref(first)),
-                       "add_geoms_batched")
+        self.ctx.check(lib().hrt_add_geoms_triangles3f_arrays(
+            self._h, n, _addresses(vs), (C.c_uint64 * n)(*map(len, vs)), _addresses(ids),
+            (C.c_uint64 * n)(*map(len, ids)), int(a_qualityLevel), 4 * width, C.byref(first)), "add_geoms_batched")
         return list(range(first.value, first.value + len(vs)))
 
     def gen_ao_rays(self, seed: int, eye_ptr: int, hits_ptr: int, n_eye: int, per_hit: int, length: float,

@@ -199,7 +199,8 @@ int hrt_clear_geom(hrt_scene* scene);
 /* ISceneObject::AddGeom_Triangles3f (core/CrossRT.h:94; reference implementation
  * core/BVH2CommonRT_host.cpp:66-98).  Host arrays: vpos has nVert vertices of
  * vByteStride bytes (0 means 12), xyz first; idx has nIdx indices (3 per
- * triangle).  The data is copied; the LBVH is built on the GPU before the call
+ * triangle).  The data is copied (read in place where the GPU reaches host
+ * memory, or device memory); the LBVH is built on the GPU before the call
  * returns.  *geomId receives the new geometry id. */
 int hrt_add_geom_triangles3f(hrt_scene* scene, const float* vpos, uint64_t nVert, const uint32_t* idx, uint64_t nIdx,
                              int quality, uint64_t vByteStride, uint32_t* geomId);
@@ -333,6 +334,12 @@ int hrt_query_counters(hrt_scene* scene, int kind, const float* rays, uint64_t n
 int hrt_add_geoms_triangles3f_batched(hrt_scene* scene, uint32_t count, const float* vpos, const uint64_t* vertOffsets,
                                       const uint32_t* idx, const uint64_t* idxOffsets, int quality,
                                       uint64_t vByteStride, uint32_t* firstGeomId);
+
+/* The same batch from arrays that lie apart: geometry i has nVert[i] vertices at
+ * vpos[i] and nIdx[i] indices at idx[i] (no joined copy of them is needed). */
+int hrt_add_geoms_triangles3f_arrays(hrt_scene* scene, uint32_t count, const float* const* vpos, const uint64_t* nVert,
+                                     const uint32_t* const* idx, const uint64_t* nIdx, int quality,
+                                     uint64_t vByteStride, uint32_t* firstGeomId);
 
 /* One traversal launch.  rays/out as for hrt_query_nearest / hrt_query_any.
  * With rayOffsets == NULL every ray is traced against the whole scene; else

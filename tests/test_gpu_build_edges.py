@@ -103,3 +103,66 @@ def test_batches_across_slices(native, layout):
             got = s.export(gid, E.EXPORT_NODES4).view(np.uint32).reshape(-1, 16)
             np.testing.assert_array_equal(got[:, 12:16], want[:, 24:28])
     s.close()
+
+
+def _off(a, words):
+    """A copy of `a` that starts `words` 4-byte words past a 16-byte boundary."""
+    buf = np.zeros(a.size + 8, a.dtype)
+    at = (-buf.ctypes.data // 4) % 4 + words
+    out = buf[at:at + a.size].reshape(a.shape)
+    out[...] = a
+    return out
+
+
+@pytest.mark.parametrize("words", [0, 1, 3])
+@pytest.mark.parametrize("columns", [3, 4, 6])
+def test_inputs_in_place(native, columns, words):
+    """Host arrays of any alignment and stride, device arrays, and a batch's
+    arrays apart and joined give the arrays of a plain load."""
+    import ctypes as C
+
+    import torch
+
+    from heavyrt_gb300 import SceneRT
+    from heavyrt_gb300 import engine as E
+    from heavyrt_gb300 import workload as wl
+
+    meshes = [wl.soup(60 + k, n, off=0.02) for k, n in enumerate((1, 5, 700, 3001))]
+    s = SceneRT()
+    plain = [s.AddGeom_Triangles3f(v, len(v), i, i.size, vByteStride=16) for v, i in meshes]
+    want = [_stages(s, g) for g in plain]
+    raw = []
+    for v, i in meshes:
+        r = np.full((len(v), columns), 7.0, np.float32)
+        r[:, :3] = v[:, :3]
+        raw.append((_off(r, words), _off(i, words)))
+    for k, (r, i) in enumerate(raw):  # host, then device (the C entry takes addresses)
+        g = s.AddGeom_Triangles3f(r, len(r), i, i.size, vByteStride=4 * columns)
+        _check(_stages(s, g), want[k], f"mesh {k}")
+        dr, di = torch.zeros(r.size + 4, device="cuda"), torch.zeros(i.size + 4, dtype=torch.int32, device="cuda")
+        dr[words:words + r.size] = torch.from_numpy(r.copy()).reshape(-1).cuda()
+        di[words:words + i.size] = torch.from_numpy(i.view(np.int32).copy()).cuda()
+        torch.cuda.synchronize()
+        gid = C.c_uint32()
+        s.ctx.check(E.lib().hrt_add_geom_triangles3f(s._h, C.c_void_p(dr.data_ptr() + 4 * words), len(r),
+                                                     C.c_void_p(di.data_ptr() + 4 * words), i.size, 2, 4 * columns,
+                                                     C.byref(gid)), "device arrays")
+        _check(_stages(s, gid.value), want[k], f"mesh {k} on the device")
+    for k, g in enumerate(s.add_geoms_batched([r for r, _ in raw], [i for _, i in raw])):
+        _check(_stages(s, g), want[k], f"batch {k}")
+    # an array of another width among them: all are widened
+    mixed = [raw[0][0][:, :3].copy()] + [r for r, _ in raw[1:]]
+    for k, g in enumerate(s.add_geoms_batched(mixed, [i for _, i in raw])):
+        _check(_stages(s, g), want[k], f"mixed batch {k}")
+    v = _off(np.concatenate([r for r, _ in raw]), words)
+    i = _off(np.concatenate([i for _, i in raw]), words)
+    voff = np.cumsum([0] + [len(r) for r, _ in raw]).astype(np.uint64)
+    ioff = np.cumsum([0] + [x.size for _, x in raw]).astype(np.uint64)
+    first = C.c_uint32()
+    s.ctx.check(E.lib().hrt_add_geoms_triangles3f_batched(s._h, len(raw), E._ptr(v), E._ptr(voff), E._ptr(i), E._ptr(ioff),
+                                                          2, 4 * columns, C.byref(first)), "joined")
+    for k in range(len(raw)):
+        _check(_stages(s, first.value + k), want[k], f"joined batch {k}")
+    with pytest.raises(ValueError):
+        s.AddGeom_Triangles3f(raw[0][0], len(raw[0][0]), raw[0][1], raw[0][1].size + 3, vByteStride=4 * columns)
+    s.close()
