@@ -19,8 +19,9 @@ namespace
 
 // Warps an SM that a small batch is spread over, and that hold a batch at once.
 constexpr int kSpreadWarps = 13, kResidentWarps = 36;
-// Idle lanes at which a warp refills unless the caller set a shape.
-constexpr int kRefillLanes = 8;
+// Unless the caller set a shape: idle lanes at which a warp refills, and
+// advances (phases of an instance tree's walk) between its looks at them.
+constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32;
 
 // The shape of one launch.
 //
@@ -38,13 +39,19 @@ constexpr int kRefillLanes = 8;
 // FP16 nodes 180 -> 170); 262,144 eye rays are faster in the pool (binary 157
 // against 172).
 //
-// The refill threshold: incoherent rays want idle lanes filled early (500,000
+// The refills: incoherent rays want idle lanes filled early (500,000
 // random rays, 8-bit nodes: 652 us at 24 lanes, 555 at 8; FP16 582 -> 520),
-// and coherent ones do not care (full-HD eye rays 156 against 157).
+// and coherent ones do not care (full-HD eye rays 156 against 157).  Looks after
+// 4, 8, 16 advances: 2M occlusion rays, FP16 nodes 391, 378, 419 us, 500,000
+// random rays 496, 497, 509; after 16 and 32 phases, 240 instances 1,161, 1,154.
 TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int numSMs)
 {
   TraceConfig s = c;
-  if (!c.given && s.refillLanes > kRefillLanes) s.refillLanes = kRefillLanes;
+  if (!c.given)
+  {
+    if (s.refillLanes > kRefillLanes) s.refillLanes = kRefillLanes;
+    s.stepsPerRefill = a.tlasRecs != nullptr && a.rayOffsets == nullptr ? kTreePhases : kAdvances;
+  }
   int perWarp = 32;
   while (perWarp > 1 && a.n <= (uint64_t)numSMs * kSpreadWarps * (perWarp / 2)) perWarp /= 2;
   if (a.n <= (uint64_t)numSMs * kResidentWarps * 32)

@@ -282,7 +282,7 @@ int hrt_scene_check(hrt_scene* scene);
  * one ray per virtual call with an 80-entry stack, core/raytrace_common.h:34).
  * Defaults: 128 threads, persistent pool, 16 steps between refills, refill at
  * 24 idle lanes, the whole stack in shared memory.  Until a shape is set for a
- * kind the engine may pick a better one per launch (refills at 8 idle lanes;
+ * kind the engine may pick a better one per launch (looks every 8 steps for 8 idle lanes;
  * eye rays of hrt_frame_* one thread per ray; an instance tree's stack in
  * local memory).  Batches whose rays all fit on the GPU at once are traced one
  * thread per ray whatever the shape, small ones with fewer rays a warp.
@@ -297,7 +297,7 @@ typedef struct hrt_trace_config
 {
   int threadsPerBlock; /* 64, 128 or 256                                          */
   int persistent;      /* 1: persistent warp pool that refills idle lanes; 0: one thread per ray */
-  int stepsPerRefill;  /* traversal steps between refill checks (1..1024)        */
+  int stepsPerRefill;  /* traversal steps (a few nodes and a leaf) between refill checks (1..1024) */
   int refillLanes;     /* a warp refills when at least this many lanes are idle (1..32) */
   int stackEntries;    /* short-stack entries in shared memory (0..HRT_MAX_STACK_ENTRIES) */
   int imageWidth;      /* > 0: the rays form row-major images this many rays wide (as a
