@@ -213,6 +213,9 @@ struct TraceArgs
   const uint32_t*     rayOffsets = nullptr;
   const uint32_t*     segInst = nullptr;
   uint32_t            nSeg = 0;
+  // segmented query whose segments' rays lie apart (optional): segment k's
+  // first ray at segRays[k] (device array); `rays` is not read then
+  const float4* const* segRays = nullptr;
   // instance tree (optional): binary LBVH over the instances' world boxes;
   // its triangle records' e1.w hold instance ids
   const PairRec*      tlasRecs = nullptr;

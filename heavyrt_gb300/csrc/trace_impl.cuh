@@ -1127,9 +1127,10 @@ struct Segments
   const uint32_t* segInst;
   uint32_t        nSeg;
   uint32_t        nInst;
+  const float4* const* segRays;  // segment k's rays, where they lie apart; nullptr: ray i at rays[2 i]
 };
 
-__device__ __forceinline__ uint32_t segment_instance(uint32_t i, const Segments& sg)
+__device__ __forceinline__ uint32_t segment_of(uint32_t i, const Segments& sg)
 {
   uint32_t lo = 0, hi = sg.nSeg;
   while (hi - lo > 1)
@@ -1138,13 +1139,13 @@ __device__ __forceinline__ uint32_t segment_instance(uint32_t i, const Segments&
     if (__ldg(sg.rayOffsets + mid) <= i) lo = mid;
     else hi = mid;
   }
-  return __ldg(sg.segInst + lo);
+  return lo;
 }
 
 template <int LAYOUT>
 __device__ __forceinline__ uint32_t first_instance(Lane<LAYOUT>& L, uint32_t i, const Segments& sg)
 {
-  const uint32_t k = sg.rayOffsets == nullptr ? 0u : segment_instance(i, sg);
+  const uint32_t k = sg.rayOffsets == nullptr ? 0u : __ldg(sg.segInst + segment_of(i, sg));
   L.instEnd = sg.rayOffsets == nullptr ? sg.nInst : (k < sg.nInst ? k + 1 : 0);
   return k;
 }
@@ -1309,7 +1310,14 @@ __device__ __forceinline__ void start_ray_one(Lane1<LAYOUT>& L, uint32_t i, cons
                                               const OneSource& src)
 {
   float4 po, di;
-  load_record(rays + 2 * (size_t)i, po, di);
+  uint32_t seg = 0;
+  const float4* at = rays + 2 * (size_t)i;
+  if (SEG)
+  {
+    seg = segment_of(i, src.sg);
+    if (src.sg.segRays != nullptr) at = src.sg.segRays[seg] + 2 * (size_t)(i - __ldg(src.sg.rayOffsets + seg));
+  }
+  load_record(at, po, di);
   L.ray = i;
   L.h.t = di.w;
   L.h.u = L.h.v = 0.0f;
@@ -1322,7 +1330,7 @@ __device__ __forceinline__ void start_ray_one(Lane1<LAYOUT>& L, uint32_t i, cons
     set_ray(L.r, po.x, po.y, po.z, po.w, di.x, di.y, di.z);
     return;
   }
-  const uint32_t k = segment_instance(i, src.sg);
+  const uint32_t k = __ldg(src.sg.segInst + seg);
   L.inst = k;
   if (k < src.sg.nInst && src.inst[k].valid)
   {
@@ -1479,7 +1487,7 @@ cudaError_t launch_one(const TraceArgs& a, const TraceConfig& c, int numSMs, cud
   if (SEG)
   {
     src.inst = a.inst;
-    src.sg = Segments{a.rayOffsets, a.segInst, a.nSeg, a.nInst};
+    src.sg = Segments{a.rayOffsets, a.segInst, a.nSeg, a.nInst, a.segRays};
     src.instId = src.geomId = 0xFFFFFFFFu;  // of a miss
   }
   else
@@ -1564,7 +1572,7 @@ template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, bool TLAS, int
 cudaError_t launch(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStream_t s)
 {
   const uint32_t n = (uint32_t)a.n;
-  const Segments sg{a.rayOffsets, a.segInst, a.nSeg, a.nInst};
+  const Segments sg{a.rayOffsets, a.segInst, a.nSeg, a.nInst, nullptr};
   const Tlas tl{a.tlasRecs, a.tlasTris, a.nInst};
   const int shared = STACK == kStackLocal ? 0
                      : STACK == kStackSplit ? shared_entries<StackDepth<LAYOUT, TLAS>::value>(c.stackEntries)
