@@ -31,13 +31,16 @@ constexpr int kThreads = 256;
 // whole lines, tightly packed vertices by way of shared memory.  Bound by the
 // link: 38 MB of numpy arrays in 186 us (205 GB/s); copied to the device first
 // 210 + 10 us, and the load 890 us instead of 824.
-constexpr uint32_t kPackTile = 4 * kThreads;  // vertices of a block's step (12-byte stride)
-
-__global__ void __launch_bounds__(kThreads)
-    k_read_inputs(const uint8_t* raw, uint64_t stride, uint32_t n, float4* out, const uint32_t* idxSrc, uint32_t* idx,
-                  uint64_t nIdx, float4* partial, uint32_t* done, BuildParams* params, int cubic, int reset)
+//
+// read_part: block `block` of `blocks` of THREADS threads takes its part of
+// the vertices to out and to their bounds, its part of the indices to idx.
+// sRaw: 3 * THREADS float4 of shared memory.
+template <int THREADS>
+__device__ __forceinline__ void read_part(const uint8_t* raw, uint64_t stride, uint32_t n, float4* out,
+                                          const uint32_t* idxSrc, uint32_t* idx, uint64_t nIdx, uint32_t block,
+                                          uint32_t blocks, float4* sRaw, float (&mn)[4], float (&mx)[4])
 {
-  float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
+  constexpr uint32_t kTile = 4 * THREADS;  // vertices of a step (12-byte stride)
   auto take = [&](uint32_t i, float x, float y, float z) {
     const float v[4] = {x, y, z, 1.0f};
     out[i] = make_float4(x, y, z, 1.0f);
@@ -51,26 +54,25 @@ __global__ void __launch_bounds__(kThreads)
   const bool aligned = (reinterpret_cast<uintptr_t>(raw) & 15u) == 0u;
   if (stride == 12 && aligned)
   {
-    __shared__ float4 s_raw[3 * kThreads];
-    for (uint64_t v0 = (uint64_t)blockIdx.x * kPackTile; v0 < n; v0 += (uint64_t)gridDim.x * kPackTile)
+    for (uint64_t v0 = (uint64_t)block * kTile; v0 < n; v0 += (uint64_t)blocks * kTile)
     {
-      const uint32_t count = (uint32_t)min((uint64_t)kPackTile, n - v0);
+      const uint32_t count = (uint32_t)min((uint64_t)kTile, n - v0);
       const uint32_t pieces = 3 * count / 4;  // whole 16-byte pieces
       const float4* src = reinterpret_cast<const float4*>(raw + 12 * v0);
 #pragma unroll
       for (int q = 0; q < 3; q++)
       {
-        const uint32_t k = q * kThreads + threadIdx.x;
-        if (k < pieces) s_raw[k] = src[k];
+        const uint32_t k = q * THREADS + threadIdx.x;
+        if (k < pieces) sRaw[k] = src[k];
       }
-      float* words = reinterpret_cast<float*>(s_raw);
+      float* words = reinterpret_cast<float*>(sRaw);
       if (threadIdx.x < 3 * count - 4 * pieces)
         words[4 * pieces + threadIdx.x] = reinterpret_cast<const float*>(src)[4 * pieces + threadIdx.x];
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < 4; q++)
       {
-        const uint32_t k = q * kThreads + threadIdx.x;
+        const uint32_t k = q * THREADS + threadIdx.x;
         if (k < count) take((uint32_t)(v0 + k), words[3 * k], words[3 * k + 1], words[3 * k + 2]);
       }
       __syncthreads();
@@ -78,48 +80,59 @@ __global__ void __launch_bounds__(kThreads)
   }
   else if (stride == 16 && aligned)
   {
-    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+    for (uint32_t i = block * THREADS + threadIdx.x; i < n; i += blocks * THREADS)
     {
       const float4 p = reinterpret_cast<const float4*>(raw)[i];
       take(i, p.x, p.y, p.z);
     }
   }
   else
-    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads)
+    for (uint32_t i = block * THREADS + threadIdx.x; i < n; i += blocks * THREADS)
     {
       const float* p = reinterpret_cast<const float*>(raw + (size_t)i * stride);
       take(i, p[0], p[1], p[2]);
     }
   if (idxSrc != idx)
   {
-    const uint64_t step = (uint64_t)gridDim.x * kThreads, first = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    const uint64_t step = (uint64_t)blocks * THREADS, first = (uint64_t)block * THREADS + threadIdx.x;
     const uint64_t whole = (reinterpret_cast<uintptr_t>(idxSrc) & 15u) == 0u ? nIdx / 4 : 0;  // idx starts an allocation
 #pragma unroll 4
     for (uint64_t k = first; k < whole; k += step)
       reinterpret_cast<uint4*>(idx)[k] = reinterpret_cast<const uint4*>(idxSrc)[k];
     for (uint64_t k = 4 * whole + first; k < nIdx; k += step) idx[k] = idxSrc[k];
   }
-  __shared__ float smn[kThreads / 32][4], smx[kThreads / 32][4];
-  __shared__ bool  s_last;
+}
+
+// The bounds of a block's threads to thread 0.
+template <int THREADS> __device__ __forceinline__ void block_bounds(float (&mn)[4], float (&mx)[4])
+{
+  __shared__ float smn[THREADS / 32][4], smx[THREADS / 32][4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // the block's bounds to thread 0
-  auto combine = [&]() {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+  for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int k = 0; k < 4; k++)
-      {
-        mn[k] = lm_min(mn[k], __shfl_down_sync(0xFFFFFFFFu, mn[k], o));
-        mx[k] = lm_max(mx[k], __shfl_down_sync(0xFFFFFFFFu, mx[k], o));
-      }
-    if (lane == 0)
-      for (int k = 0; k < 4; k++) { smn[warp][k] = mn[k]; smx[warp][k] = mx[k]; }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 1; w < kThreads / 32; w++)
-        for (int k = 0; k < 4; k++) { mn[k] = lm_min(mn[k], smn[w][k]); mx[k] = lm_max(mx[k], smx[w][k]); }
-  };
-  combine();
+    for (int k = 0; k < 4; k++)
+    {
+      mn[k] = lm_min(mn[k], __shfl_down_sync(0xFFFFFFFFu, mn[k], o));
+      mx[k] = lm_max(mx[k], __shfl_down_sync(0xFFFFFFFFu, mx[k], o));
+    }
+  if (lane == 0)
+    for (int k = 0; k < 4; k++) { smn[warp][k] = mn[k]; smx[warp][k] = mx[k]; }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < THREADS / 32; w++)
+      for (int k = 0; k < 4; k++) { mn[k] = lm_min(mn[k], smn[w][k]); mx[k] = lm_max(mx[k], smx[w][k]); }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    k_read_inputs(const uint8_t* raw, uint64_t stride, uint32_t n, float4* out, const uint32_t* idxSrc, uint32_t* idx,
+                  uint64_t nIdx, float4* partial, uint32_t* done, BuildParams* params, int cubic, int reset)
+{
+  float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
+  __shared__ float4 s_raw[3 * kThreads];
+  __shared__ bool   s_last;
+  read_part<kThreads>(raw, stride, n, out, idxSrc, idx, nIdx, blockIdx.x, gridDim.x, s_raw, mn, mx);
+  block_bounds<kThreads>(mn, mx);
   if (threadIdx.x == 0)
   {
     partial[2 * blockIdx.x + 0] = make_float4(mn[0], mn[1], mn[2], mn[3]);
@@ -135,7 +148,7 @@ __global__ void __launch_bounds__(kThreads)
     mn[0] = lm_min(mn[0], a.x); mn[1] = lm_min(mn[1], a.y); mn[2] = lm_min(mn[2], a.z); mn[3] = lm_min(mn[3], a.w);
     mx[0] = lm_max(mx[0], c.x); mx[1] = lm_max(mx[1], c.y); mx[2] = lm_max(mx[2], c.z); mx[3] = lm_max(mx[3], c.w);
   }
-  combine();
+  block_bounds<kThreads>(mn, mx);
   if (threadIdx.x != 0) return;
   bc::zindex_scale(mn, mx, params, cubic);
   if (reset)
@@ -251,7 +264,7 @@ __global__ void __launch_bounds__(kThreads) k_karras(const uint32_t* __restrict_
     if (!active) continue;
     uint32_t left, right;
     int other;
-    bc::karras_node(codes, L, i, ci, dPrev, dNext, left, right, other);
+    bc::karras_node(bc::GlobalCodes{codes}, L, i, ci, dPrev, dNext, left, right, other);
     lr[i].leftOffset = left;
     lr[i].escapeIndex = right;
     parent[left] = (uint32_t)i;
@@ -301,6 +314,149 @@ __global__ void __launch_bounds__(kThreads) k_records(BuildParams* __restrict__ 
     r.c = make_float4(b.boxMin[2], b.boxMax[0], b.boxMax[1], b.boxMax[2]);
     r.d = make_uint4(lref, rref, 0u, 0u);
     recs[i] = r;
+  }
+}
+
+// ---------------------------------------------------------------- small geometries
+// Inputs, box, codes, sort, runs and hierarchy of a geometry of at most
+// kSmallTris triangles in one block: the arrays that the kernels above would
+// write.  Each of those nine launches is shorter than the gap before it.  The
+// sort is a bitonic one of (code, triangle) pairs, which are distinct, so its
+// order is the stable one by code; steps within 64 pairs stay inside a warp.
+// Bound by the block's chain of steps, so the gain goes as the geometry grows:
+// a load of 512 triangles 147 us with one kernel a stage, 92 so; of 2,000 171
+// and 132, of 4,096 186 and 178.  The commit of 240 instances, whose tree is
+// such a geometry: 173 us, 97 so.
+constexpr int      kSmallThreads = 512;
+constexpr uint32_t kSmallTris = 4096, kSmallVerts = 3 * kSmallTris;
+
+__global__ void __launch_bounds__(kSmallThreads) k_small_front(BuildBuffers b, uint32_t* openCount)
+{
+  __shared__ union __align__(16)
+  {
+    float4             raw[3 * kSmallThreads];
+    unsigned long long pair[kSmallTris];
+    uint32_t           code[kSmallTris];
+  } sh;
+  __shared__ BuildParams s_params;
+  __shared__ uint32_t    s_warpRuns[kSmallThreads / 32];
+  const uint32_t N = b.nTris, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+
+  float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
+  read_part<kSmallThreads>(b.raw, b.rawStride, b.nVerts, b.verts, b.idxSrc, b.idx, 3 * (uint64_t)N, 0u, 1u, sh.raw, mn,
+                           mx);
+  block_bounds<kSmallThreads>(mn, mx);
+  if (tid == 0)
+  {
+    bc::zindex_scale(mn, mx, &s_params, b.mortonCubic);
+    s_params.nLeaves = s_params.error = s_params.rootRecord = s_params.pad = 0;
+    *openCount = 0;
+  }
+  __syncthreads();
+
+  // codes, padded to a power of two
+  uint32_t P = 64;
+  while (P < N) P <<= 1;
+  for (uint32_t i = tid; i < P; i += kSmallThreads)
+  {
+    if (i >= N)
+    {
+      sh.pair[i] = ~0ull;
+      continue;
+    }
+    uint32_t ia = b.idx[3 * i], ib = b.idx[3 * i + 1], ic = b.idx[3 * i + 2];
+    if (ia >= b.nVerts || ib >= b.nVerts || ic >= b.nVerts)
+    {
+      atomicOr(&s_params.error, kErrIndexRange);
+      ia = ib = ic = 0;
+    }
+    const uint32_t code = bc::morton_code(b.verts[ia], b.verts[ib], b.verts[ic], N, s_params.bmin, s_params.scale);
+    b.keysUnsorted[i] = code;
+    sh.pair[i] = (unsigned long long)code << 32 | i;
+  }
+  __syncthreads();
+
+  for (uint32_t k = 2; k <= P; k <<= 1)
+    for (uint32_t j = k >> 1; j > 0; j >>= 1)
+    {
+      for (uint32_t p = tid; p < P / 2; p += kSmallThreads)
+      {
+        const uint32_t i = 2 * p - (p & (j - 1));
+        const unsigned long long x = sh.pair[i], y = sh.pair[i + j];
+        if ((x > y) == ((i & k) == 0))
+        {
+          sh.pair[i] = y;
+          sh.pair[i + j] = x;
+        }
+      }
+      // a step within 64 pairs, before another such one, is the warp's own
+      if (j > 32 || (j == 1 && k > 32)) __syncthreads();
+      else __syncwarp();
+    }
+  __syncthreads();
+
+  // runs: a warp's codes are consecutive
+  constexpr int kPer = kSmallTris / kSmallThreads;
+  uint32_t code[kPer], starts[kPer], runs = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+  {
+    const uint32_t i = (warp * kPer + q) * 32 + lane;
+    code[q] = 0;
+    bool start = false;
+    if (i < N)
+    {
+      const unsigned long long x = sh.pair[i];
+      code[q] = (uint32_t)(x >> 32);
+      b.keys[i] = code[q];
+      b.vals[i] = (uint32_t)x;
+      start = i == 0 || (uint32_t)(sh.pair[i - 1] >> 32) != code[q];
+    }
+    starts[q] = __ballot_sync(0xFFFFFFFFu, start);
+    runs += __popc(starts[q]);
+  }
+  if (lane == 0) s_warpRuns[warp] = runs;
+  __syncthreads();
+  uint32_t at = 0, L = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kSmallThreads / 32; w++)
+  {
+    at += w < warp ? s_warpRuns[w] : 0u;
+    L += s_warpRuns[w];
+  }
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+  {
+    if ((starts[q] >> lane) & 1u)
+    {
+      const uint32_t r = at + __popc(starts[q] & ((1u << lane) - 1u));
+      sh.code[r] = code[q];
+      b.compressed[r] = code[q];
+      b.runStarts[r] = (warp * kPer + q) * 32 + lane;
+    }
+    at += __popc(starts[q]);
+  }
+  __syncthreads();
+
+  const bc::SharedCodes codes{sh.code};
+  for (int i = (int)tid; i < (int)L - 1; i += kSmallThreads)
+  {
+    const uint32_t ci = codes[i];
+    uint32_t left, right;
+    int other;
+    bc::karras_node(codes, (int)L, i, ci, bc::karras_delta(codes, (int)L, ci, i - 1),
+                    bc::karras_delta(codes, (int)L, ci, i + 1), left, right, other);
+    b.lr[i].leftOffset = left;
+    b.lr[i].escapeIndex = right;
+    b.parent[left] = (uint32_t)i;
+    b.parent[right] = (uint32_t)i;
+    b.visit[N + i] = (uint32_t)other;
+    b.visit[i] = 0u;
+  }
+  if (tid == 0)
+  {
+    s_params.nLeaves = L;
+    *b.params = s_params;
   }
 }
 
@@ -357,14 +513,19 @@ cudaError_t read_inputs(const BuildBuffers& b, float4* partial, uint32_t* done, 
   return cudaGetLastError();
 }
 
-// Leaves, hierarchy, boxes and (binary layout) pair records, from the sorted
-// triangles and the unique codes.  open: nTris words of scratch; *openCount is
-// zero before.
+cudaError_t hierarchy(const BuildBuffers& b, int numSMs, cudaStream_t s)
+{
+  k_karras<<<grid_for(b.nTris, numSMs, 8), kThreads, 0, s>>>(b.compressed, b.params, b.lr, b.parent, b.visit,
+                                                             b.visit + b.nTris);
+  return cudaGetLastError();
+}
+
+// Leaves, boxes and (binary layout) pair records, from the sorted triangles,
+// the unique codes and the hierarchy.  open: nTris words of scratch;
+// *openCount is zero before.
 cudaError_t build_tree(const BuildBuffers& b, uint32_t* open, uint32_t* openCount, int numSMs, cudaStream_t s)
 {
   const uint32_t N = b.nTris;
-  const uint32_t g = grid_for(N, numSMs, 8);
-  k_karras<<<g, kThreads, 0, s>>>(b.compressed, b.params, b.lr, b.parent, b.visit, b.visit + N);
   bc::LeafTree t = {};
   t.verts = b.verts;
   t.idx = b.idx;
@@ -385,8 +546,9 @@ cudaError_t build_tree(const BuildBuffers& b, uint32_t* open, uint32_t* openCoun
   t.vertexRecords = b.vertexRecords;
   t.params = b.params;
   bc::k_leaf_tree<false><<<(N + bc::kSlice - 1) / bc::kSlice, bc::kSlice, 0, s>>>(t);
-  bc::k_climb<false><<<bc::climb_blocks(N, numSMs), 128, 0, s>>>(t);
-  if (b.recs) k_records<<<g, kThreads, 0, s>>>(b.params, b.lr, b.visit, b.runStarts, b.recs);
+  // no walk leaves a single slice
+  if (N > bc::kSlice) bc::k_climb<false><<<bc::climb_blocks(N, numSMs), 128, 0, s>>>(t);
+  if (b.recs) k_records<<<grid_for(N, numSMs, 8), kThreads, 0, s>>>(b.params, b.lr, b.visit, b.runStarts, b.recs);
   return cudaGetLastError();
 }
 }  // namespace
@@ -399,6 +561,13 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   if (N == 0) return cudaSuccess;
   const BuildScratch q = build_scratch(b.scratch, N);
   uint32_t* err = &b.params->error;
+  if (N <= kSmallTris && b.nVerts <= kSmallVerts)
+  {
+    k_small_front<<<1, kSmallThreads, 0, s>>>(b, q.boxDone + 2);
+    const cudaError_t se = cudaGetLastError();
+    if (se != cudaSuccess) return se;
+    return build_tree(b, b.keysAlt, q.boxDone + 2, numSMs, s);
+  }
   cudaError_t e = cudaMemsetAsync(b.scratch, 0, q.zeroBytes, s);
   if (e != cudaSuccess) return e;
   // 1. inputs, scene box and Morton scale
@@ -414,7 +583,9 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   // 4. unique codes and run starts
   k_compact_runs<<<(N + kScanTile - 1) / kScanTile, kThreads, 0, s>>>(b.keys, N, b.compressed, b.runStarts, q.scanStatus,
                                                                       q.scanCounter, b.params, err);
-  // 5. leaves, hierarchy, boxes, records; the sort's spare array holds the open walks
+  // 5. hierarchy, leaves, boxes, records; the sort's spare array holds the open walks
+  e = hierarchy(b, numSMs, s);
+  if (e != cudaSuccess) return e;
   return build_tree(b, b.keysAlt, q.boxDone + 2, numSMs, s);
 }
 
@@ -432,6 +603,7 @@ cudaError_t refit_lbvh(const BuildBuffers& b, BuildParams* boxOut, int numSMs, c
   uint32_t* open = (uint32_t*)(partial + 2 * kBoxBlocks);
   cudaError_t e = cudaMemsetAsync(done, 0, 2 * sizeof(uint32_t), s);
   if (e == cudaSuccess) e = read_inputs(b, partial, done, boxOut, 0, numSMs, s);
+  if (e == cudaSuccess) e = hierarchy(b, numSMs, s);
   if (e != cudaSuccess) return e;
   return build_tree(b, open, done + 1, numSMs, s);
 }

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kThreads) k_seg_karras(const uint32_t* __restr
     if (!active) continue;
     uint32_t left, right;
     int other;
-    bc::karras_node(compressed + leafOffsets[s], L, i, ci, dPrev, dNext, left, right, other);
+    bc::karras_node(bc::GlobalCodes{compressed + leafOffsets[s]}, L, i, ci, dPrev, dNext, left, right, other);
     const uint32_t nb = nodeOffsets[s];
     lr[nb + i].leftOffset = left;
     lr[nb + i].escapeIndex = right;

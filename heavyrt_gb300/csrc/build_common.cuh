@@ -118,20 +118,30 @@ __device__ __forceinline__ void zindex_scale(const float* mn, const float* mx, B
   }
 }
 
-// delta() of core/builders/lbvh.cpp:386-403 against a code held in a
-// register: the codes are unique after compaction, so this is the count of
-// leading zeros of their XOR (32 for equal codes, -1 out of range).
-__device__ __forceinline__ int karras_delta(const uint32_t* __restrict__ c, int L, uint32_t ci, int j)
-{
-  if (j < 0 || j >= L) return -1;
-  const uint32_t x = ci ^ __ldg(c + j);
-  return x == 0u ? 32 : __clz(x);
-}
-
 __device__ __forceinline__ int clz_delta(uint32_t a, uint32_t b)
 {
   const uint32_t x = a ^ b;
   return x == 0u ? 32 : __clz(x);
+}
+
+// A tree's unique codes: written by an earlier kernel, or in shared memory.
+struct GlobalCodes
+{
+  const uint32_t* c;
+  __device__ __forceinline__ uint32_t operator[](int j) const { return __ldg(c + j); }
+};
+struct SharedCodes
+{
+  const uint32_t* c;
+  __device__ __forceinline__ uint32_t operator[](int j) const { return c[j]; }
+};
+
+// delta() of core/builders/lbvh.cpp:386-403 against a code held in a
+// register: the codes are unique after compaction, so this is the count of
+// leading zeros of their XOR (32 for equal codes, -1 out of range).
+template <typename Codes> __device__ __forceinline__ int karras_delta(const Codes& c, int L, uint32_t ci, int j)
+{
+  return j < 0 || j >= L ? -1 : clz_delta(ci, c[j]);
 }
 
 // Node i's code and its neighbours' deltas, exchanged across the warp: lane l
@@ -163,8 +173,9 @@ __device__ __forceinline__ void karras_neighbours(const uint32_t* __restrict__ a
 // range end by exponential then binary search, the split by binary search;
 // children in the LR numbering (internal 0..L-2, leaves L-1..2L-2), `other` =
 // the far end of the node's leaf range.
-__device__ __forceinline__ void karras_node(const uint32_t* __restrict__ c, int L, int i, uint32_t ci, int dPrev,
-                                            int dNext, uint32_t& left, uint32_t& right, int& other)
+template <typename Codes>
+__device__ __forceinline__ void karras_node(const Codes& c, int L, int i, uint32_t ci, int dPrev, int dNext,
+                                            uint32_t& left, uint32_t& right, int& other)
 {
   const int dl = dNext - dPrev;
   const int d = (dl > 0) - (dl < 0);

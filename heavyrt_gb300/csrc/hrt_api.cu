@@ -622,7 +622,7 @@ void instance_world_box(const Geom& g, const float* m, float* mn, float* mx)
 // per instance (min corner, max corner, max corner) whose box is the
 // instance's world box, built by the geometry LBVH build in the binary
 // layout.  Triangle record e1.w (the pseudo-triangle's index) is rewritten to
-// the instance id.  Leaves may hold more than 127 instances (coincident
+// the instance id where they differ.  Leaves may hold more than 127 instances (coincident
 // instances share a Morton code): the traversal ends a leaf at its flagged
 // record, so only the exported LR leaf count would overflow.
 int build_tlas(hrt_scene* s)
@@ -653,6 +653,7 @@ int build_tlas(hrt_scene* s)
       s->tlas.nLeaves <= n)
     st = HRT_OK;
   if (st != HRT_OK) return st;
+  if (ids.back() + 1 == n) return HRT_OK;  // every instance has triangles: pseudo-triangle k is instance k
   std::vector<TriRec> tr(n);
   HRT_CUDA(s->ctx, cudaMemcpy(tr.data(), s->tlas.tris, sizeof(TriRec) * n, cudaMemcpyDeviceToHost));
   for (TriRec& r : tr)
