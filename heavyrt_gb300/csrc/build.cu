@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kThreads) k_records(BuildParams* __restrict__ 
 constexpr int      kSmallThreads = 512;
 constexpr uint32_t kSmallTris = 4096, kSmallVerts = 3 * kSmallTris;
 
-__global__ void __launch_bounds__(kSmallThreads) k_small_front(BuildBuffers b, uint32_t* openCount)
+__global__ void __launch_bounds__(kSmallThreads) k_small_front(BuildBuffers b)
 {
   __shared__ union __align__(16)
   {
@@ -350,7 +350,6 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_front(BuildBuffers b, u
   {
     bc::zindex_scale(mn, mx, &s_params, b.mortonCubic);
     s_params.nLeaves = s_params.error = s_params.rootRecord = s_params.pad = 0;
-    *openCount = 0;
   }
   __syncthreads();
 
@@ -521,9 +520,8 @@ cudaError_t hierarchy(const BuildBuffers& b, int numSMs, cudaStream_t s)
 }
 
 // Leaves, boxes and (binary layout) pair records, from the sorted triangles,
-// the unique codes and the hierarchy.  open: nTris words of scratch;
-// *openCount is zero before.
-cudaError_t build_tree(const BuildBuffers& b, uint32_t* open, uint32_t* openCount, int numSMs, cudaStream_t s)
+// the unique codes and the hierarchy.  lists: build_list_words() of scratch.
+cudaError_t build_tree(const BuildBuffers& b, uint32_t* lists, int numSMs, cudaStream_t s)
 {
   const uint32_t N = b.nTris;
   bc::LeafTree t = {};
@@ -540,19 +538,18 @@ cudaError_t build_tree(const BuildBuffers& b, uint32_t* open, uint32_t* openCoun
   t.parent = b.parent;
   t.visit = b.visit;
   t.rangeEnd = b.visit + N;
-  t.open = open;
-  t.openCount = openCount;
+  t.lists = lists;
   t.errorWord = &b.params->error;
   t.vertexRecords = b.vertexRecords;
   t.params = b.params;
-  bc::k_leaf_tree<false><<<(N + bc::kSlice - 1) / bc::kSlice, bc::kSlice, 0, s>>>(t);
-  // no walk leaves a single slice
-  if (N > bc::kSlice) bc::k_climb<false><<<bc::climb_blocks(N, numSMs), 128, 0, s>>>(t);
+  const cudaError_t e = bc::leaf_tree<false>(t, s);
+  if (e != cudaSuccess) return e;
   if (b.recs) k_records<<<grid_for(N, numSMs, 8), kThreads, 0, s>>>(b.params, b.lr, b.visit, b.runStarts, b.recs);
   return cudaGetLastError();
 }
 }  // namespace
 
+size_t build_list_words(uint32_t nTris) { return bc::list_words(nTris); }
 size_t build_scratch_bytes(uint32_t nTris) { return build_scratch(nullptr, nTris).bytes; }
 
 cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
@@ -563,10 +560,10 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   uint32_t* err = &b.params->error;
   if (N <= kSmallTris && b.nVerts <= kSmallVerts)
   {
-    k_small_front<<<1, kSmallThreads, 0, s>>>(b, q.boxDone + 2);
+    k_small_front<<<1, kSmallThreads, 0, s>>>(b);
     const cudaError_t se = cudaGetLastError();
     if (se != cudaSuccess) return se;
-    return build_tree(b, b.keysAlt, q.boxDone + 2, numSMs, s);
+    return build_tree(b, b.keysAlt, numSMs, s);
   }
   cudaError_t e = cudaMemsetAsync(b.scratch, 0, q.zeroBytes, s);
   if (e != cudaSuccess) return e;
@@ -583,10 +580,10 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   // 4. unique codes and run starts
   k_compact_runs<<<(N + kScanTile - 1) / kScanTile, kThreads, 0, s>>>(b.keys, N, b.compressed, b.runStarts, q.scanStatus,
                                                                       q.scanCounter, b.params, err);
-  // 5. hierarchy, leaves, boxes, records; the sort's spare array holds the open walks
+  // 5. hierarchy, leaves, boxes, records; the sort's spare array holds the lists
   e = hierarchy(b, numSMs, s);
   if (e != cudaSuccess) return e;
-  return build_tree(b, b.keysAlt, q.boxDone + 2, numSMs, s);
+  return build_tree(b, b.keysAlt, numSMs, s);
 }
 
 // Refit: the geometry's vertices moved, its triangles and their sorted order
@@ -598,16 +595,15 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
 cudaError_t refit_lbvh(const BuildBuffers& b, BuildParams* boxOut, int numSMs, cudaStream_t s)
 {
   if (b.nTris == 0) return cudaSuccess;
-  uint32_t* done = (uint32_t*)b.scratch;  // refit_scratch_bytes(): counters, box parts, open walks
+  uint32_t* done = (uint32_t*)b.scratch;  // refit_scratch_bytes(): a counter, box parts, lists
   float4* partial = (float4*)((char*)b.scratch + 256);
-  uint32_t* open = (uint32_t*)(partial + 2 * kBoxBlocks);
-  cudaError_t e = cudaMemsetAsync(done, 0, 2 * sizeof(uint32_t), s);
+  cudaError_t e = cudaMemsetAsync(done, 0, sizeof(uint32_t), s);
   if (e == cudaSuccess) e = read_inputs(b, partial, done, boxOut, 0, numSMs, s);
   if (e == cudaSuccess) e = hierarchy(b, numSMs, s);
   if (e != cudaSuccess) return e;
-  return build_tree(b, open, done + 1, numSMs, s);
+  return build_tree(b, (uint32_t*)(partial + 2 * kBoxBlocks), numSMs, s);
 }
 
-size_t refit_scratch_bytes(uint32_t nTris) { return 256 + 2 * sizeof(float4) * kBoxBlocks + 4 * (size_t)nTris; }
+size_t refit_scratch_bytes(uint32_t nTris) { return 256 + 2 * sizeof(float4) * kBoxBlocks + 4 * build_list_words(nTris); }
 
 }  // namespace hrt

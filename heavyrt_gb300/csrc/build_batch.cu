@@ -441,8 +441,7 @@ cudaError_t build_lbvh_batch(const BatchBuffers& b, int numSMs, cudaStream_t s)
   t.parent = b.parent;
   t.visit = b.visit;
   t.rangeEnd = b.visit + N;
-  t.open = b.keysAlt;  // free after the sort
-  t.openCount = scanCounter + 1;
+  t.lists = b.keysAlt;  // free after the sort
   t.errorWord = b.errorWord;
   t.vertexRecords = b.vertexRecords;
   t.vertOffsets = b.vertOffsets;
@@ -454,8 +453,8 @@ cudaError_t build_lbvh_batch(const BatchBuffers& b, int numSMs, cudaStream_t s)
   t.counts = b.counts;
   t.G = G;
   t.recs = b.recs;
-  bc::k_leaf_tree<true><<<(N + bc::kSlice - 1) / bc::kSlice, bc::kSlice, 0, s>>>(t);
-  bc::k_climb<true><<<bc::climb_blocks(N, numSMs), 128, 0, s>>>(t);
+  e = bc::leaf_tree<true>(t, s);
+  if (e != cudaSuccess) return e;
   k_seg_records<<<g, kThreads, 0, s>>>(b.triOffsets, b.leafOffsets, b.intOffsets, b.nodeOffsets, b.recOffsets, G,
                                        b.counts, b.lr, b.runStarts, b.visit, b.recs, b.errorWord);
   k_seg_localize<<<g, kThreads, 0, s>>>(b.triOffsets, b.leafOffsets, G, N, b.counts, b.runStarts, b.vals);

@@ -195,7 +195,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   if (layout == HRT_LAYOUT_BVH2) HRT_CUDA(ctx, dalloc(&g.recs, N > 1 ? N - 1 : 1, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.tris, N, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.sortedIdx, 3 * (size_t)N, bytes, st));
-  HRT_CUDA(ctx, cudaMallocAsync((void**)&keysAlt, sizeof(uint32_t) * N, st));
+  HRT_CUDA(ctx, cudaMallocAsync((void**)&keysAlt, sizeof(uint32_t) * std::max<size_t>(N, build_list_words(N)), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&valsAlt, sizeof(uint32_t) * N, st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&parent, sizeof(uint32_t) * (2 * (size_t)N - 1), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&visit, sizeof(uint32_t) * 2 * (size_t)N, st));
@@ -427,7 +427,7 @@ int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geo
   HRT_CUDA(ctx, cudaMemsetAsync(offs, 0, sizeof(uint32_t) * (4 * ((size_t)G + 1) + 8), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&dIdx, sizeof(uint32_t) * 3 * (N ? N : 1), st));
   b.idx = dIdx;
-  HRT_CUDA(ctx, cudaMallocAsync((void**)&keysAlt, sizeof(uint32_t) * (N ? N : 1), st));
+  HRT_CUDA(ctx, cudaMallocAsync((void**)&keysAlt, sizeof(uint32_t) * std::max<size_t>({1, N, build_list_words(N)}), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&valsAlt, sizeof(uint32_t) * (N ? N : 1), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&parent, sizeof(uint32_t) * 2 * (N ? N : 1), st));
   HRT_CUDA(ctx, cudaMallocAsync((void**)&visit, sizeof(uint32_t) * 2 * (N ? N : 1), st));

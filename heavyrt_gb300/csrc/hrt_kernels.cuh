@@ -42,7 +42,7 @@ struct BuildBuffers
   // stage arrays (device)
   uint32_t*  keys;            // nTris: Morton codes, sorted in place
   uint32_t*  vals;            // nTris: triangle ids, sorted in place
-  uint32_t*  keysAlt;         // nTris: sort ping-pong
+  uint32_t*  keysAlt;         // nTris, build_list_words() at least: sort ping-pong, then the walks' lists
   uint32_t*  valsAlt;         // nTris
   uint32_t*  keysUnsorted;    // nTris: copy of the codes before the sort (export)
   uint32_t*  compressed;      // nTris (L used): unique codes
@@ -59,6 +59,7 @@ struct BuildBuffers
   int        vertexRecords = 0;  // 1: triangle records hold {A, B, C} (watertight test), else {A, B-A, C-A}
   int        mortonCubic = 0;    // 1: one Morton scale for x, y, z (that of the longest axis)
 };
+size_t build_list_words(uint32_t nTris);
 size_t build_scratch_bytes(uint32_t nTris);
 // Runs the whole LBVH build asynchronously on `stream`.  Errors found on the
 // device are ORed into params->error.
@@ -97,7 +98,7 @@ struct BatchBuffers
   uint32_t        nTris;        // triOffsets[G]
   uint32_t*  keys;              // nTris
   uint32_t*  vals;              // nTris: global triangle ids in sorted order
-  uint32_t*  keysAlt;           // nTris
+  uint32_t*  keysAlt;           // nTris, build_list_words() at least
   uint32_t*  valsAlt;           // nTris
   uint32_t*  keysUnsorted;      // nTris
   uint32_t*  compressed;        // nTris

@@ -18,15 +18,15 @@
 // in (left, right) order, count = children's counts + 2.  An internal node i of
 // a Karras tree has i as one end of its leaf range, so the nodes whose range
 // lies inside the slice are among i in [lo, hi - 1): their links, boxes and
-// arrival counters are in shared memory (acquire-release at block scope).  Only
-// the nodes whose range leaves the slice use the device-wide counters
-// (acquire-release at device scope, children read from L2).  Every node a
-// thread reads was written by the thread that released the counter it acquired.
+// arrival counters are in shared memory (acquire-release at block scope).  The
+// nodes whose range leaves the slice are left to k_climb.  Every node a thread
+// reads was written by the thread that released the counter it acquired, or by
+// an earlier kernel.
 //
 // What bounds it: the walks are chains of dependent steps and the leaves are
 // gathers and AoS writes.  As a kernel of leaves, a thread per leaf with its own 48-byte
 // stores, and one of walks with links and boxes read from L2, the 2M-triangle
-// heightfield took 93 + 107 us; in one kernel 153; in these two 97 + 41.
+// heightfield took 93 + 107 us; in one kernel 153; in this one and k_climb 101 + 32.
 #pragma once
 
 #include "build_common.cuh"
@@ -37,6 +37,46 @@ namespace bc
 {
 
 constexpr uint32_t kSlice = 512;  // leaves, threads and triangles of a chunk
+// k_climb: a group is kFan slices, or kFan groups of the tier below.  Each
+// slice or group hands at most kEdge nodes of either list to the next tier: a
+// range of leaves of a tree at most 31 levels deep is covered by 62 nodes, and
+// at most 62 ancestors of its ends have an index in it and leave it.
+constexpr uint32_t kFan = 32, kEdge = 64, kSlots = kFan * kEdge;
+constexpr int      kClimbThreads = 1024;
+
+constexpr uint32_t kSlotMark = 0x80000000u;  // of a slot in visit; a root's visit ends as 2
+constexpr uint32_t kNone = 0xFFFFFFFFu;
+
+// Where tier t's lists are: `producers` slices (t = 0) or groups, each with
+// kEdge open nodes (outermost finished ones: {LR index, parent | kUpRight of a
+// right child}), kEdge leaving nodes (LR index, the far end of its range, parent
+// as above) and a word of both counts.
+constexpr uint32_t kUpRight = 0x80000000u;
+struct TierLists
+{
+  uint2*    open;
+  uint32_t *leaving, *end, *up, *counts;
+  uint32_t  producers;
+};
+__host__ __device__ inline TierLists tier_lists(uint32_t* lists, uint32_t nTris, int tier)
+{
+  uint32_t producers = (nTris + kSlice - 1) / kSlice;
+  for (int t = 0; t < tier; t++)
+  {
+    lists += (5 * kEdge + 2) * (size_t)producers;
+    producers = (producers + kFan - 1) / kFan;
+  }
+  const size_t n = kEdge * (size_t)producers;
+  return {reinterpret_cast<uint2*>(lists), lists + 2 * n, lists + 3 * n, lists + 4 * n, lists + 5 * n, producers};
+}
+// Words of all of a build's lists.
+inline size_t list_words(uint32_t nTris)
+{
+  size_t words = 0;
+  for (uint32_t producers = (nTris + kSlice - 1) / kSlice; producers > 1; producers = (producers + kFan - 1) / kFan)
+    words += (5 * kEdge + 2) * (size_t)producers;
+  return words;
+}
 
 struct LeafTree
 {
@@ -53,8 +93,7 @@ struct LeafTree
   const uint32_t* parent;
   uint32_t*       visit;
   const uint32_t* rangeEnd;
-  uint32_t*       open;       // LR indices of the outermost finished nodes of the slices
-  uint32_t*       openCount;  // zero before
+  uint32_t*       lists;  // list_words() of scratch, 8-byte aligned: tier_lists()
   uint32_t*       errorWord;
   int             vertexRecords;
   // one geometry: its leaf count
@@ -115,6 +154,9 @@ __global__ void __launch_bounds__(kSlice, 3) k_leaf_tree(LeafTree a)
   const uint32_t hi = min(lo + kSlice, Ltot);
   const uint32_t tid = threadIdx.x, g = lo + tid;
   const bool active = g < hi;
+  __shared__ uint32_t s_open, s_leaving;
+  const TierLists out = tier_lists(a.lists, a.nTris, 0);
+  if (tid == 0) s_open = s_leaving = 0u;
 
   // the leaf's geometry: first leaf, triangle, LR node and internal node, leaf count
   uint32_t lb = 0, tb = 0, te = a.nTris, nb = 0, ib = 0, L = Ltot, seg = 0;
@@ -239,6 +281,21 @@ __global__ void __launch_bounds__(kSlice, 3) k_leaf_tree(LeafTree a)
         sh.t.rangeEnd[tid] = a.rangeEnd[ib + k];
         sh.t.left[tid] = a.lr[nb + k].leftOffset;
         sh.t.right[tid] = a.lr[nb + k].escapeIndex;
+        const uint32_t j = sh.t.rangeEnd[tid];
+        if (min(k, j) + lb < lo || max(k, j) + lb >= hi)  // a node that leaves the slice
+        {
+          const uint32_t e = atomicAdd(&s_leaving, 1u);
+          if (e < kEdge)
+          {
+            const size_t at = kEdge * (size_t)blockIdx.x + e;
+            out.leaving[at] = nb + k;
+            out.end[at] = j;
+            out.up[at] = k ? sh.t.nodeParent[tid] | (a.lr[nb + sh.t.nodeParent[tid]].escapeIndex == k ? kUpRight : 0u) : 0u;
+            a.visit[ib + k] = kSlotMark | (kEdge * (blockIdx.x % kFan) + e);
+          }
+          else
+            atomicOr(a.errorWord, kErrLayout);
+        }
       }
     }
     if (SEG && L == 1u && a.recs != nullptr)
@@ -252,13 +309,12 @@ __global__ void __launch_bounds__(kSlice, 3) k_leaf_tree(LeafTree a)
     }
   }
   __syncthreads();
-  if (!active) return;
 
   // the walk; slot of a node or leaf of the slice: its index + lb - lo.  The
   // finished node's own box and count stay in registers; only the sibling's
   // are read.
   const uint32_t off = lb - lo;
-  uint32_t node = L - 1 + k, count = 0, p = 0;
+  uint32_t node = active ? L - 1 + k : 0, count = 0, p = 0;
   if (node != 0) p = sh.t.leafParent[tid];
   for (int level = 0; node != 0; level++)
   {
@@ -276,7 +332,11 @@ __global__ void __launch_bounds__(kSlice, 3) k_leaf_tree(LeafTree a)
     }
     if (!inSlice)
     {
-      a.open[atomicAdd(a.openCount, 1u)] = nb + node;  // one per leaf at most: the list holds them
+      const uint32_t e = atomicAdd(&s_open, 1u);
+      if (e < kEdge)
+        out.open[kEdge * (size_t)blockIdx.x + e] =
+            make_uint2(nb + node, p | (a.lr[nb + p].escapeIndex == node ? kUpRight : 0u));
+      else atomicOr(a.errorWord, kErrLayout);
       break;
     }
     if (atomic_add_acq_rel_cta(&sh.t.visit[slot], 1u) == 0u) break;  // the sibling is not finished yet
@@ -303,58 +363,228 @@ __global__ void __launch_bounds__(kSlice, 3) k_leaf_tree(LeafTree a)
     node = p;
     p = sh.t.nodeParent[slot];
   }
+  if (a.nTris <= kSlice) return;
+  __syncthreads();
+  if (tid == 0) out.counts[blockIdx.x] = min(s_open, kEdge) | min(s_leaving, kEdge) << 16;
 }
 
-// The walks on from the slices' outermost nodes.  A level is a chain of memory
-// latencies, so the links (static) are read beside the arrival and the next
-// parent beside the sibling.
-template <bool SEG> __global__ void __launch_bounds__(128) k_climb(LeafTree a)
+// The walks on from the slices' outermost nodes, tier by tier: a block takes a
+// group of kFan slices (or groups), reads the nodes that leave those into
+// shared memory, a slot each (their links are static), and walks from the
+// outermost finished nodes below as far as nodes whose range lies in the group.
+// A level is then a chain of shared-memory accesses; a node's box goes out
+// beside it.  Slot of a node: its place in the lists, which `visit` holds.
+// With links, boxes and arrival counters in L2, one kernel, a level was two
+// latencies and a release at device scope: 41 us for 2M triangles, 40 for
+// 500,000, 24 for 15,000; so 32 (three tiers), 22 and 8.
+// a slot's link: its parent's slot, its side there, what it is
+constexpr uint32_t kLinkSlot = 0xFFFu, kLinkRight = 1u << 12, kLinkOut = 1u << 13, kLinkIn = 1u << 14,
+                   kLinkRoot = 1u << 15, kLinkArrived = 1u << 16;
+
+struct ClimbShared
 {
-  const uint32_t n = *a.openCount;
-  for (uint32_t e = blockIdx.x * 128 + threadIdx.x; e < n; e += gridDim.x * 128)
+  float    box[2][6][kSlots];  // of a slot's left and right child
+  uint32_t link[kSlots], node[kSlots], up[kSlots];
+};
+
+__device__ __forceinline__ uint32_t arrive_cta(uint32_t* link)
+{
+  uint32_t old;
+  asm volatile("atom.acq_rel.cta.shared::cta.or.b32 %0, [%1], %2;"
+               : "=r"(old)
+               : "r"((uint32_t)__cvta_generic_to_shared(link)), "r"(kLinkArrived)
+               : "memory");
+  return old;
+}
+
+template <bool SEG> __global__ void __launch_bounds__(kClimbThreads) k_climb(LeafTree a, int tier, uint64_t groupLeaves)
+{
+  extern __shared__ uint4 s_climb[];
+  ClimbShared& sh = *reinterpret_cast<ClimbShared*>(s_climb);
+  __shared__ uint32_t s_counts[kFan], s_open, s_leaving;
+  const uint32_t Ltot = SEG ? a.counts[0] : (a.params->nLeaves <= a.nTris ? a.params->nLeaves : 0u);
+  if (blockIdx.x * groupLeaves >= Ltot) return;
+  const uint32_t tid = threadIdx.x, lo = (uint32_t)(blockIdx.x * groupLeaves);
+  const TierLists in = tier_lists(a.lists, a.nTris, tier), out = tier_lists(a.lists, a.nTris, tier + 1);
+  const bool last = gridDim.x == 1;
+  if (tid < kFan)
   {
-    const uint32_t at = a.open[e];
-    uint32_t nb = 0, ib = 0, L = SEG ? 0u : a.params->nLeaves;
-    if (SEG)
+    const uint64_t first = lo + tid * (groupLeaves / kFan);
+    s_counts[tid] = first < Ltot ? in.counts[blockIdx.x * kFan + tid] : 0u;
+  }
+  if (tid == 0) s_open = s_leaving = 0u;
+  __syncthreads();
+
+  // list item s: producer s % kFan, its item s / kFan; slot kEdge * producer + item
+  auto slot_of = [](uint32_t s) { return kEdge * (s % kFan) + s / kFan; };
+  // geometry of LR node `at`: first LR node, internal node and leaf, leaves
+  auto geometry = [&](uint32_t at, uint32_t& nb, uint32_t& ib, uint32_t& lb, uint32_t& L) {
+    nb = ib = lb = 0;
+    L = Ltot;
+    if (!SEG) return;
+    const uint32_t s = find_segment(a.nodeOffsets, a.G, at);
+    nb = a.nodeOffsets[s];
+    ib = a.intOffsets[s];
+    lb = a.leafOffsets[s];
+    L = a.leafOffsets[s + 1] - lb;
+  };
+  // The loads go in stages over all of a thread's items, so that a stage is one
+  // latency.  Item q of a list is producer c's number k.
+  constexpr int kPer = kSlots / kClimbThreads;
+  struct Item
+  {
+    uint32_t at, end, up;
+  } edge[kPer], open[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+  {
+    const uint32_t s = q * kClimbThreads + tid, c = s % kFan, k = s / kFan, n = s_counts[c];
+    const size_t list = kEdge * ((size_t)blockIdx.x * kFan + c) + k;
+    edge[q].at = open[q].at = kNone;
+    if (k < n >> 16) edge[q] = {in.leaving[list], in.end[list], in.up[list]};
+    if (k < (n & 0xFFFFu))
     {
-      const uint32_t s = find_segment(a.nodeOffsets, a.G, at);
-      nb = a.nodeOffsets[s];
-      ib = a.intOffsets[s];
-      L = a.leafOffsets[s + 1] - a.leafOffsets[s];
-    }
-    uint32_t node = at - nb, p = a.parent[at];
-    float4 lo4, hi4;
-    load_node_cg(a.lr + at, lo4, hi4);
-    uint32_t count = __ldcg(&a.lrCount[at]);
-    float mn[3] = {lo4.x, lo4.y, lo4.z}, mx[3] = {hi4.x, hi4.y, hi4.z};
-    for (int level = 0; node != 0; level++)
-    {
-      if (p + 1u >= L || level > kMaxDepth)
-      {
-        atomicOr(a.errorWord, kErrLayout);
-        break;
-      }
-      const uint32_t l = __ldcg(&a.lr[nb + p].leftOffset), r = __ldcg(&a.lr[nb + p].escapeIndex);
-      if (atomic_add_acq_rel(&a.visit[ib + p], 1u) == 0u) break;
-      const uint32_t sib = l == node ? r : l;
-      const uint32_t above = p != 0u ? a.parent[nb + p] : 0u;
-      load_node_cg(a.lr + nb + sib, lo4, hi4);
-      count += __ldcg(&a.lrCount[nb + sib]) + 2u;
-      unite(l == node, mn, mx, lo4, hi4);
-      store_node(a.lr + nb + p, mn, mx, l, r);
-      a.lrCount[nb + p] = count;
-      node = p;
-      p = above;
+      const uint2 v = in.open[list];
+      open[q] = {v.x, 0u, v.y};
     }
   }
+  // where a node goes on: its parent's slot and its side there
+  auto link_up = [&](const Item& t, uint32_t ib, uint32_t lb, uint32_t L) {
+    const uint32_t p = t.up & ~kUpRight;
+    if (p + 1u >= L)
+    {
+      atomicOr(a.errorWord, kErrLayout);
+      return kLinkOut;
+    }
+    const bool inside = p + lb >= lo && p + lb - lo < groupLeaves;
+    return ((t.up & kUpRight) ? kLinkRight : 0u) | (inside ? a.visit[ib + p] & (kSlots - 1u) : kLinkOut);
+  };
+  uint32_t moved[kPer], from[kPer], fromLink[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+  {
+    const Item& t = edge[q];
+    uint32_t nb, ib, lb, L;
+    moved[q] = kNone;
+    from[q] = open[q].at;
+    if (t.at != kNone)
+    {
+      geometry(t.at, nb, ib, lb, L);
+      const uint32_t i = t.at - nb, r0 = min(i, t.end), r1 = max(i, t.end);
+      uint32_t link = 0u;
+      if (r0 + lb >= lo && r1 + lb - lo < groupLeaves)
+      {
+        link = kLinkIn | (i == 0u ? kLinkRoot : link_up(t, ib, lb, L));
+        a.lrCount[t.at] = 2u * (r1 - r0);  // two for each node below
+      }
+      else
+      {
+        const uint32_t e = atomicAdd(&s_leaving, 1u);
+        if (last || e >= kEdge) atomicOr(a.errorWord, kErrLayout);
+        else
+        {
+          const size_t to = kEdge * (size_t)blockIdx.x + e;
+          out.leaving[to] = t.at;
+          out.end[to] = t.end;
+          out.up[to] = t.up;
+          moved[q] = ib + i;
+          link = e;
+        }
+      }
+      const uint32_t slot = slot_of(q * kClimbThreads + tid);
+      sh.link[slot] = link;
+      sh.node[slot] = t.at;
+      sh.up[slot] = t.up;
+    }
+    if (from[q] != kNone)
+    {
+      geometry(from[q], nb, ib, lb, L);
+      fromLink[q] = link_up(open[q], ib, lb, L);
+    }
+  }
+  __syncthreads();  // every slot that the block needs has been read from visit
+#pragma unroll
+  for (int q = 0; q < kPer; q++)
+    if (moved[q] != kNone)
+      a.visit[moved[q]] = kSlotMark | (kEdge * (blockIdx.x % kFan) + sh.link[slot_of(q * kClimbThreads + tid)]);
+#pragma unroll 1
+  for (int q = 0; q < kPer; q++)
+  {
+    uint32_t at = kNone, link = 0, up = 0;
+#pragma unroll
+    for (int w = 0; w < kPer; w++)
+      if (w == q)
+      {
+        at = from[w];
+        link = fromLink[w];
+        up = open[w].up;
+      }
+    if (at == kNone) continue;
+    float4 lo4, hi4;
+    load_node_cg(a.lr + at, lo4, hi4);
+    float mn[3] = {lo4.x, lo4.y, lo4.z}, mx[3] = {hi4.x, hi4.y, hi4.z};
+    for (int level = 0; level <= kMaxDepth; level++)
+    {
+      const uint32_t slot = link & (kSlots - 1u), side = (link & kLinkRight) ? 1u : 0u;
+      if ((link & kLinkOut) || !(sh.link[slot] & kLinkIn))
+      {
+        const uint32_t e = atomicAdd(&s_open, 1u);
+        if (last || e >= kEdge) atomicOr(a.errorWord, kErrLayout);
+        else out.open[kEdge * (size_t)blockIdx.x + e] = make_uint2(at, up);
+        break;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+      {
+        sh.box[side][c][slot] = mn[c];
+        sh.box[side][3 + c][slot] = mx[c];
+      }
+      link = arrive_cta(&sh.link[slot]);
+      if (!(link & kLinkArrived)) break;  // the sibling is not finished yet
+      const float4 slo = make_float4(sh.box[side ^ 1u][0][slot], sh.box[side ^ 1u][1][slot], sh.box[side ^ 1u][2][slot], 0.0f);
+      const float4 shi = make_float4(sh.box[side ^ 1u][3][slot], sh.box[side ^ 1u][4][slot], sh.box[side ^ 1u][5][slot], 0.0f);
+      unite(side == 0u, mn, mx, slo, shi);
+      at = sh.node[slot];
+      up = sh.up[slot];
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+      {
+        a.lr[at].boxMin[c] = mn[c];
+        a.lr[at].boxMax[c] = mx[c];
+      }
+      if (link & kLinkRoot)
+      {
+        uint32_t nb, ib, lb, L;
+        geometry(at, nb, ib, lb, L);
+        a.visit[ib] = 2u;
+        break;
+      }
+    }
+  }
+  if (last) return;
+  __syncthreads();
+  if (tid == 0) out.counts[blockIdx.x] = min(s_open, kEdge) | min(s_leaving, kEdge) << 16;
 }
 
-// Blocks of k_climb: an entry or two a thread at the usual dozen per slice.
-inline uint32_t climb_blocks(uint32_t nTris, int numSMs)
+// Leaves and boxes; a single slice leaves nothing to walk on from.
+template <bool SEG> cudaError_t leaf_tree(const LeafTree& t, cudaStream_t s)
 {
-  const uint64_t want = ((uint64_t)(nTris + kSlice - 1) / kSlice * 12 + 127) / 128;
-  const uint64_t most = (uint64_t)numSMs * 16;
-  return (uint32_t)(want < 1 ? 1 : (want > most ? most : want));
+  uint32_t producers = (t.nTris + kSlice - 1) / kSlice;
+  uint64_t leaves = kSlice;
+  k_leaf_tree<SEG><<<producers, kSlice, 0, s>>>(t);
+  if (producers > 1)
+  {
+    const cudaError_t e = cudaFuncSetAttribute(k_climb<SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(ClimbShared));
+    if (e != cudaSuccess) return e;
+  }
+  for (int tier = 0; producers > 1; tier++)
+  {
+    producers = (producers + kFan - 1) / kFan;
+    leaves *= kFan;
+    k_climb<SEG><<<producers, kClimbThreads, sizeof(ClimbShared), s>>>(t, tier, leaves);
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace bc
