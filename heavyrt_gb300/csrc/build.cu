@@ -181,7 +181,6 @@ __global__ void __launch_bounds__(kThreads) k_morton(const float4* __restrict__ 
   __shared__ uint32_t s_hist[4 * 256];
   for (int k = threadIdx.x; k < 4 * 256; k += kThreads) s_hist[k] = 0u;
   __syncthreads();
-  const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll 1
   for (int it = 0; it < kMortonItems; it++)
   {
@@ -204,19 +203,7 @@ __global__ void __launch_bounds__(kThreads) k_morton(const float4* __restrict__ 
       unsorted[i] = code;
       vals[i] = i;
     }
-    const uint32_t first = __shfl_sync(0xFFFFFFFFu, code, 0);  // lane 0 is in when any lane is
-    const uint32_t differ = __reduce_or_sync(0xFFFFFFFFu, in ? code ^ first : 0u);
-#pragma unroll
-    for (int p = 0; p < 4; p++)
-    {
-      const uint32_t d = (code >> (8 * p)) & 0xFFu;
-      if (((differ >> (8 * p)) & 0xFFu) == 0u)
-      {
-        if (lane == 0) atomicAdd(&s_hist[p * 256 + d], (uint32_t)__popc(mask));
-      }
-      else if (in)
-        atomicAdd(&s_hist[p * 256 + d], 1u);
-    }
+    bc::count_digits(code, in, mask, s_hist);
   }
   __syncthreads();
   for (int k = threadIdx.x; k < 4 * 256; k += kThreads)

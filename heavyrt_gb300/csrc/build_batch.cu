@@ -161,26 +161,52 @@ __global__ void __launch_bounds__(kThreads) k_seg_box_final(const uint32_t* __re
   }
 }
 
+// The codes, their digits' counts for the sort (hist, zero before) and the
+// unsorted codes, as k_morton in build.cu.  Counted and copied in passes of
+// their own, 7 + 5 us of a batch of 48 geometries.
+constexpr int kMortonItems = 4;
+
 __global__ void __launch_bounds__(kThreads) k_seg_morton(const float4* __restrict__ v, const uint32_t* __restrict__ idx,
                                                          const uint32_t* __restrict__ vertOffsets,
                                                          const uint32_t* __restrict__ triOffsets, uint32_t G,
                                                          uint32_t N, const BuildParams* __restrict__ params,
                                                          uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                         uint32_t* __restrict__ unsorted, uint32_t* __restrict__ hist,
                                                          uint32_t* errorWord)
 {
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
-  if (t >= N) return;
-  const uint32_t s = find_segment(triOffsets, G, t);
-  const uint32_t nT = triOffsets[s + 1] - triOffsets[s];
-  const uint32_t vb = vertOffsets[s], nV = vertOffsets[s + 1] - vb;
-  uint32_t ia = idx[3 * (size_t)t + 0], ib = idx[3 * (size_t)t + 1], ic = idx[3 * (size_t)t + 2];
-  if (ia >= nV || ib >= nV || ic >= nV)
+  __shared__ uint32_t s_hist[4 * 256];
+  for (int k = threadIdx.x; k < 4 * 256; k += kThreads) s_hist[k] = 0u;
+  __syncthreads();
+#pragma unroll 1
+  for (int it = 0; it < kMortonItems; it++)
   {
-    atomicOr(errorWord, kErrIndexRange);
-    ia = ib = ic = 0;
+    const uint64_t at = ((uint64_t)blockIdx.x * kMortonItems + it) * kThreads + threadIdx.x;
+    const bool in = at < N;
+    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, in);
+    if (mask == 0u) break;
+    uint32_t code = 0;
+    if (in)
+    {
+      const uint32_t t = (uint32_t)at;
+      const uint32_t s = find_segment(triOffsets, G, t);
+      const uint32_t nT = triOffsets[s + 1] - triOffsets[s];
+      const uint32_t vb = vertOffsets[s], nV = vertOffsets[s + 1] - vb;
+      uint32_t ia = idx[3 * (size_t)t + 0], ib = idx[3 * (size_t)t + 1], ic = idx[3 * (size_t)t + 2];
+      if (ia >= nV || ib >= nV || ic >= nV)
+      {
+        atomicOr(errorWord, kErrIndexRange);
+        ia = ib = ic = 0;
+      }
+      code = bc::morton_code(v[vb + ia], v[vb + ib], v[vb + ic], nT, params[s].bmin, params[s].scale);
+      keys[t] = code;
+      unsorted[t] = code;
+      vals[t] = t;
+    }
+    bc::count_digits(code, in, mask, s_hist);
   }
-  keys[t] = bc::morton_code(v[vb + ia], v[vb + ib], v[vb + ic], nT, params[s].bmin, params[s].scale);
-  vals[t] = t;
+  __syncthreads();
+  for (int k = threadIdx.x; k < 4 * 256; k += kThreads)
+    if (s_hist[k]) atomicAdd(&hist[k], s_hist[k]);
 }
 
 __global__ void __launch_bounds__(kThreads) k_seg_compact(const uint32_t* __restrict__ keys, uint32_t n,
@@ -410,14 +436,17 @@ cudaError_t build_lbvh_batch(const BatchBuffers& b, int numSMs, cudaStream_t s)
   if (b.nBoxChunks + b.nIdxChunks) k_seg_read_inputs<<<b.nBoxChunks + b.nIdxChunks, kThreads, 0, s>>>(b);
   k_seg_box_final<<<(G + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, s>>>(b.boxChunkOffsets, G, b.boxPartial,
                                                                                   b.params, b.mortonCubic);
-  k_seg_morton<<<(N + kThreads - 1) / kThreads, kThreads, 0, s>>>(b.verts, b.idx, b.vertOffsets, b.triOffsets, G, N,
-                                                                   b.params, b.keys, b.vals, b.errorWord);
-  cudaError_t e = cudaMemcpyAsync(b.keysUnsorted, b.keys, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, s);
+  // an odd number of sort passes starts from the spare arrays and ends in keys and vals
+  const bool swap = radix_sort_segmented_passes(G) & 1;
+  uint32_t *keys0 = swap ? b.keysAlt : b.keys, *vals0 = swap ? b.valsAlt : b.vals;
+  constexpr uint32_t kPerBlock = kThreads * kMortonItems;
+  cudaError_t e = cudaMemsetAsync(b.scratch, 0, build_batch_scratch_bytes(N, G), s);
   if (e != cudaSuccess) return e;
-  e = radix_sort_pairs_segmented(b.keys, b.vals, b.keysAlt, b.valsAlt, N, b.triOffsets, G, sortScratch, b.errorWord,
-                                 numSMs, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(scratch, 0, scanBytes, s);
+  k_seg_morton<<<(N + kPerBlock - 1) / kPerBlock, kThreads, 0, s>>>(b.verts, b.idx, b.vertOffsets, b.triOffsets, G, N,
+                                                                     b.params, keys0, vals0, b.keysUnsorted,
+                                                                     (uint32_t*)sortScratch, b.errorWord);
+  e = radix_sort_pairs_segmented(keys0, vals0, swap ? b.keys : b.keysAlt, swap ? b.vals : b.valsAlt, N, b.triOffsets, G,
+                                 sortScratch, b.errorWord, s);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(b.counts, 0, 4 * sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;

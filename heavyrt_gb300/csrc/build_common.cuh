@@ -91,6 +91,26 @@ __device__ __forceinline__ uint32_t morton_code(const float4& a, const float4& b
   return spread_bits(q[0], 0) | spread_bits(q[1], 1) | spread_bits(q[2], 2);
 }
 
+// The four 8-bit digits of a warp's codes to a block's counters (4 x 256);
+// `mask` = the lanes that are `in`, lane 0 among them.  A warp whose codes agree
+// in a digit adds once.
+__device__ __forceinline__ void count_digits(uint32_t code, bool in, uint32_t mask, uint32_t* hist)
+{
+  const uint32_t first = __shfl_sync(0xFFFFFFFFu, code, 0);
+  const uint32_t differ = __reduce_or_sync(0xFFFFFFFFu, in ? code ^ first : 0u);
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+  {
+    const uint32_t d = (code >> (8 * p)) & 0xFFu;
+    if (((differ >> (8 * p)) & 0xFFu) == 0u)
+    {
+      if ((threadIdx.x & 31u) == 0u) atomicAdd(&hist[p * 256 + d], (uint32_t)__popc(mask));
+    }
+    else if (in)
+      atomicAdd(&hist[p * 256 + d], 1u);
+  }
+}
+
 // ZIndexMultCoeff on the box widened by 1e-4 (core/builders/lbvh.cpp:41-51,263).
 // cubic = 1 (the engine's HRT_MORTON_CUBIC frame, no reference counterpart):
 // x, y and z share the scale of the longest widened extent, so a cell of the

@@ -22,11 +22,15 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keysAlt, 
                              void* scratch, uint32_t* errorWord, int numSMs, cudaStream_t stream, bool counted = false);
 // Stable sort by (segment, key) where the segment of a pair is the segment of
 // its value in segOffsets[0..segCount] (device, ascending, offsets[0] = 0):
-// each segment ends up sorted by key in place of its input range.
+// each segment ends up sorted by key in place of its input range.  The result
+// is in keys/vals after an even number of passes, in keysAlt/valsAlt after an
+// odd one.  scratch was cleared before, and its first 4 x 256 words hold the
+// counts of the keys' four digits.
 size_t radix_sort_segmented_scratch_bytes(uint32_t n, uint32_t segCount);
+int radix_sort_segmented_passes(uint32_t segCount);
 cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t* keysAlt, uint32_t* valsAlt,
                                        uint32_t n, const uint32_t* segOffsets, uint32_t segCount, void* scratch,
-                                       uint32_t* errorWord, int numSMs, cudaStream_t stream);
+                                       uint32_t* errorWord, cudaStream_t stream);
 
 // ---------------------------------------------------------------- build.cu
 struct BuildBuffers

@@ -318,6 +318,8 @@ static int segment_passes(uint32_t segCount)
   return p;
 }
 
+int radix_sort_segmented_passes(uint32_t segCount) { return kPasses + segment_passes(segCount); }
+
 size_t radix_sort_segmented_scratch_bytes(uint32_t n, uint32_t segCount)
 {
   const size_t tiles = (n + kTile - 1) / kTile;
@@ -327,21 +329,14 @@ size_t radix_sort_segmented_scratch_bytes(uint32_t n, uint32_t segCount)
 
 cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t* keysAlt, uint32_t* valsAlt,
                                        uint32_t n, const uint32_t* segOffsets, uint32_t segCount, void* scratch,
-                                       uint32_t* errorWord, int numSMs, cudaStream_t stream)
+                                       uint32_t* errorWord, cudaStream_t stream)
 {
-  if (n <= 1) return cudaSuccess;
   const int segPasses = segment_passes(segCount);
   const int passes = kPasses + segPasses;
   const uint32_t tiles = (n + kTile - 1) / kTile;
   uint32_t* hist = (uint32_t*)scratch;
   uint32_t* counters = hist + passes * kRadix;
   uint32_t* status = counters + passes + 4;
-  cudaError_t e = cudaMemsetAsync(scratch, 0, radix_sort_segmented_scratch_bytes(n, segCount), stream);
-  if (e != cudaSuccess) return e;
-  uint32_t hb = (n + kThreads - 1) / kThreads;
-  const uint32_t maxHb = (uint32_t)numSMs * 4u;
-  if (hb > maxHb) hb = maxHb;
-  k_histogram<<<hb, kThreads, 0, stream>>>(keys, n, hist);
   for (int q = 0; q < segPasses; q++)
     k_segment_histogram<<<(segCount + 255) / 256, 256, 0, stream>>>(segOffsets, segCount, 8u * q,
                                                                      hist + (kPasses + q) * kRadix);
@@ -360,13 +355,6 @@ cudaError_t radix_sort_pairs_segmented(uint32_t* keys, uint32_t* vals, uint32_t*
                                          errorWord, segOffsets, segCount);
     uint32_t* t = srcK; srcK = dstK; dstK = t;
     t = srcV; srcV = dstV; dstV = t;
-  }
-  if (srcK != keys)
-  {
-    e = cudaMemcpyAsync(keys, srcK, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, stream);
-    if (e != cudaSuccess) return e;
-    e = cudaMemcpyAsync(vals, srcV, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, stream);
-    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
