@@ -124,41 +124,56 @@ template <int THREADS> __device__ __forceinline__ void block_bounds(float (&mn)[
       for (int k = 0; k < 4; k++) { mn[k] = lm_min(mn[k], smn[w][k]); mx[k] = lm_max(mx[k], smx[w][k]); }
 }
 
-__global__ void __launch_bounds__(kThreads)
-    k_read_inputs(const uint8_t* raw, uint64_t stride, uint32_t n, float4* out, const uint32_t* idxSrc, uint32_t* idx,
-                  uint64_t nIdx, float4* partial, uint32_t* done, BuildParams* params, int cubic, int reset)
+struct ReadArgs
+{
+  const uint8_t*  raw;
+  uint64_t        stride;
+  uint32_t        n;
+  float4*         out;
+  const uint32_t* idxSrc;
+  uint32_t*       idx;
+  uint64_t        nIdx;
+  float4*         partial;
+  uint32_t*       done;
+  BuildParams*    params;
+  int             cubic, reset;
+};
+
+__device__ __forceinline__ void read_inputs(const ReadArgs& a, uint32_t block, uint32_t blocks)
 {
   float mn[4] = {1e10f, 1e10f, 1e10f, 1e10f}, mx[4] = {-1e10f, -1e10f, -1e10f, -1e10f};
   __shared__ float4 s_raw[3 * kThreads];
   __shared__ bool   s_last;
-  read_part<kThreads>(raw, stride, n, out, idxSrc, idx, nIdx, blockIdx.x, gridDim.x, s_raw, mn, mx);
+  read_part<kThreads>(a.raw, a.stride, a.n, a.out, a.idxSrc, a.idx, a.nIdx, block, blocks, s_raw, mn, mx);
   block_bounds<kThreads>(mn, mx);
   if (threadIdx.x == 0)
   {
-    partial[2 * blockIdx.x + 0] = make_float4(mn[0], mn[1], mn[2], mn[3]);
-    partial[2 * blockIdx.x + 1] = make_float4(mx[0], mx[1], mx[2], mx[3]);
-    s_last = bc::atomic_add_acq_rel(done, 1u) == gridDim.x - 1u;
+    a.partial[2 * block + 0] = make_float4(mn[0], mn[1], mn[2], mn[3]);
+    a.partial[2 * block + 1] = make_float4(mx[0], mx[1], mx[2], mx[3]);
+    s_last = bc::atomic_add_acq_rel(a.done, 1u) == blocks - 1u;
   }
   __syncthreads();
   if (!s_last) return;
   for (int k = 0; k < 4; k++) { mn[k] = 1e10f; mx[k] = -1e10f; }
-  for (uint32_t b = threadIdx.x; b < gridDim.x; b += kThreads)
+  for (uint32_t b = threadIdx.x; b < blocks; b += kThreads)
   {
-    const float4 a = __ldcg(partial + 2 * b), c = __ldcg(partial + 2 * b + 1);
-    mn[0] = lm_min(mn[0], a.x); mn[1] = lm_min(mn[1], a.y); mn[2] = lm_min(mn[2], a.z); mn[3] = lm_min(mn[3], a.w);
-    mx[0] = lm_max(mx[0], c.x); mx[1] = lm_max(mx[1], c.y); mx[2] = lm_max(mx[2], c.z); mx[3] = lm_max(mx[3], c.w);
+    const float4 lo = __ldcg(a.partial + 2 * b), hi = __ldcg(a.partial + 2 * b + 1);
+    mn[0] = lm_min(mn[0], lo.x); mn[1] = lm_min(mn[1], lo.y); mn[2] = lm_min(mn[2], lo.z); mn[3] = lm_min(mn[3], lo.w);
+    mx[0] = lm_max(mx[0], hi.x); mx[1] = lm_max(mx[1], hi.y); mx[2] = lm_max(mx[2], hi.z); mx[3] = lm_max(mx[3], hi.w);
   }
   block_bounds<kThreads>(mn, mx);
   if (threadIdx.x != 0) return;
-  bc::zindex_scale(mn, mx, params, cubic);
-  if (reset)
+  bc::zindex_scale(mn, mx, a.params, a.cubic);
+  if (a.reset)
   {
-    params->nLeaves = 0;
-    params->error = 0;
-    params->rootRecord = 0;
-    params->pad = 0;
+    a.params->nLeaves = 0;
+    a.params->error = 0;
+    a.params->rootRecord = 0;
+    a.params->pad = 0;
   }
 }
+
+__global__ void __launch_bounds__(kThreads) k_read_inputs(ReadArgs a) { read_inputs(a, blockIdx.x, gridDim.x); }
 
 // ---------------------------------------------------------------- Morton codes
 // kernel1D_EvalMortonCodesFromTriangles, core/builders/lbvh.cpp:259-287: box
@@ -231,17 +246,17 @@ __global__ void __launch_bounds__(kThreads) k_compact_runs(const uint32_t* __res
 // delta() and kernel1D_Karras12, core/builders/lbvh.cpp:386-441.  The codes
 // are unique after compaction, so delta(i,j) is the count of leading zeros of
 // their XOR (32 for equal codes, -1 out of range, as the reference defines).
-__global__ void __launch_bounds__(kThreads) k_karras(const uint32_t* __restrict__ codes,
-                                                     const BuildParams* __restrict__ params, BVHNode32* __restrict__ lr,
-                                                     uint32_t* __restrict__ parent, uint32_t* __restrict__ visit,
-                                                     uint32_t* __restrict__ rangeEnd)
+__device__ __forceinline__ void karras(const uint32_t* __restrict__ codes, const BuildParams* __restrict__ params,
+                                       BVHNode32* __restrict__ lr, uint32_t* __restrict__ parent,
+                                       uint32_t* __restrict__ visit, uint32_t* __restrict__ rangeEnd, uint32_t block,
+                                       uint32_t blocks)
 {
   const int L = (int)params->nLeaves;
   // one node per thread; a warp's 32 consecutive nodes exchange their codes
   // for the direction test (karras_neighbours), so the loop bound is uniform
   // over the warp
   const int lane = (int)(threadIdx.x & 31u);
-  for (int base = (int)(blockIdx.x * kThreads + (threadIdx.x & ~31u)); base < L - 1; base += gridDim.x * kThreads)
+  for (int base = (int)(block * kThreads + (threadIdx.x & ~31u)); base < L - 1; base += blocks * kThreads)
   {
     const int i = base + lane;
     const bool active = i < L - 1;
@@ -259,6 +274,27 @@ __global__ void __launch_bounds__(kThreads) k_karras(const uint32_t* __restrict_
     rangeEnd[i] = (uint32_t)other;
     visit[i] = 0u;
   }
+}
+
+__global__ void __launch_bounds__(kThreads) k_karras(const uint32_t* __restrict__ codes,
+                                                     const BuildParams* __restrict__ params, BVHNode32* __restrict__ lr,
+                                                     uint32_t* __restrict__ parent, uint32_t* __restrict__ visit,
+                                                     uint32_t* __restrict__ rangeEnd)
+{
+  karras(codes, params, lr, parent, visit, rangeEnd, blockIdx.x, gridDim.x);
+}
+
+// A refit's new vertices and, by the blocks after the first readBlocks, its
+// unchanged hierarchy's links: the reads wait on the host link and the links
+// on L2 (a refit of 500,000 triangles with its frame 266 us, 242 so).
+__global__ void __launch_bounds__(kThreads) k_read_and_link(ReadArgs a, uint32_t readBlocks,
+                                                            const uint32_t* __restrict__ codes,
+                                                            const BuildParams* __restrict__ params,
+                                                            BVHNode32* __restrict__ lr, uint32_t* __restrict__ parent,
+                                                            uint32_t* __restrict__ visit, uint32_t* __restrict__ rangeEnd)
+{
+  if (blockIdx.x < readBlocks) read_inputs(a, blockIdx.x, readBlocks);
+  else karras(codes, params, lr, parent, visit, rangeEnd, blockIdx.x - readBlocks, gridDim.x - readBlocks);
 }
 
 // ---------------------------------------------------------------- traversal records
@@ -488,22 +524,14 @@ BuildScratch build_scratch(void* scratch, uint32_t nTris)
   return q;
 }
 
-cudaError_t read_inputs(const BuildBuffers& b, float4* partial, uint32_t* done, BuildParams* params, int reset,
-                        int numSMs, cudaStream_t s)
+ReadArgs read_args(const BuildBuffers& b, float4* partial, uint32_t* done, BuildParams* params, int reset)
 {
-  const uint64_t nIdx = 3 * (uint64_t)b.nTris;
-  uint32_t g = grid_for(std::max<uint64_t>(b.nVerts, nIdx / 4), numSMs, 4);
-  if (g > kBoxBlocks) g = kBoxBlocks;
-  k_read_inputs<<<g, kThreads, 0, s>>>(b.raw, b.rawStride, b.nVerts, b.verts, b.idxSrc, b.idx, nIdx, partial, done,
-                                       params, b.mortonCubic, reset);
-  return cudaGetLastError();
+  return {b.raw, b.rawStride, b.nVerts, b.verts, b.idxSrc, b.idx, 3 * (uint64_t)b.nTris, partial, done, params,
+          b.mortonCubic, reset};
 }
-
-cudaError_t hierarchy(const BuildBuffers& b, int numSMs, cudaStream_t s)
+uint32_t read_blocks(const BuildBuffers& b, int numSMs)
 {
-  k_karras<<<grid_for(b.nTris, numSMs, 8), kThreads, 0, s>>>(b.compressed, b.params, b.lr, b.parent, b.visit,
-                                                             b.visit + b.nTris);
-  return cudaGetLastError();
+  return std::min(kBoxBlocks, grid_for(std::max<uint64_t>(b.nVerts, 3 * (uint64_t)b.nTris / 4), numSMs, 4));
 }
 
 // Leaves, boxes and (binary layout) pair records, from the sorted triangles,
@@ -555,8 +583,7 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   cudaError_t e = cudaMemsetAsync(b.scratch, 0, q.zeroBytes, s);
   if (e != cudaSuccess) return e;
   // 1. inputs, scene box and Morton scale
-  e = read_inputs(b, q.partial, q.boxDone, b.params, 1, numSMs, s);
-  if (e != cudaSuccess) return e;
+  k_read_inputs<<<read_blocks(b, numSMs), kThreads, 0, s>>>(read_args(b, q.partial, q.boxDone, b.params, 1));
   // 2. Morton codes and their digits' counts
   constexpr uint32_t kPerBlock = kThreads * kMortonItems;
   k_morton<<<(N + kPerBlock - 1) / kPerBlock, kThreads, 0, s>>>(b.verts, b.idx, N, b.nVerts, b.params, b.keys,
@@ -568,8 +595,7 @@ cudaError_t build_lbvh(const BuildBuffers& b, int numSMs, cudaStream_t s)
   k_compact_runs<<<(N + kScanTile - 1) / kScanTile, kThreads, 0, s>>>(b.keys, N, b.compressed, b.runStarts, q.scanStatus,
                                                                       q.scanCounter, b.params, err);
   // 5. hierarchy, leaves, boxes, records; the sort's spare array holds the lists
-  e = hierarchy(b, numSMs, s);
-  if (e != cudaSuccess) return e;
+  k_karras<<<grid_for(N, numSMs, 8), kThreads, 0, s>>>(b.compressed, b.params, b.lr, b.parent, b.visit, b.visit + N);
   return build_tree(b, b.keysAlt, numSMs, s);
 }
 
@@ -585,9 +611,10 @@ cudaError_t refit_lbvh(const BuildBuffers& b, BuildParams* boxOut, int numSMs, c
   uint32_t* done = (uint32_t*)b.scratch;  // refit_scratch_bytes(): a counter, box parts, lists
   float4* partial = (float4*)((char*)b.scratch + 256);
   cudaError_t e = cudaMemsetAsync(done, 0, sizeof(uint32_t), s);
-  if (e == cudaSuccess) e = read_inputs(b, partial, done, boxOut, 0, numSMs, s);
-  if (e == cudaSuccess) e = hierarchy(b, numSMs, s);
   if (e != cudaSuccess) return e;
+  const uint32_t reads = read_blocks(b, numSMs), links = grid_for(b.nTris, numSMs, 4);
+  k_read_and_link<<<reads + links, kThreads, 0, s>>>(read_args(b, partial, done, boxOut, 0), reads, b.compressed, b.params,
+                                                     b.lr, b.parent, b.visit, b.visit + b.nTris);
   return build_tree(b, (uint32_t*)(partial + 2 * kBoxBlocks), numSMs, s);
 }
 
