@@ -30,6 +30,7 @@
 #include <cstring>
 #include <vector>
 
+#include "build_common.cuh"
 #include "hrt_internal.cuh"
 #include "raygen_common.cuh"
 
@@ -41,7 +42,6 @@ namespace
 {
 
 constexpr int      kThreads = 256;
-constexpr int      kChunk = 4;  // items per thread in the compaction blocks
 constexpr uint32_t kAoTile = HRT_AO_TILE_SIZE;
 constexpr float    kHitBack = 10000000.0f;  // RTAO::AO_HIT_BACK
 
@@ -131,13 +131,21 @@ __device__ __forceinline__ void mul3x3(const float* m, const float v[3], float o
 // ray's flag (1 = the pixel gets AO rays).  The triangle is read from the
 // geometry's index buffer in sorted order at the hit's primId (its sorted
 // position), i.e. the triangle that was hit.
+//
+// A block takes kThreads consecutive rays and counts its flags; the last block
+// to finish (counted in *done, zero before) turns the counts into each block's
+// first AO slot and the total.  Bound by the reads and the dependent gathers of
+// the hit triangle (several rays a thread: 1280 x 720, 26 us, one 23).
 __global__ void __launch_bounds__(kThreads)
     k_rtao_positions(const float4* __restrict__ rays, const hrt_hit* __restrict__ hits,
                      const uint32_t* __restrict__ pixel, uint64_t n, const FrameGeom* __restrict__ geoms,
                      uint32_t nGeoms, const float* __restrict__ normMatrices, uint32_t nInst,
-                     float4* __restrict__ positions, uint8_t* __restrict__ flag, uint32_t* errorWord)
+                     float4* __restrict__ positions, uint8_t* __restrict__ flag, uint32_t* blockCount,
+                     unsigned long long* total, uint32_t* done, uint32_t* errorWord)
 {
-  for (uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x; k < n; k += (uint64_t)gridDim.x * kThreads)
+  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+  bool flagged = false;
+  if (k < n)
   {
     const hrt_hit h = hits[k];
     float4 out;
@@ -188,181 +196,170 @@ __global__ void __launch_bounds__(kThreads)
       out = make_float4(p[0], p[1], p[2], __uint_as_float(e));
     }
     positions[pixel[k]] = out;
-    flag[k] = out.y < kHitBack ? 1 : 0;
+    flagged = out.y < kHitBack;
+    flag[k] = flagged ? 1 : 0;
   }
-}
-
-// Flagged rays per block of kThreads * kChunk traced rays.
-__global__ void __launch_bounds__(kThreads) k_flag_count(const uint8_t* __restrict__ flag, uint64_t n,
-                                                         uint32_t* __restrict__ blockCount)
-{
   __shared__ uint32_t s_warp[kThreads / 32];
-  const uint64_t base = (uint64_t)blockIdx.x * kThreads * kChunk;
-  uint32_t c = 0;
-#pragma unroll
-  for (int j = 0; j < kChunk; j++)
-  {
-    const uint64_t k = base + (uint64_t)j * kThreads + threadIdx.x;
-    c += (k < n && flag[k]) ? 1u : 0u;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xFFFFFFFFu, c, o);
-  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = c;
+  __shared__ bool     s_last;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t inWarp = __popc(__ballot_sync(0xFFFFFFFFu, flagged));
+  if (lane == 0) s_warp[warp] = inWarp;
   __syncthreads();
   if (threadIdx.x == 0)
   {
     uint32_t t = 0;
     for (int w = 0; w < kThreads / 32; w++) t += s_warp[w];
     blockCount[blockIdx.x] = t;
+    s_last = bc::atomic_add_acq_rel(done, 1u) == gridDim.x - 1u;
   }
-}
-
-// Exclusive scan of the block counts in one block; the total -> *total.
-__global__ void __launch_bounds__(1024) k_scan_counts(uint32_t* blockCount, uint32_t nBlocks, unsigned long long* total)
-{
-  __shared__ uint32_t s[1024];
-  __shared__ unsigned long long s_carry;
-  if (threadIdx.x == 0) s_carry = 0;
   __syncthreads();
-  for (uint32_t b0 = 0; b0 < nBlocks; b0 += 1024)
+  if (!s_last) return;
+  // exclusive scan, a run of blocks a thread (counts below 2^32: a ray each)
+  const uint32_t per = (gridDim.x + kThreads - 1) / kThreads;
+  const uint32_t b0 = min(threadIdx.x * per, gridDim.x), b1 = min(b0 + per, gridDim.x);
+  uint32_t sum = 0;
+#pragma unroll 8
+  for (uint32_t b = b0; b < b1; b++) sum += __ldcg(blockCount + b);
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
   {
-    const uint32_t b = b0 + threadIdx.x;
-    const uint32_t v = b < nBlocks ? blockCount[b] : 0u;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (uint32_t o = 1; o < 1024; o <<= 1)
-    {
-      const uint32_t y = threadIdx.x >= o ? s[threadIdx.x - o] : 0u;
-      __syncthreads();
-      s[threadIdx.x] += y;
-      __syncthreads();
-    }
-    if (b < nBlocks) blockCount[b] = (uint32_t)s_carry + s[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == 1023) s_carry += s[1023];
-    __syncthreads();
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
   }
-  if (threadIdx.x == 0) *total = s_carry;
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  uint32_t at = incl - sum;
+  for (uint32_t w = 0; w < warp; w++) at += s_warp[w];
+  for (uint32_t b = b0; b < b1; b += 8)
+  {
+    uint32_t c[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; q++) c[q] = b + q < b1 ? __ldcg(blockCount + b + q) : 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < 8; q++)
+    {
+      if (b + q < b1) blockCount[b + q] = at;
+      at += c[q];
+    }
+  }
+  if (threadIdx.x == kThreads - 1) *total = at;
 }
 
-// Pixel of every AO slot: the flagged traced rays, ranked in trace order
-// (block offsets from k_scan_counts, ranks inside a block by warp ballots).
-__global__ void __launch_bounds__(kThreads)
-    k_rtao_slots(const uint8_t* __restrict__ flag, uint64_t n, const uint32_t* __restrict__ blockOffset,
-                 const uint32_t* __restrict__ pixel, uint32_t* __restrict__ aoPixel, uint64_t slotCapacity,
-                 uint32_t* errorWord)
-{
-  __shared__ uint32_t s_warp[kThreads / 32 + 1];
-  const uint64_t base = (uint64_t)blockIdx.x * kThreads * kChunk;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t run = 0;
-  for (int j = 0; j < kChunk; j++)
-  {
-    const uint64_t k = base + (uint64_t)j * kThreads + threadIdx.x;
-    const bool f = k < n && flag[k];
-    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, f);
-    if (lane == 0) s_warp[warp] = __popc(ballot);
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-      uint32_t t = 0;
-      for (int w = 0; w < kThreads / 32; w++)
-      {
-        const uint32_t c = s_warp[w];
-        s_warp[w] = t;
-        t += c;
-      }
-      s_warp[kThreads / 32] = t;
-    }
-    __syncthreads();
-    const uint64_t slot = (uint64_t)blockOffset[blockIdx.x] + run + s_warp[warp] + __popc(ballot & ((1u << lane) - 1u));
-    run += s_warp[kThreads / 32];
-    __syncthreads();
-    if (!f) continue;
-    if (slot >= slotCapacity)
-    {
-      atomicOr(errorWord, kErrLayout);
-      continue;
-    }
-    aoPixel[slot] = pixel[k];
-  }
-}
-
-// The per-pixel part of kernel_InitAORay (examples/02_rtao/rtao.cpp:147-165),
-// once per slot: the packed normal decoded (decodeNormal,
+// kernel_InitAORay (examples/02_rtao/rtao.cpp:147-165) for every flagged traced
+// ray: its AO slot is its rank in trace order (block offsets from
+// k_rtao_positions, ranks inside a block by warp ballots), its rays' starts and
+// directions follow from its pixel's frame.  A block makes the frames of its
+// rays' pixels in shared memory, then all its threads the AO rays of those
+// (slot s, sample z at s * raysPerPixel + z), consecutive threads consecutive
+// rays.  The other pixels' colour and visibility become 0 here.  Bound by the
+// rays written.  (Counts, slots, frames, rays and the clearing of the outputs in
+// launches of their own, a frame: 1280 x 720, 16 samples 510 us, 502 so; 1
+// sample 284, 265; 640 x 360, 16 samples 255, 238; 160 x 90, 1 sample 120, 94.)
+//
+// Frame, per slot: the packed normal decoded (decodeNormal,
 // examples/render_common.h:126-137), CoordinateSystem's frame about it
 // (:38-54, the second branch's division in double as the renderer's
 // unqualified sqrt makes it), the offset size epsilonOfPos (:96-98) and the
-// pixel's row of the sample tile.  Record: {pos, eps}, {normal, invSign},
-// {nx, tile row}, {ny, 0}.
-__global__ void __launch_bounds__(kThreads)
-    k_rtao_frames(const uint32_t* __restrict__ aoPixel, uint64_t slots, const float4* __restrict__ positions,
-                  uint32_t width, uint32_t raysPerPixel, float4* __restrict__ frames)
+// pixel's row of the sample tile.  Ray: MapSampleToCosineDistribution with the
+// tile entry's sample direction (dev: (sinT cosP, sinT sinP, cosT) per entry)
+// and OffsRayPos (:56-112).
+struct AoFrame
 {
-  for (uint64_t s = (uint64_t)blockIdx.x * kThreads + threadIdx.x; s < slots; s += (uint64_t)gridDim.x * kThreads)
+  float4 p;  // position, eps
+  float4 n;  // normal, invSign
+  float4 x;  // nx, tile row
+  float4 y;  // ny
+};
+
+__device__ __forceinline__ AoFrame ao_frame(uint32_t pix, const float4& pos, uint32_t width, uint32_t raysPerPixel)
+{
+  const uint32_t x = pix % width, y = pix / width;
+  const uint32_t a = __float_as_uint(pos.w);
+  const uint32_t ex = a & 0x0000FFFFu, ey = (a & 0xFFFF0000u) >> 16;
+  const float sign = (ex & 1u) != 0 ? -1.0f : 1.0f;
+  const float kInv = __fdiv_rn(1.0f, 32767.0f);
+  float nrm[3];
+  nrm[0] = __fmul_rn((float)(int16_t)(uint16_t)(ex & 0xfffeu), kInv);
+  nrm[1] = __fmul_rn((float)(int16_t)(uint16_t)(ey & 0xffffu), kInv);
+  const float zz = __fsub_rn(__fsub_rn(1.0f, __fmul_rn(nrm[0], nrm[0])), __fmul_rn(nrm[1], nrm[1]));
+  nrm[2] = __fmul_rn(sign, __fsqrt_rn(zz < 0.0f ? 0.0f : zz));
+  float nx[3];
+  if (fabsf(nrm[0]) > fabsf(nrm[1]))
   {
-    const uint32_t pix = aoPixel[s];
-    const uint32_t x = pix % width, y = pix / width;
-    const float4 pos = positions[pix];
-    const uint32_t a = __float_as_uint(pos.w);
-    const uint32_t ex = a & 0x0000FFFFu, ey = (a & 0xFFFF0000u) >> 16;
-    const float sign = (ex & 1u) != 0 ? -1.0f : 1.0f;
-    const float kInv = __fdiv_rn(1.0f, 32767.0f);
-    float nrm[3];
-    nrm[0] = __fmul_rn((float)(int16_t)(uint16_t)(ex & 0xfffeu), kInv);
-    nrm[1] = __fmul_rn((float)(int16_t)(uint16_t)(ey & 0xffffu), kInv);
-    const float zz = __fsub_rn(__fsub_rn(1.0f, __fmul_rn(nrm[0], nrm[0])), __fmul_rn(nrm[1], nrm[1]));
-    nrm[2] = __fmul_rn(sign, __fsqrt_rn(zz < 0.0f ? 0.0f : zz));
-    float nx[3];
-    if (fabsf(nrm[0]) > fabsf(nrm[1]))
-    {
-      const float invLen = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(nrm[0], nrm[0]), __fmul_rn(nrm[2], nrm[2]))));
-      nx[0] = __fmul_rn(__fmul_rn(-1.0f, nrm[2]), invLen);
-      nx[1] = 0.0f;
-      nx[2] = __fmul_rn(nrm[0], invLen);
-    }
-    else
-    {
-      const float s2 = __fadd_rn(__fmul_rn(nrm[1], nrm[1]), __fmul_rn(nrm[2], nrm[2]));
-      const float invLen = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn((double)s2)));
-      nx[0] = 0.0f;
-      nx[1] = __fmul_rn(nrm[2], invLen);
-      nx[2] = __fmul_rn(__fmul_rn(-1.0f, nrm[1]), invLen);
-    }
-    const float ny[3] = {__fsub_rn(__fmul_rn(nrm[1], nx[2]), __fmul_rn(nrm[2], nx[1])),
-                         __fsub_rn(__fmul_rn(nrm[2], nx[0]), __fmul_rn(nrm[0], nx[2])),
-                         __fsub_rn(__fmul_rn(nrm[0], nx[1]), __fmul_rn(nrm[1], nx[0]))};
-    const float invSign = hrt::rg::dot3(nrm, nrm) > 0.0f ? 1.0f : -1.0f;
-    // std::max(a, b) = a < b ? b : a
-    const float ax = fabsf(pos.x), ay = fabsf(pos.y), az = fabsf(pos.z);
-    const float myz = ay < az ? az : ay;
-    const float mxyz = ax < myz ? myz : ax;
-    const float gEps = 2e-5f, twoGEps = __fmul_rn(2.0f, gEps);
-    const float eps = __fmul_rn(mxyz < twoGEps ? twoGEps : mxyz, gEps);
-    const uint32_t tileRow = ((y % kAoTile) * kAoTile + (x % kAoTile)) * raysPerPixel;
-    float4* o = frames + 4 * s;
-    o[0] = make_float4(pos.x, pos.y, pos.z, eps);
-    o[1] = make_float4(nrm[0], nrm[1], nrm[2], invSign);
-    o[2] = make_float4(nx[0], nx[1], nx[2], __uint_as_float(tileRow));
-    o[3] = make_float4(ny[0], ny[1], ny[2], 0.0f);
+    const float invLen = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(nrm[0], nrm[0]), __fmul_rn(nrm[2], nrm[2]))));
+    nx[0] = __fmul_rn(__fmul_rn(-1.0f, nrm[2]), invLen);
+    nx[1] = 0.0f;
+    nx[2] = __fmul_rn(nrm[0], invLen);
   }
+  else
+  {
+    const float s2 = __fadd_rn(__fmul_rn(nrm[1], nrm[1]), __fmul_rn(nrm[2], nrm[2]));
+    const float invLen = __double2float_rn(__ddiv_rn(1.0, __dsqrt_rn((double)s2)));
+    nx[0] = 0.0f;
+    nx[1] = __fmul_rn(nrm[2], invLen);
+    nx[2] = __fmul_rn(__fmul_rn(-1.0f, nrm[1]), invLen);
+  }
+  const float ny[3] = {__fsub_rn(__fmul_rn(nrm[1], nx[2]), __fmul_rn(nrm[2], nx[1])),
+                       __fsub_rn(__fmul_rn(nrm[2], nx[0]), __fmul_rn(nrm[0], nx[2])),
+                       __fsub_rn(__fmul_rn(nrm[0], nx[1]), __fmul_rn(nrm[1], nx[0]))};
+  const float invSign = hrt::rg::dot3(nrm, nrm) > 0.0f ? 1.0f : -1.0f;
+  // std::max(a, b) = a < b ? b : a
+  const float ax = fabsf(pos.x), ay = fabsf(pos.y), az = fabsf(pos.z);
+  const float myz = ay < az ? az : ay;
+  const float mxyz = ax < myz ? myz : ax;
+  const float gEps = 2e-5f, twoGEps = __fmul_rn(2.0f, gEps);
+  const float eps = __fmul_rn(mxyz < twoGEps ? twoGEps : mxyz, gEps);
+  const uint32_t tileRow = ((y % kAoTile) * kAoTile + (x % kAoTile)) * raysPerPixel;
+  return {make_float4(pos.x, pos.y, pos.z, eps), make_float4(nrm[0], nrm[1], nrm[2], invSign),
+          make_float4(nx[0], nx[1], nx[2], __uint_as_float(tileRow)), make_float4(ny[0], ny[1], ny[2], 0.0f)};
 }
 
-// The per-ray part of kernel_InitAORay: one thread per AO ray (slot s, sample
-// z at s * raysPerPixel + z), MapSampleToCosineDistribution with the tile
-// entry's sample direction (dev: (sinT cosP, sinT sinP, cosT) per entry) and
-// OffsRayPos (examples/render_common.h:56-112).  Consecutive threads write
-// consecutive rays.
 __global__ void __launch_bounds__(kThreads)
-    k_rtao_ao_rays(const float4* __restrict__ frames, uint64_t nRays, uint32_t raysPerPixel,
-                   const float4* __restrict__ dev, float aoMaxRadius, float4* __restrict__ aoRays)
+    k_rtao_ao_rays(const uint8_t* __restrict__ flag, uint64_t n, const uint32_t* __restrict__ blockOffset,
+                   const uint32_t* __restrict__ pixel, const float4* __restrict__ positions, uint32_t width,
+                   uint32_t raysPerPixel, const float4* __restrict__ dev, float aoMaxRadius,
+                   uint32_t* __restrict__ aoPixel, uint64_t slotCapacity, float4* __restrict__ aoRays,
+                   float* __restrict__ visibility, uint32_t* __restrict__ colors, uint32_t* errorWord)
 {
-  for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < nRays; i += (uint64_t)gridDim.x * kThreads)
+  __shared__ AoFrame  s_frame[kThreads];
+  __shared__ uint32_t s_warp[kThreads / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t first = blockOffset[blockIdx.x];  // slot of the block's first flagged ray
+  const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+  const bool in = k < n, f = in && flag[k];
+  const uint32_t pix = in ? pixel[k] : 0u;
+  const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, f);
+  if (lane == 0) s_warp[warp] = __popc(ballot);
+  __syncthreads();
+  uint32_t rank = __popc(ballot & ((1u << lane) - 1u)), count = 0;
+  for (uint32_t w = 0; w < kThreads / 32; w++)
   {
-    const uint64_t s = i / raysPerPixel;
-    const uint32_t z = (uint32_t)(i - s * raysPerPixel);
-    const float4* fr = frames + 4 * s;
-    const float4 P = fr[0], N = fr[1], X = fr[2], Y = fr[3];
+    rank += w < warp ? s_warp[w] : 0u;
+    count += s_warp[w];
+  }
+  if (first + count > slotCapacity)
+  {
+    if (threadIdx.x == 0) atomicOr(errorWord, kErrLayout);
+    count = first < slotCapacity ? (uint32_t)(slotCapacity - first) : 0u;
+  }
+  if (f && rank < count)
+  {
+    aoPixel[first + rank] = pix;
+    s_frame[rank] = ao_frame(pix, positions[pix], width, raysPerPixel);
+  }
+  else if (in && !f)
+  {
+    visibility[pix] = 0.0f;
+    colors[pix] = 0u;
+  }
+  __syncthreads();
+  float4* out = aoRays + 2 * first * raysPerPixel;
+  const uint32_t rays = count * raysPerPixel;
+  for (uint32_t i = threadIdx.x; i < rays; i += kThreads)
+  {
+    const uint32_t s = i / raysPerPixel, z = i - s * raysPerPixel;
+    const float4 P = s_frame[s].p, N = s_frame[s].n, X = s_frame[s].x, Y = s_frame[s].y;
     const float nrm[3] = {N.x, N.y, N.z}, nx[3] = {X.x, X.y, X.z}, ny[3] = {Y.x, Y.y, Y.z};
     const float4 dv = dev[__float_as_uint(X.w) + z];
     float res[3];
@@ -377,9 +374,9 @@ __global__ void __launch_bounds__(kThreads)
                            __fmul_rn(nrm[c], dv.z));
     }
     const float se = __fmul_rn(hrt::rg::dot3(res, nrm) < 0.0f ? -1.0f : 1.0f, P.w);
-    aoRays[2 * i + 0] = make_float4(__fadd_rn(P.x, __fmul_rn(se, nrm[0])), __fadd_rn(P.y, __fmul_rn(se, nrm[1])),
-                                    __fadd_rn(P.z, __fmul_rn(se, nrm[2])), 0.0f);
-    aoRays[2 * i + 1] = make_float4(res[0], res[1], res[2], aoMaxRadius);
+    out[2 * i + 0] = make_float4(__fadd_rn(P.x, __fmul_rn(se, nrm[0])), __fadd_rn(P.y, __fmul_rn(se, nrm[1])),
+                                 __fadd_rn(P.z, __fmul_rn(se, nrm[2])), 0.0f);
+    out[2 * i + 1] = make_float4(res[0], res[1], res[2], aoMaxRadius);
   }
 }
 
@@ -499,7 +496,6 @@ struct hrt_frame
   // AO pass
   float4*   aoRays = nullptr;
   uint32_t* aoPixel = nullptr;
-  float4*   frames = nullptr;  // per slot: the pixel's AO frame (k_rtao_frames)
   uint8_t*  aoHit = nullptr;
   uint64_t  slotCap = 0, aoCap = 0;
   // sample tile: sample directions per entry
@@ -512,7 +508,7 @@ struct hrt_frame
   uint32_t              geomCap = 0;
   float*                dNormMat = nullptr;
   uint32_t              normMatCap = 0;
-  // small state: total (u64) + error word, device and pinned host
+  // small state: total (u64), error word, count of finished blocks; device and pinned host
   unsigned long long* dTotal = nullptr;
   unsigned long long* hTotal = nullptr;
   // colours for a destination in pageable host memory
@@ -547,7 +543,7 @@ int ensure_pixels(hrt_frame* f, uint64_t n)
     return st;
   }
   f->pixCap = n;
-  const uint64_t blocks = (n + kThreads * kChunk - 1) / (kThreads * kChunk);
+  const uint64_t blocks = (n + kThreads - 1) / kThreads;
   if (blocks > f->blockCap)
   {
     if ((st = grow(ctx, (void**)&f->blockCount, 4 * blocks))) return st;
@@ -661,7 +657,7 @@ int hrt_frame_destroy(hrt_frame* f)
   if (!f) return HRT_ERR_INVALID_ARGUMENT;
   cudaSetDevice(f->ctx->device);
   void* dev[] = {f->rays, f->pixel, f->hits, f->positions, f->flag, f->visibility, f->blockCount, f->aoRays,
-                 f->aoPixel, f->aoHit, f->dev, f->dGeoms, f->dNormMat, f->dTotal, f->colorBuf, f->frames};
+                 f->aoPixel, f->aoHit, f->dev, f->dGeoms, f->dNormMat, f->dTotal, f->colorBuf};
   for (void* p : dev)
     if (p) cudaFree(p);
   for (float4* p : f->normals)
@@ -799,17 +795,15 @@ int hrt_frame_render_rtao(hrt_frame* f, hrt_scene* s, const hrt_rtao_params* prm
   std::memcpy(p.m, prm->projInv, sizeof(p.m));
   std::memcpy(v.m, prm->worldViewInv, sizeof(v.m));
   const int packed = (prm->width % 8 == 0 && prm->height % 8 == 0) ? 1 : 0;
-  const uint32_t grid = grid_for(n, ctx->numSMs);
-  k_frame_eye_rays<<<grid, kThreads, 0, cs>>>(p, v, prm->width, prm->height, packed, prm->zNear, prm->zFar, f->rays,
-                                              f->pixel);
+  k_frame_eye_rays<<<grid_for(n, ctx->numSMs), kThreads, 0, cs>>>(p, v, prm->width, prm->height, packed, prm->zNear,
+                                                                  prm->zFar, f->rays, f->pixel);
   HRT_CUDA(ctx, cudaGetLastError());
   if ((st = query_eye_rays(s, reinterpret_cast<const float*>(f->rays), n, packed ? 0 : (int)prm->width, f->hits, cs)))
     return st;
-  k_rtao_positions<<<grid, kThreads, 0, cs>>>(f->rays, f->hits, f->pixel, n, f->dGeoms, (uint32_t)hg.size(),
-                                              f->dNormMat, nInst, f->positions, f->flag, dErr);
-  const uint32_t nBlocks = (uint32_t)((n + kThreads * kChunk - 1) / (kThreads * kChunk));
-  k_flag_count<<<nBlocks, kThreads, 0, cs>>>(f->flag, n, f->blockCount);
-  k_scan_counts<<<1, 1024, 0, cs>>>(f->blockCount, nBlocks, f->dTotal);
+  const uint32_t nBlocks = (uint32_t)((n + kThreads - 1) / kThreads);
+  k_rtao_positions<<<nBlocks, kThreads, 0, cs>>>(f->rays, f->hits, f->pixel, n, f->dGeoms, (uint32_t)hg.size(),
+                                                 f->dNormMat, nInst, f->positions, f->flag, f->blockCount, f->dTotal,
+                                                 dErr + 1, dErr);
   HRT_CUDA(ctx, cudaGetLastError());
   HRT_CUDA(ctx, cudaMemcpyAsync(f->hTotal, f->dTotal, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, cs));
   HRT_CUDA(ctx, cudaStreamSynchronize(cs));
@@ -822,8 +816,7 @@ int hrt_frame_render_rtao(hrt_frame* f, hrt_scene* s, const hrt_rtao_params* prm
   if (slots > f->slotCap)
   {
     f->slotCap = 0;
-    if ((st = grow(ctx, (void**)&f->aoPixel, 4 * slots)) || (st = grow(ctx, (void**)&f->frames, 64 * slots)))
-      return st;
+    if ((st = grow(ctx, (void**)&f->aoPixel, 4 * slots))) return st;
     f->slotCap = slots;
   }
   if (nAo > f->aoCap)
@@ -834,16 +827,11 @@ int hrt_frame_render_rtao(hrt_frame* f, hrt_scene* s, const hrt_rtao_params* prm
   }
   uint32_t* out = nullptr;
   if ((st = color_target(f, colors, n, &out))) return st;
-  HRT_CUDA(ctx, cudaMemsetAsync(out, 0, 4 * n, cs));
-  HRT_CUDA(ctx, cudaMemsetAsync(f->visibility, 0, 4 * n, cs));
+  k_rtao_ao_rays<<<nBlocks, kThreads, 0, cs>>>(f->flag, n, f->blockCount, f->pixel, f->positions, prm->width, R, f->dev,
+                                               prm->aoMaxRadius, f->aoPixel, slots, f->aoRays, f->visibility, out, dErr);
+  HRT_CUDA(ctx, cudaGetLastError());
   if (slots > 0)
   {
-    k_rtao_slots<<<nBlocks, kThreads, 0, cs>>>(f->flag, n, f->blockCount, f->pixel, f->aoPixel, f->slotCap, dErr);
-    k_rtao_frames<<<grid_for(slots, ctx->numSMs), kThreads, 0, cs>>>(f->aoPixel, slots, f->positions, prm->width, R,
-                                                                     f->frames);
-    k_rtao_ao_rays<<<grid_for(nAo, ctx->numSMs), kThreads, 0, cs>>>(f->frames, nAo, R, f->dev, prm->aoMaxRadius,
-                                                                    f->aoRays);
-    HRT_CUDA(ctx, cudaGetLastError());
     if ((st = hrt_query_any(s, reinterpret_cast<const float*>(f->aoRays), nAo, f->aoHit, stream))) return st;
     k_rtao_colors<<<grid_for(slots, ctx->numSMs), kThreads, 0, cs>>>(f->aoHit, f->aoPixel, slots, R, prm->power,
                                                                      f->visibility, out);
