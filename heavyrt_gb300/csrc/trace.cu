@@ -21,7 +21,10 @@ namespace
 constexpr int kSpreadWarps = 13, kResidentWarps = 36;
 // Unless the caller set a shape: idle lanes at which a warp refills, and
 // advances (phases of an instance tree's walk) between its looks at them.
-constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32;
+constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32, kTreeSteps = 4;
+// Warps an SM that hold a batch on an instance tree at once, and the batch (in
+// warps of 32 rays an SM) from which its nearest hits go by vote.
+constexpr int kTreeResidentWarps = 24, kVoteWarps = 128;
 
 // The shape of one launch.
 //
@@ -44,17 +47,31 @@ constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32;
 // and coherent ones do not care (full-HD eye rays 156 against 157).  Looks after
 // 4, 8, 16 advances: 2M occlusion rays, FP16 nodes 391, 378, 419 us, 500,000
 // random rays 496, 497, 509; after 16 and 32 phases, 240 instances 1,161, 1,154.
-TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int numSMs)
+//
+// On an instance tree lanes wait for the warp's vote only in large batches
+// (trace_impl.cuh).  Nearest hits, 8 and 100 instances, us, pool without a vote
+// against with it: binary, 170,000 rays 913, 1,091 against 1,002, 1,221; 400,000
+// 1,642, 1,627 against 1,684, 1,709; 900,000 3,282, 2,927 against 3,191, 2,864;
+// FP16 nodes 798, 914 against 847, 1,051; 1,435, 1,408 against 1,437, 1,486;
+// 2,832, 2,533 against 2,709, 2,439.  Any hits are faster without at every size
+// (binary, 900,000 rays 1,452 and 1,126 against 1,532 and 1,226), 8-bit nodes by
+// vote (129,600 eye rays, 60 instances 266 against 332).  One thread per ray, no
+// vote, while all rays are resident (100,000 rays, 100 instances, binary 924,
+// in the pool 927; FP16 764, 798; 10,000 rays 555, 681); 170,000 rays are faster
+// in the pool (1,091 against 1,340).
+TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int kind, int layout, int numSMs)
 {
   TraceConfig s = c;
+  const bool tree = a.tlasRecs != nullptr && a.rayOffsets == nullptr;
+  s.alone = tree && layout != 3 && (kind == 1 || a.n <= (uint64_t)numSMs * kVoteWarps * 32);
   if (!c.given)
   {
     if (s.refillLanes > kRefillLanes) s.refillLanes = kRefillLanes;
-    s.stepsPerRefill = a.tlasRecs != nullptr && a.rayOffsets == nullptr ? kTreePhases : kAdvances;
+    s.stepsPerRefill = !tree ? kAdvances : s.alone ? kTreeSteps : kTreePhases;
   }
   int perWarp = 32;
   while (perWarp > 1 && a.n <= (uint64_t)numSMs * kSpreadWarps * (perWarp / 2)) perWarp /= 2;
-  if (a.n <= (uint64_t)numSMs * kResidentWarps * 32)
+  if (a.n <= (uint64_t)numSMs * (tree ? kTreeResidentWarps : kResidentWarps) * 32)
   {
     s.raysPerWarp = perWarp;
     s.persistent = 0;
@@ -70,7 +87,7 @@ cudaError_t trace(const TraceArgs& a, int kind, int counting, int layout, const 
 {
   if (a.n == 0) return cudaSuccess;
   if (a.n > 0x7FFFFFFFull) return cudaErrorInvalidValue;  // the pool's counter may overshoot n by a few warps
-  const TraceConfig c = counting ? config : launch_shape(a, config, numSMs);
+  const TraceConfig c = counting ? config : launch_shape(a, config, kind, layout, numSMs);
   if (a.triTest == 1)
     switch (layout)
     {

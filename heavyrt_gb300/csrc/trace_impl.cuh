@@ -1011,91 +1011,143 @@ __device__ __forceinline__ void tlas_enter(Lane<LAYOUT>& L, const InstanceDesc* 
 // nodes: (1, 2), (2, 1), (2, 2), (4, 2), (2, 4) node and tree visits 1,239,
 // 1,219, 1,193, 1,177, 1,169 us).
 constexpr int kTlasNodeRun = 2, kTlasTreeRun = 4;
+// The same for a lane that walks without a vote, one thread per ray and in the
+// pool (63,000 rays into 100 instances, FP16 nodes, one thread per ray, (node,
+// tree) runs of (1, 1), (2, 1), (3, 1), (4, 2), (6, 6): 737, 683, 673, 755, 757
+// us; 170,000 rays in the pool 972, 1,005, 1,091, 950, 994).
+constexpr int kGridNodeRun = 3, kGridTreeRun = 1, kAloneNodeRun = 4, kAloneTreeRun = 2;
 
-// Up to `phases` phases of a warp over its lanes' rays, all 32 lanes calling
-// together.  The walk of a two-level tree has four kinds of work; in each
-// phase the warp does the kind that most of its lanes wait for, and the others
-// wait.  A lane's own order of visits does not depend on the votes; every
-// phase advances at least one lane.  A finished lane has L.cur = kDone.
-// (921,600 rays into 240 instances: 6.8 threads per instruction and 1,320 us
-// with every lane stepping at once, 13.0 and 1,190 us by vote.)
-template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
-__device__ __forceinline__ void run_phases(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, const Tlas& tl,
-                                           Stack<THREADS, STACK>& st, uint64_t& nPairs, uint64_t& nTris,
-                                           uint32_t* errorWord, int phases)
+// The walk of a two-level tree has four kinds of work.  tlas_walk_* do the one
+// that the lane waits for (as `state` of it says).
+struct TlasState
+{
+  bool tree, enter, node, leaf;
+};
+template <int LAYOUT> __device__ __forceinline__ TlasState tlas_state(const Lane<LAYOUT>& L)
+{
+  const bool live = L.cur != kDone, inTree = L.inst == kTlasMode, leaf = (L.cur & kLeafBit) != 0u;
+  const bool enter = live && inTree && (leaf || L.stale);
+  return {live && inTree && !enter, enter, live && !inTree && !leaf, live && !inTree && leaf};
+}
+
+template <int RUN, int LAYOUT, bool ANY, bool COUNT, int THREADS, int STACK>
+__device__ __forceinline__ void tlas_walk_nodes(Lane<LAYOUT>& L, Stack<THREADS, STACK>& st, uint64_t& nPairs,
+                                                uint32_t* errorWord)
 {
   constexpr int DEPTH = StackDepth<LAYOUT, true>::value;
-  for (int s = 0; s < phases; s++)
+  if (out_of_budget(L, errorWord)) L.cur = kDone;
+#pragma unroll 1
+  for (int k = 0; k < RUN && (L.cur & kLeafBit) == 0u; k++)
   {
-    const bool live = L.cur != kDone, inTree = L.inst == kTlasMode, leaf = (L.cur & kLeafBit) != 0u;
-    const bool enter = live && inTree && (leaf || L.stale), tree = live && inTree && !enter;
-    const bool atNode = live && !inTree && !leaf, atLeaf = live && !inTree && leaf;
-    const int nEnter = __popc(__ballot_sync(0xFFFFFFFFu, enter)), nTree = __popc(__ballot_sync(0xFFFFFFFFu, tree));
-    const int nNode = __popc(__ballot_sync(0xFFFFFFFFu, atNode)), nLeaf = __popc(__ballot_sync(0xFFFFFFFFu, atLeaf));
-    const int most = max(max(nEnter, nTree), max(nNode, nLeaf));
-    if (most == 0) return;
-    if (nNode == most)
+    const int r = visit_node<LAYOUT, ANY, COUNT, THREADS, DEPTH, STACK>(L, st, nPairs, errorWord);
+    if (r < 0) L.cur = kDone;
+    else if (r == 1)
     {
-      if (atNode)
-      {
-        if (out_of_budget(L, errorWord)) L.cur = kDone;
-#pragma unroll 1
-        for (int k = 0; k < kTlasNodeRun && (L.cur & kLeafBit) == 0u; k++)
-        {
-          const int r = visit_node<LAYOUT, ANY, COUNT, THREADS, DEPTH, STACK>(L, st, nPairs, errorWord);
-          if (r < 0) L.cur = kDone;
-          else if (r == 1)
-          {
-            if (L.top > L.base)
-            {
-              L.top--;
-              L.cur = st.get(L.top);
-            }
-            else
-            {
-              tlas_leave(L, st);
-              break;
-            }
-          }
-        }
-      }
-    }
-    else if (nTree == most)
-    {
-      if (tree)
-      {
-        if (out_of_budget(L, errorWord)) L.cur = kDone;
-#pragma unroll 1
-        for (int k = 0; k < kTlasTreeRun && (L.cur & kLeafBit) == 0u; k++)
-        {
-          const int r = visit_pair<COUNT, THREADS, DEPTH, STACK, LAYOUT>(L, L.r, tl.recs, st, nPairs, errorWord);
-          if (r < 0) L.cur = kDone;
-          else if (r == 1) tlas_pop(L, st);
-        }
-      }
-    }
-    else if (nEnter == most)
-    {
-      if (enter)
-      {
-        if (out_of_budget(L, errorWord)) L.cur = kDone;
-        else tlas_enter<LAYOUT, THREADS, STACK>(L, inst, tl, st);
-      }
-    }
-    else if (atLeaf)
-    {
-      if (out_of_budget(L, errorWord) ||
-          (L.cur != kEmptyRef &&
-           test_leaf<TRI, ANY, COUNT, EndBit<LAYOUT>::value>(L.tris, L.cur & ~kLeafBit, L.r, L.h, L.inst, nTris)))
-        L.cur = kDone;
-      else if (L.top > L.base)
+      if (L.top > L.base)
       {
         L.top--;
         L.cur = st.get(L.top);
       }
       else
+      {
         tlas_leave(L, st);
+        break;
+      }
     }
+  }
+}
+
+template <int RUN, int LAYOUT, bool COUNT, int THREADS, int STACK>
+__device__ __forceinline__ void tlas_walk_tree(Lane<LAYOUT>& L, const Tlas& tl, Stack<THREADS, STACK>& st,
+                                               uint64_t& nPairs, uint32_t* errorWord)
+{
+  constexpr int DEPTH = StackDepth<LAYOUT, true>::value;
+  if (out_of_budget(L, errorWord)) L.cur = kDone;
+#pragma unroll 1
+  for (int k = 0; k < RUN && (L.cur & kLeafBit) == 0u; k++)
+  {
+    const int r = visit_pair<COUNT, THREADS, DEPTH, STACK, LAYOUT>(L, L.r, tl.recs, st, nPairs, errorWord);
+    if (r < 0) L.cur = kDone;
+    else if (r == 1) tlas_pop(L, st);
+  }
+}
+
+template <int LAYOUT, int THREADS, int STACK>
+__device__ __forceinline__ void tlas_walk_enter(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, const Tlas& tl,
+                                                const Stack<THREADS, STACK>& st, uint32_t* errorWord)
+{
+  if (out_of_budget(L, errorWord)) L.cur = kDone;
+  else tlas_enter<LAYOUT, THREADS, STACK>(L, inst, tl, st);
+}
+
+template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
+__device__ __forceinline__ void tlas_walk_leaf(Lane<LAYOUT>& L, const Stack<THREADS, STACK>& st, uint64_t& nTris,
+                                               uint32_t* errorWord)
+{
+  if (out_of_budget(L, errorWord) ||
+      (L.cur != kEmptyRef &&
+       test_leaf<TRI, ANY, COUNT, EndBit<LAYOUT>::value>(L.tris, L.cur & ~kLeafBit, L.r, L.h, L.inst, nTris)))
+    L.cur = kDone;
+  else if (L.top > L.base)
+  {
+    L.top--;
+    L.cur = st.get(L.top);
+  }
+  else
+    tlas_leave(L, st);
+}
+
+// Up to `phases` phases of a warp over its lanes' rays, all 32 lanes calling
+// together: in each phase the warp does the kind of work that most of its lanes
+// wait for, and the others wait.  A lane's own order of visits does not depend
+// on the votes; every phase advances at least one lane.  A finished lane has
+// L.cur = kDone.  (921,600 rays into 240 instances: 6.8 threads per instruction
+// and 1,320 us with every lane stepping at once, 13.0 and 1,190 us by vote.)
+template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
+__device__ __forceinline__ void run_phases(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, const Tlas& tl,
+                                           Stack<THREADS, STACK>& st, uint64_t& nPairs, uint64_t& nTris,
+                                           uint32_t* errorWord, int phases)
+{
+  for (int s = 0; s < phases; s++)
+  {
+    const TlasState a = tlas_state(L);
+    const int nEnter = __popc(__ballot_sync(0xFFFFFFFFu, a.enter)), nTree = __popc(__ballot_sync(0xFFFFFFFFu, a.tree));
+    const int nNode = __popc(__ballot_sync(0xFFFFFFFFu, a.node)), nLeaf = __popc(__ballot_sync(0xFFFFFFFFu, a.leaf));
+    const int most = max(max(nEnter, nTree), max(nNode, nLeaf));
+    if (most == 0) return;
+    if (nNode == most)
+    {
+      if (a.node) tlas_walk_nodes<kTlasNodeRun, LAYOUT, ANY, COUNT>(L, st, nPairs, errorWord);
+    }
+    else if (nTree == most)
+    {
+      if (a.tree) tlas_walk_tree<kTlasTreeRun, LAYOUT, COUNT>(L, tl, st, nPairs, errorWord);
+    }
+    else if (nEnter == most)
+    {
+      if (a.enter) tlas_walk_enter(L, inst, tl, st, errorWord);
+    }
+    else if (a.leaf)
+      tlas_walk_leaf<LAYOUT, TRI, ANY, COUNT>(L, st, nTris, errorWord);
+  }
+}
+
+// Up to `steps` steps of a lane's walk with no vote, a run of each kind of work
+// that it comes to.  A batch that does not fill the machine is bound by its
+// slowest warps' chains, and lanes that wait for a vote make them longer
+// (63,000 rays into 100 instances, nearest and any hits: binary 1,012 and 563
+// us by vote, 857 and 408 so; FP16 nodes 758, 368; 674, 318).
+template <int NODES, int PAIRS, int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
+__device__ __forceinline__ void run_alone(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, const Tlas& tl,
+                                          Stack<THREADS, STACK>& st, uint64_t& nPairs, uint64_t& nTris,
+                                          uint32_t* errorWord, int steps)
+{
+  for (int k = 0; k < steps && L.cur != kDone; k++)
+  {
+    if (tlas_state(L).tree) tlas_walk_tree<PAIRS, LAYOUT, COUNT>(L, tl, st, nPairs, errorWord);
+    if (tlas_state(L).enter) tlas_walk_enter(L, inst, tl, st, errorWord);
+    if (tlas_state(L).node) tlas_walk_nodes<NODES, LAYOUT, ANY, COUNT>(L, st, nPairs, errorWord);
+    if (tlas_state(L).leaf) tlas_walk_leaf<LAYOUT, TRI, ANY, COUNT>(L, st, nTris, errorWord);
   }
 }
 
@@ -1186,7 +1238,7 @@ template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, bool TLAS, int
 __global__ void __launch_bounds__(THREADS, TLAS ? 768 / THREADS : 0) k_trace_pool(const float4* __restrict__ rays, uint32_t n,
                                                         const InstanceDesc* __restrict__ inst, Segments sg, Tlas tl,
                                                         void* out, unsigned long long* counters, uint32_t* errorWord,
-                                                        unsigned int* rayCounter, int steps, int refill,
+                                                        unsigned int* rayCounter, int steps, int refill, int alone,
                                                         int stackShared, RayOrder order)
 {
   extern __shared__ uint32_t s_stack[];  // stackShared * THREADS entries
@@ -1228,7 +1280,9 @@ __global__ void __launch_bounds__(THREADS, TLAS ? 768 / THREADS : 0) k_trace_poo
         }
       }
     }
-    if (TLAS)
+    if (TLAS && alone)
+      run_alone<kAloneNodeRun, kAloneTreeRun, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, steps);
+    else if (TLAS)
       run_phases<LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, steps);
     else if (L.cur != kDone)
     {
@@ -1269,8 +1323,7 @@ __global__ void __launch_bounds__(THREADS) k_trace_grid(const float4* __restrict
       while (!out_of_budget(L, errorWord) &&
              !step<LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord)) {}
   }
-  if (TLAS)
-    run_phases<LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, 0x7FFFFFFF);
+  if (TLAS) run_alone<kGridNodeRun, kGridTreeRun, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, 0x7FFFFFFF);
   if (i != kNoRay) write_result<ANY>(L, inst, out);
   flush_counters<COUNT>(nPairs, nTris, counters);
 }
@@ -1595,7 +1648,7 @@ cudaError_t launch(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStr
     if (e != cudaSuccess) return e;
     k_trace_pool<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK><<<(uint32_t)blocks, THREADS, smem, s>>>(
         a.rays, n, a.inst, sg, tl, a.hits, a.counters, a.errorWord, a.rayCounter, c.stepsPerRefill, c.refillLanes,
-        shared, order);
+        c.alone, shared, order);
   }
   else
   {
