@@ -22,9 +22,10 @@ constexpr int kSpreadWarps = 13, kResidentWarps = 36;
 // Unless the caller set a shape: idle lanes at which a warp refills, and
 // advances (phases of an instance tree's walk) between its looks at them.
 constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32, kTreeSteps = 4;
-// Warps an SM that hold a batch on an instance tree at once, and the batch (in
-// warps of 32 rays an SM) from which its nearest hits go by vote.
-constexpr int kTreeResidentWarps = 24, kVoteWarps = 128;
+// The same on an instance tree, and (4-wide nodes) on a transformed instance or
+// several in turn, whose lanes hold more registers; the batch on a tree (in
+// warps of 32 rays an SM) from which nearest hits go by vote.
+constexpr int kTreeResidentWarps = 24, kGeneralResidentWarps = 18, kVoteWarps = 128;
 
 // The shape of one launch.
 //
@@ -58,7 +59,9 @@ constexpr int kTreeResidentWarps = 24, kVoteWarps = 128;
 // vote (129,600 eye rays, 60 instances 266 against 332).  One thread per ray, no
 // vote, while all rays are resident (100,000 rays, 100 instances, binary 924,
 // in the pool 927; FP16 764, 798; 10,000 rays 555, 681); 170,000 rays are faster
-// in the pool (1,091 against 1,340).
+// in the pool (1,091 against 1,340).  One transformed instance, binary: 150,000
+// rays 159 us in the pool, 203 one thread per ray; 90,000, watertight, 165, 157.
+// Eight in turn, FP32 nodes, watertight: 100,000 rays 626, 852.
 TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int kind, int layout, int numSMs)
 {
   TraceConfig s = c;
@@ -71,7 +74,10 @@ TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int kind, int
   }
   int perWarp = 32;
   while (perWarp > 1 && a.n <= (uint64_t)numSMs * kSpreadWarps * (perWarp / 2)) perWarp /= 2;
-  if (a.n <= (uint64_t)numSMs * (tree ? kTreeResidentWarps : kResidentWarps) * 32)
+  const int resident = !tree && (a.one || a.rayOffsets) ? kResidentWarps
+                       : tree || layout == 0            ? kTreeResidentWarps
+                                                        : kGeneralResidentWarps;
+  if (a.n <= (uint64_t)numSMs * resident * 32)
   {
     s.raysPerWarp = perWarp;
     s.persistent = 0;

@@ -907,9 +907,14 @@ template <int LAYOUT> __device__ __forceinline__ void tlas_begin(Lane<LAYOUT>& L
 // per step against this: 4M occlusion rays, FP16 nodes 632 -> 580 (runs of 3
 // and 4: 597, 628); 1M random rays, 8-bit nodes 1,646 -> 1,482 (runs of 2 and
 // 4: 1,587, 1,530); full-HD eye rays, binary 255 -> 215 (a run of 4: 217).
-template <int LAYOUT, bool ANY> struct NodeRun
+// Watertight any hits are faster at 3 in 4-wide trees (1M random rays, 20,000
+// triangles, 8-bit nodes 617 -> 583, FP16 506 -> 479), and one thread per ray
+// in binary ones at 2 (100,000 rays, 20,000 and 500,000 triangles 165 and 438
+// us at 6, 141 and 349 at 2, 153 and 364 at 1; in the pool 6 and 2 are even).
+template <int LAYOUT, int TRI, bool ANY, bool GRID> struct NodeRun
 {
-  static constexpr int value = LAYOUT == 0 ? 6 : (ANY ? 2 : 3);
+  static constexpr bool wt = TRI == 1 && ANY;
+  static constexpr int  value = LAYOUT == 0 ? (wt && GRID ? 2 : 6) : (ANY && !wt ? 2 : 3);
 };
 
 // Stride of the pools' step loops.  It changes nothing but the registers that
@@ -917,12 +922,12 @@ template <int LAYOUT, bool ANY> struct NodeRun
 // 694 at the run's length; FP16 nodes, Moller-Trumbore: 501 at 1, 523).
 template <int LAYOUT, bool ANY> struct PoolStep
 {
-  static constexpr int value = LAYOUT == 0 ? NodeRun<LAYOUT, ANY>::value : 1;
+  static constexpr int value = LAYOUT == 0 ? 6 : 1;
 };
 
 // One advance of a lane that walks its instances in order: nodes, then a leaf
 // when it holds one.  Returns true when the lane's ray is finished.
-template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
+template <bool GRID, int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
 __device__ __forceinline__ bool step(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, Stack<THREADS, STACK>& st,
                                      uint64_t& nPairs, uint64_t& nTris, uint32_t* errorWord)
 {
@@ -934,7 +939,7 @@ __device__ __forceinline__ bool step(Lane<LAYOUT>& L, const InstanceDesc* __rest
     return false;
   };
 #pragma unroll 1
-  for (int k = 0; k < NodeRun<LAYOUT, ANY>::value; k++)
+  for (int k = 0; k < NodeRun<LAYOUT, TRI, ANY, GRID>::value; k++)
   {
     if ((L.cur & kLeafBit) != 0u) break;
     const int r = visit_node<LAYOUT, ANY, COUNT, THREADS, DEPTH, STACK>(L, st, nPairs, errorWord);
@@ -1289,7 +1294,7 @@ __global__ void __launch_bounds__(THREADS, TLAS ? 768 / THREADS : 0) k_trace_poo
       for (int s = 0; s < steps * kStep; s += kStep)
       {
         if (out_of_budget(L, errorWord) ||
-            step<LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord))
+            step<false, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord))
         {
           L.cur = kDone;
           break;
@@ -1321,7 +1326,7 @@ __global__ void __launch_bounds__(THREADS) k_trace_grid(const float4* __restrict
     if (TLAS) tlas_begin(L);
     else if (begin_instance<LAYOUT>(L, inst, first_instance(L, i, sg)))
       while (!out_of_budget(L, errorWord) &&
-             !step<LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord)) {}
+             !step<true, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord)) {}
   }
   if (TLAS) run_alone<kGridNodeRun, kGridTreeRun, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, 0x7FFFFFFF);
   if (i != kNoRay) write_result<ANY>(L, inst, out);
@@ -1398,13 +1403,13 @@ __device__ __forceinline__ void start_ray_one(Lane1<LAYOUT>& L, uint32_t i, cons
 
 // One advance of the single-instance kernel (nodes, then a leaf when the lane
 // holds one); true when the ray is finished.
-template <int LAYOUT, int TRI, bool ANY, int THREADS, int STACK>
+template <bool GRID, int LAYOUT, int TRI, bool ANY, int THREADS, int STACK>
 __device__ __forceinline__ bool step_one(Lane1<LAYOUT>& L, Stack<THREADS, STACK>& st, uint32_t* errorWord)
 {
   constexpr int DEPTH = StackDepth<LAYOUT, false>::value;
   uint64_t none = 0;
 #pragma unroll 1
-  for (int k = 0; k < NodeRun<LAYOUT, ANY>::value; k++)
+  for (int k = 0; k < NodeRun<LAYOUT, TRI, ANY, GRID>::value; k++)
   {
     if ((L.cur & kLeafBit) != 0u) break;
     const int r = visit_node<LAYOUT, ANY, false, THREADS, DEPTH, STACK>(L, st, none, errorWord);
@@ -1488,7 +1493,7 @@ __global__ void __launch_bounds__(THREADS) k_trace_one(const float4* __restrict_
     {
       for (int s = 0; s < steps * kStep; s += kStep)
       {
-        if (out_of_budget(L, errorWord) || step_one<LAYOUT, TRI, ANY, THREADS, STACK>(L, st, errorWord))
+        if (out_of_budget(L, errorWord) || step_one<false, LAYOUT, TRI, ANY, THREADS, STACK>(L, st, errorWord))
         {
           L.cur = kDone;
           break;
@@ -1517,7 +1522,7 @@ __global__ void __launch_bounds__(THREADS)
   L.tris = src.tris;
   start_ray_one<SEG>(L, i, rays, src);
   if (L.cur != kDone)
-    while (!out_of_budget(L, errorWord) && !step_one<LAYOUT, TRI, ANY, THREADS, STACK>(L, st, errorWord)) {}
+    while (!out_of_budget(L, errorWord) && !step_one<true, LAYOUT, TRI, ANY, THREADS, STACK>(L, st, errorWord)) {}
   write_result_one<ANY, SEG>(L, src, out);
 }
 
