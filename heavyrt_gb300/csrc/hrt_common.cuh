@@ -104,9 +104,6 @@ struct BuildParams
 // (core/builders/lbvh.cpp:220-221,374-378,475-476): returns b on ties.
 __device__ __forceinline__ float lm_min(float a, float b) { return (a < b) ? a : b; }
 __device__ __forceinline__ float lm_max(float a, float b) { return (a > b) ? a : b; }
-// std::min / std::max as the slab test uses them (core/raytrace_common.h:72-75).
-__device__ __forceinline__ float std_min(float a, float b) { return (b < a) ? b : a; }
-__device__ __forceinline__ float std_max(float a, float b) { return (a < b) ? b : a; }
 
 __device__ __forceinline__ uint32_t pack_offset_and_size(uint32_t start, uint32_t size)
 {

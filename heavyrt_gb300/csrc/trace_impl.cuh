@@ -537,8 +537,6 @@ __device__ __forceinline__ void load_piece(const void* p, uint32_t (&v)[8])
       : "l"(p));
 }
 
-__device__ __forceinline__ float2 h2f(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
-
 // Entry and exit distances of the four child boxes (RayBoxIntersection2,
 // core/raytrace_common.h:67-80: the differences, products and their rounding
 // are the reference's; min and max as explained above) and the child

@@ -455,9 +455,9 @@ int hrt_server_scene_state(hrt_server* server, uint32_t sceneId, double timeoutS
 int hrt_server_remove_scene(hrt_server* server, uint32_t sceneId);
 /* Queues a request: n rays (host, 8 floats each) against one scene; kind 0
  * writes hrt_hit[n] to out, kind 1 uint8_t[n].  Both arrays must stay valid
- * until the request is waited for.  A request batched alone whose rays are
- * page-locked is traced from them in place (its any-hit flags written in
- * place when out is page-locked); otherwise the rays are copied in.  Ray
+ * until the request is waited for.  Page-locked rays at a 16-byte boundary are
+ * read in place, others are copied in; a request batched alone has its results
+ * written in place when out is page-locked (hits at a 16-byte boundary).  Ray
  * batches run at the highest stream priority, scene builds at the lowest. */
 int hrt_server_submit(hrt_server* server, uint32_t sceneId, int kind, const float* rays, uint64_t n, void* out,
                       uint64_t* ticket);
