@@ -1,7 +1,8 @@
-// Leaves, triangle records and bottom-up boxes of the LBVH in one kernel, for a
-// single geometry and for a segmented batch.
+// Leaves, triangle records and bottom-up boxes of the LBVH, for a single geometry
+// and for a segmented batch: a kernel over slices of leaves, and the walks above
+// the slices in tiers.
 //
-// A block owns the leaves [lo, hi) of one slice, a thread each.
+// A block of k_leaf_tree owns the leaves [lo, hi) of one slice, a thread each.
 //
 // Leaves (kernel1D_MakeLeavesFromTriangles, core/builders/lbvh.cpp:350-384):
 // leaf i is node L-1+i, its box the union of its run's triangle boxes taken in
@@ -24,9 +25,10 @@
 // an earlier kernel.
 //
 // What bounds it: the walks are chains of dependent steps and the leaves are
-// gathers and AoS writes.  As a kernel of leaves, a thread per leaf with its own 48-byte
-// stores, and one of walks with links and boxes read from L2, the 2M-triangle
-// heightfield took 93 + 107 us; in one kernel 153; in this one and k_climb 101 + 32.
+// gathers and AoS writes.  As a kernel of leaves, a thread per leaf with its own
+// 48-byte stores, and one of walks with links and boxes read from L2, the
+// 2M-triangle heightfield took 93 + 107 us; in one kernel 153; in this one and
+// k_climb 101 + 32.
 #pragma once
 
 #include "build_common.cuh"
@@ -377,9 +379,9 @@ __global__ void __launch_bounds__(kSlice, 3) k_leaf_tree(LeafTree a)
 // With links, boxes and arrival counters in L2, one kernel, a level was two
 // latencies and a release at device scope: 41 us for 2M triangles, 40 for
 // 500,000, 24 for 15,000; so 32 (three tiers), 22 and 8.
-// a slot's link: its parent's slot, its side there, what it is
-constexpr uint32_t kLinkSlot = 0xFFFu, kLinkRight = 1u << 12, kLinkOut = 1u << 13, kLinkIn = 1u << 14,
-                   kLinkRoot = 1u << 15, kLinkArrived = 1u << 16;
+// a slot's link: its parent's slot (below kSlots), its side there, what it is
+constexpr uint32_t kLinkRight = 1u << 12, kLinkOut = 1u << 13, kLinkIn = 1u << 14, kLinkRoot = 1u << 15,
+                   kLinkArrived = 1u << 16;
 
 struct ClimbShared
 {
