@@ -803,8 +803,13 @@ __device__ __forceinline__ int visit_node(LaneT& L, Stack<THREADS, STACK>& st, u
   if constexpr (LAYOUT != 0)
   {
     // 4-wide node: HeavyRT's BVH4 order (core/BVH4CommonRT.cpp:49-246).  An
-    // unused slot (kEmptyRef, a box that is the point 0) may pass the test for
-    // a ray through that point: it then counts as a leaf without triangles.
+    // unused slot (kEmptyRef; its box is a point: 0, or the corner of an 8-bit
+    // node's frame) may pass the test for a ray through that point.  For any
+    // hits it then counts as a leaf without triangles.  Nearest hits leave it
+    // out: the network that sorts the children is not stable, so one key more
+    // can swap children of equal entry distance, and with them the triangle
+    // that a ray through a shared edge reports.  Slot 1 may be unused only in
+    // the node of a lone leaf, where nothing can be swapped.
     using N = typename Node4Type<LAYOUT>::type;
     float key[4], tf[4];
     uint4 r4;
@@ -813,7 +818,8 @@ __device__ __forceinline__ int visit_node(LaneT& L, Stack<THREADS, STACK>& st, u
     uint32_t ref[4] = {r4.x, r4.y, r4.z, r4.w};
     bool hit[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) hit[k] = box_hit(key[k], tf[k], L.r.tNear, L.h.t);
+    for (int k = 0; k < 4; k++)
+      hit[k] = box_hit(key[k], tf[k], L.r.tNear, L.h.t) && (ANY || k < 2 || ref[k] != kEmptyRef);
     // at most three pushes; near the stack's bound they are counted first
     if (L.top > DEPTH - 3 && L.top + (int)hit[0] + (int)hit[1] + (int)hit[2] + (int)hit[3] - 1 > DEPTH)
     {
