@@ -12,9 +12,9 @@
 // Slab distances only feed comparisons (hit tests, near-first choice, pruning
 // against the current t), so the slab test takes min/max with the hardware
 // fminf/fmaxf instead of the reference's std::min/std::max selects: the two
-// differ only in the sign of a zero result (and for NaN, which finite rays
-// never produce because SafeInverse keeps |1/d| <= 1e36), and +0 == -0 in
-// every comparison, so every decision is unchanged.
+// differ only in the sign of a zero result and in one axis whose distances are
+// NaN (finite rays have none, because SafeInverse keeps |1/d| <= 1e36), and
+// +0 == -0 in every comparison, so every decision is unchanged.
 //
 // Scheduling: a persistent warp pool.  Each warp keeps one ray per lane; when
 // enough lanes have finished, the warp refills them from a global ray counter
@@ -728,11 +728,31 @@ template <int LAYOUT> struct EndBit
   static constexpr uint32_t value = LAYOUT == 0 ? 1u : 2u;  // flag bit that ends a leaf of this layout
 };
 
+// min and max of which either gives NaN when an operand is NaN.
+__device__ __forceinline__ float max_or_nan(float a, float b)
+{
+  float v;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(v) : "f"(a), "f"(b));
+  return v;
+}
+
+__device__ __forceinline__ float min_or_nan(float a, float b)
+{
+  float v;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(v) : "f"(a), "f"(b));
+  return v;
+}
+
 // A box is entered when its interval meets the ray's: tn <= tf, tf >= tNear,
 // tn <= t (core/raytrace_common.h:67-80).  Taken as one comparison of the
 // clamped ends, which also asks tNear <= t: without that no triangle can be
-// accepted.
-__device__ __forceinline__ bool box_hit(float tn, float tf, float tNear, float t) { return fmaxf(tn, tNear) <= fminf(tf, t); }
+// accepted.  Each of those comparisons fails on a NaN, and so does this one: the
+// ends keep a NaN operand (a ray without a number for its origin, tNear or t
+// ends at the root; with a min and max that drop it, it walked the whole tree).
+__device__ __forceinline__ bool box_hit(float tn, float tf, float tNear, float t)
+{
+  return max_or_nan(tn, tNear) <= min_or_nan(tf, t);
+}
 
 // Visits the internal node L.cur: tests its children, continues with the
 // nearest hit child (child 0 on equal entry distance) and pushes the others,
