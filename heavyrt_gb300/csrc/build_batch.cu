@@ -83,14 +83,14 @@ __global__ void __launch_bounds__(kThreads) k_seg_read_inputs(BatchBuffers b)
   const bool aligned = (reinterpret_cast<uintptr_t>(raw) & 15u) == 0u;
   if (b.rawStride == 12 && aligned)
   {
-    __shared__ float s_raw[3 * kBatchBoxChunk];
+    __shared__ float4 s_raw[3 * kBatchBoxChunk / 4];
+    float* words = reinterpret_cast<float*>(s_raw);
     const uint32_t pieces = 3 * n / 4;  // whole 16-byte pieces
 #pragma unroll 6
-    for (uint32_t q = threadIdx.x; q < pieces; q += kThreads)
-      reinterpret_cast<float4*>(s_raw)[q] = reinterpret_cast<const float4*>(raw)[q];
-    for (uint32_t q = 4 * pieces + threadIdx.x; q < 3 * n; q += kThreads) s_raw[q] = reinterpret_cast<const float*>(raw)[q];
+    for (uint32_t q = threadIdx.x; q < pieces; q += kThreads) s_raw[q] = reinterpret_cast<const float4*>(raw)[q];
+    for (uint32_t q = 4 * pieces + threadIdx.x; q < 3 * n; q += kThreads) words[q] = reinterpret_cast<const float*>(raw)[q];
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += kThreads) take(i, s_raw[3 * i], s_raw[3 * i + 1], s_raw[3 * i + 2]);
+    for (uint32_t i = threadIdx.x; i < n; i += kThreads) take(i, words[3 * i], words[3 * i + 1], words[3 * i + 2]);
   }
   else if (b.rawStride == 16 && aligned)
   {
