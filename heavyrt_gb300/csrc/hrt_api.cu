@@ -1111,6 +1111,10 @@ static int add_batch(hrt_scene* s, uint32_t count, BatchInputs in, uint32_t* fir
       return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "a geometry's index count is not a multiple of 3");
     if ((in.iOff[i + 1] - in.iOff[i]) / 3 > HRT_MAX_TRIS_PER_GEOM)
       return fail(ctx, HRT_ERR_CAPACITY, "more than 2^24-1 triangles in one geometry");
+    // no index can be in range; the kernels read vertex 0 of the geometry in a
+    // bad one's place, which lies past the batch's vertices if it is the last
+    if (in.iOff[i + 1] > in.iOff[i] && in.vOff[i + 1] == in.vOff[i])
+      return fail(ctx, HRT_ERR_INVALID_ARGUMENT, "a geometry of the batch has triangles but no vertices");
   }
   const uint64_t V = in.vOff[count], nIdx = in.iOff[count];
   for (uint32_t i = 0; i < (in.joined ? 1u : count); i++)
