@@ -136,11 +136,25 @@ bool is_identity(const float* m)
   return true;
 }
 
+// Kernels read a build's inputs where the caller has them.  A build that fails
+// after its first launch therefore waits for its stream before it returns: the
+// caller may free the arrays at once.
+struct InputsInUse
+{
+  cudaStream_t stream;
+  bool         idle = false;  // the stream was waited for at the end
+  ~InputsInUse()
+  {
+    if (!idle) cudaStreamSynchronize(stream);
+  }
+};
+
 int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, const uint32_t* idx, uint64_t nIdx,
                    uint64_t stride, int layout, int triTest)
 {
   hrt_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
+  InputsInUse inputs{st};
   const uint32_t N = (uint32_t)(nIdx / 3);
   g.nTris = N;
   g.triTest = triTest;
@@ -165,6 +179,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
     if (rc != HRT_OK) return rc;
     if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
     HRT_CUDA(ctx, cudaStreamSynchronize(st));
+    inputs.idle = true;
     for (int c = 0; c < 4; c++)
     {
       g.box[c] = INFINITY;
@@ -276,6 +291,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   HRT_CUDA(ctx, cudaFreeAsync(visit, st));
   HRT_CUDA(ctx, cudaFreeAsync(scratch, st));
   HRT_CUDA(ctx, cudaStreamSynchronize(st));
+  inputs.idle = true;
   cudaEventElapsedTime(&g.buildMs, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -339,6 +355,9 @@ int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geo
   // one table for the device: source addresses, then the offsets of vertices,
   // triangles, vertex chunks and index chunks
   std::vector<uint64_t> table(2 * (size_t)G + 2 * ((size_t)G + 1));
+  std::vector<BuildParams> hp(G);
+  std::vector<uint32_t> ho(4 * ((size_t)G + 1) + 8), hostCounts;
+  InputsInUse inputs{st};  // of the arrays above too
   uint64_t* srcV = table.data();
   uint64_t* srcI = srcV + G;
   uint32_t* hv = reinterpret_cast<uint32_t*>(srcI + G);
@@ -445,8 +464,6 @@ int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geo
   HRT_CUDA(ctx, cudaEventRecord(e0, st));
   cudaError_t be = build_lbvh_batch(b, ctx->numSMs, st);
   if (be != cudaSuccess) return cuda_fail(ctx, be, "build_lbvh_batch");
-  std::vector<BuildParams> hp(G);
-  std::vector<uint32_t> ho(4 * ((size_t)G + 1) + 8);
   HRT_CUDA(ctx, cudaMemcpyAsync(ho.data(), offs, sizeof(uint32_t) * ho.size(), cudaMemcpyDeviceToHost, st));
   HRT_CUDA(ctx, cudaMemcpyAsync(hp.data(), b.params, sizeof(BuildParams) * G, cudaMemcpyDeviceToHost, st));
   HRT_CUDA(ctx, cudaStreamSynchronize(st));
@@ -482,7 +499,7 @@ int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geo
     q.mergeMode = s->bvh4Merge;
     q.collapse = s->bvh4Collapse;
     HRT_CUDA(ctx, cudaMallocAsync(&scratch4, bvh4_batch_scratch_bytes(nInt, G), st));
-    std::vector<uint32_t> hostCounts(2 * (size_t)G + 1);
+    hostCounts.resize(2 * (size_t)G + 1);
     HRT_CUDA(ctx, bvh4_plan_batch(q, nInt, scratch4, hostCounts.data(), hostCounts.data() + G, b.errorWord, ctx->numSMs, st));
     HRT_CUDA(ctx, cudaStreamSynchronize(st));
     for (uint32_t i = 0; i < G; i++)
@@ -513,6 +530,7 @@ int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geo
   HRT_CUDA(ctx, cudaFreeAsync(boxPartial, st));
   if (scratch4) HRT_CUDA(ctx, cudaFreeAsync(scratch4, st));
   HRT_CUDA(ctx, cudaStreamSynchronize(st));
+  inputs.idle = true;
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
@@ -675,6 +693,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
 {
   hrt_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
+  InputsInUse inputs{st};
   const uint32_t N = g.nTris;
   const uint64_t nVert = g.nVerts;
   const uint8_t* src = nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos)) : nullptr;
@@ -692,6 +711,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
     if (rc != HRT_OK) return rc;
     if (raw) HRT_CUDA(ctx, cudaFreeAsync(raw, st));
     HRT_CUDA(ctx, cudaStreamSynchronize(st));
+    inputs.idle = true;
     return HRT_OK;
   }
   uint32_t *dIdx = nullptr, *parent = nullptr, *visit = nullptr;
@@ -773,6 +793,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   HRT_CUDA(ctx, cudaFreeAsync(box, st));
   HRT_CUDA(ctx, cudaFreeAsync(scratch, st));
   HRT_CUDA(ctx, cudaStreamSynchronize(st));
+  inputs.idle = true;
   cudaEventElapsedTime(&g.buildMs, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
