@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "hrt_internal.cuh"
+#include "input_range.h"
 
 using namespace hrt;
 using namespace hrt::api;
@@ -136,6 +137,9 @@ bool is_identity(const float* m)
   return true;
 }
 
+// Bytes that a build reads of its vertices: xyz of the last, not its padding.
+static uint64_t vertex_bytes(uint64_t n, uint64_t stride) { return n ? stride * (n - 1) + 12 : 0; }
+
 // Kernels read a build's inputs where the caller has them.  A build that fails
 // after its first launch therefore waits for its stream before it returns: the
 // caller may free the arrays at once.
@@ -163,7 +167,8 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   HRT_CUDA(ctx, dalloc(&g.verts, nVert, bytes, st));
   HRT_CUDA(ctx, dalloc(&g.params, 1, bytes, st));
   // inputs are read where they are when the kernels reach them, else copied
-  const uint8_t* src = nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos)) : nullptr;
+  const uint8_t* src =
+      nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos, vertex_bytes(nVert, stride))) : nullptr;
   uint8_t* raw = nullptr;
   if (nVert && !src)
   {
@@ -192,7 +197,7 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
   uint32_t *keysAlt = nullptr, *valsAlt = nullptr, *parent = nullptr, *visit = nullptr;
   void* scratch = nullptr;
   HRT_CUDA(ctx, cudaMallocAsync((void**)&dIdx, sizeof(uint32_t) * nIdx, st));
-  const uint32_t* idxSrc = static_cast<const uint32_t*>(input_in_place(ctx, idx));
+  const uint32_t* idxSrc = static_cast<const uint32_t*>(input_in_place(ctx, idx, sizeof(uint32_t) * nIdx));
   if (!idxSrc)
   {
     HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * nIdx, cudaMemcpyDefault, st));
@@ -377,10 +382,11 @@ int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geo
   {
     const uint64_t nv = vOff[i + 1] - vOff[i], ni = iOff[i + 1] - iOff[i];
     const bool derive = in.joined && i > 0;
-    srcV[i] = derive ? (srcV[0] ? srcV[0] + stride * vOff[i] : 0)
-                     : (uint64_t)(uintptr_t)((nv || in.joined) && V ? input_in_place(ctx, in.vpos[i]) : nullptr);
-    srcI[i] = derive ? (srcI[0] ? srcI[0] + 4 * iOff[i] : 0)
-                     : (uint64_t)(uintptr_t)((ni || in.joined) && N ? input_in_place(ctx, in.idx[i]) : nullptr);
+    auto where = [&](const void* p, uint64_t bytes) { return (uint64_t)(uintptr_t)input_in_place(ctx, p, bytes); };
+    if (derive) srcV[i] = srcV[0] ? srcV[0] + stride * vOff[i] : 0;
+    else srcV[i] = (nv || in.joined) && V ? where(in.vpos[i], vertex_bytes(in.joined ? V : nv, stride)) : 0;
+    if (derive) srcI[i] = srcI[0] ? srcI[0] + 4 * iOff[i] : 0;
+    else srcI[i] = (ni || in.joined) && N ? where(in.idx[i], 4 * (in.joined ? 3 * N : ni)) : 0;
     const bool copyV = !srcV[i] && (derive ? false : (in.joined ? V : nv) > 0);
     const bool copyI = !srcI[i] && (derive ? false : (in.joined ? N : ni) > 0);
     if (copyV)
@@ -696,7 +702,8 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   InputsInUse inputs{st};
   const uint32_t N = g.nTris;
   const uint64_t nVert = g.nVerts;
-  const uint8_t* src = nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos)) : nullptr;
+  const uint8_t* src =
+      nVert ? static_cast<const uint8_t*>(input_in_place(ctx, vpos, vertex_bytes(nVert, stride))) : nullptr;
   uint8_t* raw = nullptr;
   if (nVert && !src)
   {
@@ -718,7 +725,7 @@ int refit_geometry(hrt_scene* s, Geom& g, const float* vpos, const uint32_t* idx
   BuildParams* box = nullptr;
   void* scratch = nullptr;
   HRT_CUDA(ctx, cudaMallocAsync((void**)&dIdx, sizeof(uint32_t) * 3 * (size_t)N, st));
-  const uint32_t* idxSrc = static_cast<const uint32_t*>(input_in_place(ctx, idx));
+  const uint32_t* idxSrc = static_cast<const uint32_t*>(input_in_place(ctx, idx, sizeof(uint32_t) * 3 * (size_t)N));
   if (!idxSrc)
   {
     HRT_CUDA(ctx, cudaMemcpyAsync(dIdx, idx, sizeof(uint32_t) * 3 * (size_t)N, cudaMemcpyDefault, st));
@@ -842,30 +849,42 @@ bool pageable_access()
   return k == 2;
 }
 
-void* mapped_host(const void* p, bool pageable)
+// The runtime's answer for one address; as for managed memory, which is copied,
+// where it has none.
+static cudaPointerAttributes attributes_of(const void* p)
 {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess)
   {
     cudaGetLastError();
-    return nullptr;
+    a = {};
+    a.type = cudaMemoryTypeManaged;
   }
-  if (a.type == cudaMemoryTypeHost) return a.devicePointer;
-  if (pageable && a.type == cudaMemoryTypeUnregistered && pageable_access()) return const_cast<void*>(p);
-  return nullptr;
+  return a;
 }
 
-const void* input_in_place(const hrt_context* ctx, const void* p)
+// Whether the kernels reach all of `bytes` bytes from p, at first.devicePointer.
+// One question suffices for host memory at its own address where the device
+// translates through the host's page tables, page-locked or not.
+static bool reached(const void* p, uint64_t bytes, const cudaPointerAttributes& first)
 {
-  cudaPointerAttributes a;
+  if (bytes == 0 || (first.type == cudaMemoryTypeHost && first.devicePointer == p && pageable_access())) return true;
+  return same_block(first, attributes_of(static_cast<const char*>(p) + (bytes - 1)), bytes);
+}
+
+void* mapped_host(const void* p, uint64_t bytes, bool pageable)
+{
+  const cudaPointerAttributes a = attributes_of(p);
+  if (a.type == cudaMemoryTypeHost) return reached(p, bytes, a) ? a.devicePointer : nullptr;
+  return pageable && a.type == cudaMemoryTypeUnregistered && pageable_access() ? const_cast<void*>(p) : nullptr;
+}
+
+const void* input_in_place(const hrt_context* ctx, const void* p, uint64_t bytes)
+{
   if (!aligned_to(p, 4)) return nullptr;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess)
-  {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (a.type == cudaMemoryTypeDevice) return a.device == ctx->device ? p : nullptr;
-  if (a.type == cudaMemoryTypeHost) return a.devicePointer;
+  const cudaPointerAttributes a = attributes_of(p);
+  if (a.type == cudaMemoryTypeDevice) return a.device == ctx->device && reached(p, bytes, a) ? p : nullptr;
+  if (a.type == cudaMemoryTypeHost) return reached(p, bytes, a) ? a.devicePointer : nullptr;
   return a.type == cudaMemoryTypeUnregistered && pageable_access() ? p : nullptr;
 }
 
@@ -1390,8 +1409,9 @@ static int query_host(hrt_scene* s, int kind, const float* rays, uint64_t n, voi
   // pool writes each hit when its ray ends, scattered 32-byte writes that the
   // link serves poorly).  Other host memory (or arrays that are not 16-byte
   // aligned) goes through the staging buffers.
-  const float* mappedRays = aligned_to(rays, 16) ? static_cast<const float*>(mapped_host(rays, true)) : nullptr;
-  void* mappedOut = kind == 1 || aligned_to(out, 16) ? mapped_host(out) : nullptr;
+  const float* mappedRays = aligned_to(rays, 16) ? static_cast<const float*>(mapped_host(rays, 32 * n, true)) : nullptr;
+  const size_t outBytes = (kind == 0 ? sizeof(hrt_hit) : 1) * n;
+  void* mappedOut = kind == 1 || aligned_to(out, 16) ? mapped_host(out, outBytes) : nullptr;
   const bool inPlace = mappedRays && mappedOut;
   if (inPlace)
   {
@@ -1473,8 +1493,9 @@ static int query_host_async(hrt_scene* s, int kind, const float* rays, uint64_t 
   if (!rays || !out) return fail(s->ctx, HRT_ERR_INVALID_ARGUMENT, "null ray or output pointer");
   hrt_context* ctx = s->ctx;
   cudaSetDevice(ctx->device);
-  const float* mappedRays = aligned_to(rays, 16) ? static_cast<const float*>(mapped_host(rays, true)) : nullptr;
-  void* mappedOut = kind == 1 || aligned_to(out, 16) ? mapped_host(out) : nullptr;
+  const float* mappedRays = aligned_to(rays, 16) ? static_cast<const float*>(mapped_host(rays, 32 * n, true)) : nullptr;
+  const size_t outBytes = (kind == 0 ? sizeof(hrt_hit) : 1) * n;
+  void* mappedOut = kind == 1 || aligned_to(out, 16) ? mapped_host(out, outBytes) : nullptr;
   const size_t outSize = kind == 0 ? sizeof(hrt_hit) : 1;
   float* dRays = nullptr;
   void* dOut = nullptr;

@@ -133,16 +133,18 @@ int query_eye_rays(hrt_scene* s, const float* rays, uint64_t n, int imageWidth, 
 // Column-major 4x4 -> rows 0..2 of its inverse (the reference checker's evaluation).
 void inverse4x4(const float* mc, float* inv12);
 bool is_identity(const float* m);
-// The address at which a kernel reaches host memory in place: the mapped
-// device address of page-locked memory; with `pageable`, pageable memory
-// itself where the device translates through the host's page tables
-// (pageable_access); null otherwise.
-void* mapped_host(const void* p, bool pageable = false);
+// The address at which a kernel reaches `bytes` bytes of host memory in place:
+// the mapped device address of page-locked memory; with `pageable`, pageable
+// memory itself where the device translates through the host's page tables
+// (pageable_access); null otherwise, and where only a part is page-locked and
+// the rest out of reach.
+void* mapped_host(const void* p, uint64_t bytes, bool pageable = false);
 bool pageable_access();
-// The address at which this device's kernels read a build's input in place:
-// device memory of the context's device, or host memory as mapped_host with
-// pageable; null where it has to be copied first.
-const void* input_in_place(const hrt_context* ctx, const void* p);
+// The address at which this device's kernels read `bytes` bytes of a build's
+// input in place: device memory of the context's device, or host memory as
+// mapped_host with pageable; null where it has to be copied first (which
+// refuses a range that goes past its allocation).
+const void* input_in_place(const hrt_context* ctx, const void* p, uint64_t bytes);
 // True when p is a multiple of `bytes` (a power of two).  Kernels read rays
 // and write hits as 16-byte vectors, so arrays they access in place must be
 // 16-byte aligned; the entry points check this before any launch.

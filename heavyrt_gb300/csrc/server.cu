@@ -180,11 +180,13 @@ cudaError_t issue(hrt_server* S, Slot* sl)
   const Request* only = sl->reqs.size() == 1 ? sl->reqs[0] : nullptr;
   // page-locked rays, read in place over the host link (no copy in)
   auto rays_in_place = [](const Request* r) {
-    return aligned_to(r->rays, 16) ? static_cast<const float4*>(mapped_host(r->rays)) : nullptr;
+    return aligned_to(r->rays, 16) ? static_cast<const float4*>(mapped_host(r->rays, 32 * r->n)) : nullptr;
   };
   // a batch of one request: results written in place, when page-locked
   void* inPlaceOut =
-      only && (only->kind == 1 || aligned_to(only->out, 16)) ? mapped_host(only->out) : nullptr;
+      only && (only->kind == 1 || aligned_to(only->out, 16))
+          ? mapped_host(only->out, (only->kind == 0 ? sizeof(hrt_hit) : 1) * only->n)
+          : nullptr;
   if (only && sl->one.valid)
   {
     // One request against one scene of one untransformed geometry: the

@@ -29,7 +29,7 @@ CUDA_SOURCES = ["radix_sort.cu", "build.cu", "build_batch.cu", "bvh4.cu", "trace
                 "trace_l2.cu", "trace_l3.cu", "trace_w0.cu", "trace_w1.cu", "trace_w2.cu", "trace_w3.cu", "hrt_api.cu",
                 "server.cu", "raygen.cu", "render.cu", "formats.cu"]
 CUDA_HEADERS = ["hrt_common.cuh", "build_common.cuh", "hrt_kernels.cuh", "hrt_internal.cuh", "trace_impl.cuh",
-                "raygen_common.cuh", "leaf_tree.cuh"]
+                "raygen_common.cuh", "leaf_tree.cuh", "input_range.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off", "--expt-relaxed-constexpr"]
 HOST_CFLAGS = ["-O3", "-fPIC", "-ffp-contract=off", "-Wall"]
