@@ -1690,11 +1690,14 @@ cudaError_t launch(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStr
   return cudaGetLastError();
 }
 
+// An instance tree's stack is all in local memory unless the caller set a shape,
+// and all in shared memory when that shape asks for the whole of it: the split
+// variant's, whose shared part is then the whole.
 template <int LAYOUT, int TRI, bool ANY, int THREADS, bool TLAS>
 cudaError_t launch_any_stack(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStream_t s)
 {
   constexpr int DEPTH = StackDepth<LAYOUT, TLAS>::value;
-  return shared_entries<DEPTH>(c.stackEntries) < DEPTH
+  return shared_entries<DEPTH>(c.stackEntries) < DEPTH || (TLAS && c.given)
              ? launch<LAYOUT, TRI, ANY, false, THREADS, TLAS, kStackSplit>(a, c, numSMs, s)
              : launch<LAYOUT, TRI, ANY, false, THREADS, TLAS, TLAS ? kStackLocal : kStackShared>(a, c, numSMs, s);
 }
