@@ -250,7 +250,7 @@ struct TraceConfig
   int imageWidth = 0;         // > 0: rays form row-major images this wide, traced in 4 x 8 tiles
   int raysPerWarp = 32;       // one thread per ray: rays of a warp (its first lanes); set per launch
   int alone = 0;              // instance tree: 1 = lanes walk without the warp's vote; set per launch
-  bool given = false;         // the caller set this shape; else a launch may choose its refill threshold
+  bool given = false;         // the caller set this shape; else a launch may choose another (trace.cu)
 };
 
 // kind 0: nearest, 1: any.  counting = 1 also accumulates counters (node

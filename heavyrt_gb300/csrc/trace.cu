@@ -27,7 +27,9 @@ constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32, kTreeSteps = 4;
 // warps of 32 rays an SM) from which nearest hits go by vote.
 constexpr int kTreeResidentWarps = 24, kGeneralResidentWarps = 18, kVoteWarps = 128;
 
-// The shape of one launch.
+// The shape of one launch.  A shape that the caller set is kept; only how many
+// rays a warp of a one-thread-per-ray launch holds, which no shape says, follows
+// the batch.
 //
 // A batch that does not fill the GPU's warps is bound by the slowest warp's
 // chain of dependent instructions, and a warp of 32 rays that part ways runs
@@ -77,12 +79,12 @@ TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int kind, int
   const int resident = !tree && (a.one || a.rayOffsets) ? kResidentWarps
                        : tree || layout == 0            ? kTreeResidentWarps
                                                         : kGeneralResidentWarps;
-  if (a.n <= (uint64_t)numSMs * resident * 32)
+  if (!c.given && a.n <= (uint64_t)numSMs * resident * 32)
   {
-    s.raysPerWarp = perWarp;
     s.persistent = 0;
     s.threadsPerBlock = 64;
   }
+  if (!s.persistent) s.raysPerWarp = perWarp;
   return s;
 }
 

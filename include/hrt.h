@@ -282,10 +282,11 @@ int hrt_scene_check(hrt_scene* scene);
  * one ray per virtual call with an 80-entry stack, core/raytrace_common.h:34).
  * Defaults: 128 threads, persistent pool, 16 steps between refills, refill at
  * 24 idle lanes, the whole stack in shared memory.  Until a shape is set for a
- * kind the engine may pick a better one per launch (looks every 8 steps for 8 idle lanes;
- * eye rays of hrt_frame_* one thread per ray; an instance tree's stack in
- * local memory).  Batches whose rays all fit on the GPU at once are traced one
- * thread per ray whatever the shape, small ones with fewer rays a warp.
+ * kind the engine may pick a better one per launch (looks every 8 steps for 8
+ * idle lanes; batches whose rays all fit on the GPU at once, and eye rays of
+ * hrt_frame_*, one thread per ray; an instance tree's stack in local memory).  A
+ * shape that is set is launched as it is.  Either way a small batch that goes one
+ * thread per ray has fewer rays a warp.
  * imageWidth is a property of the rays the kind's queries pass (the
  * autotuner keeps it).
  * stackEntries: traversal stack entries per ray kept in shared memory; deeper
