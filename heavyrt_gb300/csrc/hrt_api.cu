@@ -318,19 +318,33 @@ int build_geometry(hrt_scene* s, Geom& g, const float* vpos, uint64_t nVert, con
 
 // Device allocation owned by a batch: recorded in `owned` (freed together,
 // free_batch), from the device's stream-ordered pool like a geometry's.
-template <typename T> cudaError_t balloc(T** p, size_t count, std::vector<void*>& owned, cudaStream_t st)
+template <typename T> cudaError_t balloc(T** p, size_t count, BatchMemory& owned, cudaStream_t st)
 {
-  const cudaError_t e = cudaMallocAsync((void**)p, sizeof(T) * (count ? count : 1), st);
-  if (e == cudaSuccess) owned.push_back(*p);
+  const size_t bytes = sizeof(T) * (count ? count : 1);
+  const cudaError_t e = cudaMallocAsync((void**)p, bytes, st);
+  if (e != cudaSuccess) return e;
+  owned.blocks.push_back(*p);
+  owned.bytes += bytes;
   return e;
 }
 
-// Frees batch allocations, after the queries that may still read them.
-void free_batch(std::vector<void*>& owned)
+// Frees batch allocations, after the queries that may still read them, to the
+// pool: a scene that is cleared and loaded again finds them there.
+void free_batch(BatchMemory& owned)
 {
-  if (!owned.empty()) cudaDeviceSynchronize();
-  for (void* p : owned) cudaFree(p);
-  owned.clear();
+  if (!owned.blocks.empty()) cudaDeviceSynchronize();
+  for (void* p : owned.blocks) cudaFree(p);
+  owned = BatchMemory();
+}
+
+// Returns up to `bytes` of what the pool holds unused to the driver.
+void shrink_pool(int device, uint64_t bytes)
+{
+  cudaMemPool_t pool;
+  uint64_t reserved = 0;
+  if (bytes && cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, reserved > bytes ? reserved - bytes : 0);
 }
 
 inline size_t align_up(size_t b, size_t a) { return (b + a - 1) / a * a; }
@@ -351,7 +365,7 @@ struct BatchInputs
 // Builds G geometries with one segmented LBVH build (build_batch.cu) and, for
 // a 4-wide layout, collapses each.  On success appends G geometries whose
 // arrays point into allocations recorded in `owned`.
-int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geom>& out, std::vector<void*>& owned)
+int build_batch(hrt_scene* s, uint32_t G, const BatchInputs& in, std::vector<Geom>& out, BatchMemory& owned)
 {
   hrt_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
@@ -1083,7 +1097,7 @@ int hrt_clear_geom(hrt_scene* s)
   cudaStreamSynchronize(s->ctx->stream);
   for (Geom& gm : s->geoms) free_geom(gm);
   free_geom(s->tlas);
-  free_batch(s->batchAllocs);
+  free_batch(s->batch);
   s->geoms.clear();
   s->insts.clear();
   s->committed = false;
@@ -1102,6 +1116,7 @@ int hrt_scene_destroy(hrt_scene* s)
   if (s->stageOut) cudaFree(s->stageOut);
   for (cudaStream_t p : s->pipe)
     if (p) cudaStreamDestroy(p);
+  shrink_pool(s->ctx->device, s->batchMost);
   delete s;
   return HRT_OK;
 }
@@ -1168,7 +1183,7 @@ static int add_batch(hrt_scene* s, uint32_t count, BatchInputs in, uint32_t* fir
   std::lock_guard<std::mutex> lk(s->mu);
   cudaSetDevice(ctx->device);
   std::vector<Geom> built;
-  std::vector<void*> owned;
+  BatchMemory owned;
   const int st = build_batch(s, count, in, built, owned);
   if (st != HRT_OK)
   {
@@ -1178,7 +1193,9 @@ static int add_batch(hrt_scene* s, uint32_t count, BatchInputs in, uint32_t* fir
   }
   const uint32_t first = (uint32_t)s->geoms.size();
   for (Geom& g : built) s->geoms.push_back(g);
-  for (void* p : owned) s->batchAllocs.push_back(p);
+  s->batch.blocks.insert(s->batch.blocks.end(), owned.blocks.begin(), owned.blocks.end());
+  s->batch.bytes += owned.bytes;
+  s->batchMost = std::max(s->batchMost, s->batch.bytes);
   s->committed = false;
   if (firstGeomId) *firstGeomId = first;
   return HRT_OK;

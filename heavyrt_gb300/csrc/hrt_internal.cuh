@@ -63,6 +63,13 @@ struct Instance
   bool     identity = true;
 };
 
+// Device memory of a scene's batch builds.
+struct BatchMemory
+{
+  std::vector<void*> blocks;
+  uint64_t           bytes = 0;
+};
+
 }  // namespace api
 }  // namespace hrt
 
@@ -75,7 +82,8 @@ struct hrt_scene
   hrt_context*          ctx = nullptr;
   std::vector<Geom>     geoms;
   std::vector<Instance> insts;
-  std::vector<void*>    batchAllocs;  // device allocations shared by batch-built geometries
+  hrt::api::BatchMemory batch;          // shared by the batch-built geometries
+  uint64_t              batchMost = 0;  // most that it held at a time: given back with the scene
   bool                  committed = false;
   int                   layout = HRT_LAYOUT_BVH2;
   int                   bvh4Merge = 0;  // HRT_OPTION_BVH4_MERGE

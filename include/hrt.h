@@ -74,7 +74,12 @@ typedef struct hrt_hit
 /* ---------------------------------------------------------------- context */
 
 /* Opens the engine on CUDA device `device`.  No reference counterpart: the
- * reference runs on the host only. */
+ * reference runs on the host only.
+ * Device memory of geometries, batches and builds comes from the device's
+ * default stream-ordered pool (cudaMallocAsync).  The engine raises the pool's
+ * release threshold to 2 GiB: up to that much freed memory stays in the pool for
+ * later builds, out of reach of other allocators, until
+ * cudaMemPoolTrimTo(cudaDeviceGetDefaultMemPool(...), ...) or the process ends. */
 int hrt_context_create(int device, hrt_context** out);
 int hrt_context_destroy(hrt_context* ctx);
 /* Text of the most recent failure on this context ("" if none). */
@@ -193,7 +198,8 @@ int hrt_scene_get_layout(const hrt_scene* scene, int* layout);
 #define HRT_BVH4_COLLAPSE_LARGEST_FIRST   1
 int hrt_scene_set_option(hrt_scene* scene, int option, int value);
 
-/* ISceneObject::ClearGeom (core/CrossRT.h:82): drops every geometry and instance. */
+/* ISceneObject::ClearGeom (core/CrossRT.h:82): drops every geometry and instance.
+ * Their device memory goes back to the pool (hrt_context_create). */
 int hrt_clear_geom(hrt_scene* scene);
 
 /* ISceneObject::AddGeom_Triangles3f (core/CrossRT.h:94; reference implementation
@@ -328,7 +334,8 @@ int hrt_query_counters(hrt_scene* scene, int kind, const float* rays, uint64_t n
  * idxOffsets[i+1]-1 of idx (a multiple of 3 each), its indices counting from
  * its own first vertex.  Both offset arrays have count+1 entries starting at
  * 0.  The geometries get ids *firstGeomId .. *firstGeomId+count-1; their
- * device memory is shared and freed by hrt_clear_geom / hrt_scene_destroy.
+ * device memory is shared; hrt_clear_geom gives it back to the pool
+ * (hrt_context_create), hrt_scene_destroy to the driver.
  * Limits: each geometry HRT_MAX_TRIS_PER_GEOM, the batch
  * HRT_MAX_TRIS_PER_BATCH triangles and 2^32-1 vertices. */
 #define HRT_MAX_TRIS_PER_BATCH ((1u << 30) - 1u)
