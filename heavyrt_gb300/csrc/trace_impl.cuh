@@ -661,7 +661,6 @@ template <int LAYOUT> struct Lane
   float4   po, di;    // the ray as given (world space)
   uint32_t ray;       // ray index or kNoRay
   uint32_t inst;      // current instance
-  uint32_t instEnd;   // one past the last instance this ray is traced against
   const void*   nodes;  // the current instance's records (binary) or 4-wide nodes
   const TriRec* tris;   // the current instance's triangle records
   uint32_t cur;       // current record / leaf reference
@@ -707,12 +706,12 @@ __device__ __forceinline__ void enter_instance(Lane<LAYOUT>& L, const InstanceDe
 }
 
 // Advances the lane's instance cursor to the next instance with triangles,
-// starting at `from` and ending before L.instEnd; prepares the ray for it.
-// Returns false when none is left.
+// starting at `from`; prepares the ray for it.  Returns false when none is left.
 template <int LAYOUT>
-__device__ __forceinline__ bool begin_instance(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, uint32_t from)
+__device__ __forceinline__ bool begin_instance(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, uint32_t nInst,
+                                               uint32_t from)
 {
-  for (uint32_t k = from; k < L.instEnd; k++)
+  for (uint32_t k = from; k < nInst; k++)
     if (inst[k].valid)
     {
       enter_instance<LAYOUT>(L, inst, k);
@@ -944,7 +943,7 @@ template <int LAYOUT, int TRI, bool ANY, bool GRID> struct NodeRun
 // Stride of the pools' step loops.  It changes nothing but the registers that
 // the compiler finds (500,000 random rays, binary, watertight: 784 us at 1,
 // 694 at the run's length; FP16 nodes, Moller-Trumbore: 501 at 1, 523).
-template <int LAYOUT, bool ANY> struct PoolStep
+template <int LAYOUT> struct PoolStep
 {
   static constexpr int value = LAYOUT == 0 ? 6 : 1;
 };
@@ -952,12 +951,12 @@ template <int LAYOUT, bool ANY> struct PoolStep
 // One advance of a lane that walks its instances in order: nodes, then a leaf
 // when it holds one.  Returns true when the lane's ray is finished.
 template <bool GRID, int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, int STACK>
-__device__ __forceinline__ bool step(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, Stack<THREADS, STACK>& st,
-                                     uint64_t& nPairs, uint64_t& nTris, uint32_t* errorWord)
+__device__ __forceinline__ bool step(Lane<LAYOUT>& L, const InstanceDesc* __restrict__ inst, uint32_t nInst,
+                                     Stack<THREADS, STACK>& st, uint64_t& nPairs, uint64_t& nTris, uint32_t* errorWord)
 {
   constexpr int DEPTH = StackDepth<LAYOUT, false>::value;
   auto leave = [&]() {
-    if (L.top == 0) return !begin_instance<LAYOUT>(L, inst, L.inst + 1);
+    if (L.top == 0) return !begin_instance<LAYOUT>(L, inst, nInst, L.inst + 1);
     L.top--;
     L.cur = st.get(L.top);
     return false;
@@ -1198,13 +1197,12 @@ __device__ __forceinline__ void write_result(const Lane<LAYOUT>& L, const Instan
   }
 }
 
-// Instances a ray is traced against: all of them, or - for a segmented query -
-// the one instance of the ray's segment (rayOffsets[0..nSeg] ascending, ray i
-// in segment k when rayOffsets[k] <= i < rayOffsets[k+1]); an instance id out
-// of range leaves the ray a miss.
+// A segmented query: ray i is traced against the one instance of its segment
+// (rayOffsets[0..nSeg] ascending, ray i in segment k when rayOffsets[k] <= i <
+// rayOffsets[k+1]); an instance id out of range leaves the ray a miss.
 struct Segments
 {
-  const uint32_t* rayOffsets;  // nullptr: no segments
+  const uint32_t* rayOffsets;
   const uint32_t* segInst;
   uint32_t        nSeg;
   uint32_t        nInst;
@@ -1221,14 +1219,6 @@ __device__ __forceinline__ uint32_t segment_of(uint32_t i, const Segments& sg)
     else hi = mid;
   }
   return lo;
-}
-
-template <int LAYOUT>
-__device__ __forceinline__ uint32_t first_instance(Lane<LAYOUT>& L, uint32_t i, const Segments& sg)
-{
-  const uint32_t k = sg.rayOffsets == nullptr ? 0u : __ldg(sg.segInst + segment_of(i, sg));
-  L.instEnd = sg.rayOffsets == nullptr ? sg.nInst : (k < sg.nInst ? k + 1 : 0);
-  return k;
 }
 
 template <int LAYOUT>
@@ -1263,21 +1253,21 @@ __device__ __forceinline__ void flush_counters(uint64_t nPairs, uint64_t nTris, 
 // `refill` lanes are idle (or all are).  The two-level kernels are held to six
 // blocks of 128 threads an SM (80 registers; 921,600 rays, 240 instances: 1,136
 // us unbounded, 1,113 at 6, 1,185 at 7, 1,275 at 8 blocks).
-template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, bool TLAS, int STACK>
+template <int LAYOUT, int TRI, bool ANY, int THREADS, bool TLAS, int STACK>
 __global__ void __launch_bounds__(THREADS, TLAS ? 768 / THREADS : 0) k_trace_pool(const float4* __restrict__ rays, uint32_t n,
-                                                        const InstanceDesc* __restrict__ inst, Segments sg, Tlas tl,
-                                                        void* out, unsigned long long* counters, uint32_t* errorWord,
-                                                        unsigned int* rayCounter, int steps, int refill, int alone,
-                                                        int stackShared, RayOrder order)
+                                                        const InstanceDesc* __restrict__ inst, uint32_t nInst, Tlas tl,
+                                                        void* out, uint32_t* errorWord, unsigned int* rayCounter,
+                                                        int steps, int refill, int alone, int stackShared,
+                                                        RayOrder order)
 {
   extern __shared__ uint32_t s_stack[];  // stackShared * THREADS entries
   uint32_t local[STACK != kStackShared ? StackDepth<LAYOUT, TLAS>::value : 1];
   Stack<THREADS, STACK> st{s_stack + threadIdx.x, local, stackShared};
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t ltMask = (1u << lane) - 1u;
-  uint64_t nPairs = 0, nTris = 0;
+  uint64_t none = 0;
   Lane<LAYOUT> L;
-  constexpr int kStep = PoolStep<LAYOUT, ANY>::value;
+  constexpr int kStep = PoolStep<LAYOUT>::value;
   L.ray = kNoRay;
   L.cur = kDone;
   bool exhausted = false;
@@ -1304,21 +1294,21 @@ __global__ void __launch_bounds__(THREADS, TLAS ? 768 / THREADS : 0) k_trace_poo
           start_ray(L, i, rays);
           bool live = true;
           if (TLAS) tlas_begin(L);
-          else live = begin_instance<LAYOUT>(L, inst, first_instance(L, i, sg));
+          else live = begin_instance<LAYOUT>(L, inst, nInst, 0);
           if (!live) L.cur = kDone;
         }
       }
     }
     if (TLAS && alone)
-      run_alone<kAloneNodeRun, kAloneTreeRun, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, steps);
+      run_alone<kAloneNodeRun, kAloneTreeRun, LAYOUT, TRI, ANY, false, THREADS, STACK>(L, inst, tl, st, none, none, errorWord, steps);
     else if (TLAS)
-      run_phases<LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, steps);
+      run_phases<LAYOUT, TRI, ANY, false, THREADS, STACK>(L, inst, tl, st, none, none, errorWord, steps);
     else if (L.cur != kDone)
     {
       for (int s = 0; s < steps * kStep; s += kStep)
       {
         if (out_of_budget(L, errorWord) ||
-            step<false, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord))
+            step<false, LAYOUT, TRI, ANY, false, THREADS, STACK>(L, inst, nInst, st, none, none, errorWord))
         {
           L.cur = kDone;
           break;
@@ -1326,13 +1316,12 @@ __global__ void __launch_bounds__(THREADS, TLAS ? 768 / THREADS : 0) k_trace_poo
       }
     }
   }
-  flush_counters<COUNT>(nPairs, nTris, counters);
 }
 
 // One thread per ray.
 template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, bool TLAS, int STACK>
 __global__ void __launch_bounds__(THREADS) k_trace_grid(const float4* __restrict__ rays, uint32_t n,
-                                                        const InstanceDesc* __restrict__ inst, Segments sg, Tlas tl,
+                                                        const InstanceDesc* __restrict__ inst, uint32_t nInst, Tlas tl,
                                                         void* out, unsigned long long* counters, uint32_t* errorWord,
                                                         int stackShared, RayOrder order)
 {
@@ -1348,9 +1337,9 @@ __global__ void __launch_bounds__(THREADS) k_trace_grid(const float4* __restrict
   {
     start_ray(L, i, rays);
     if (TLAS) tlas_begin(L);
-    else if (begin_instance<LAYOUT>(L, inst, first_instance(L, i, sg)))
+    else if (begin_instance<LAYOUT>(L, inst, nInst, 0))
       while (!out_of_budget(L, errorWord) &&
-             !step<true, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, st, nPairs, nTris, errorWord)) {}
+             !step<true, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, nInst, st, nPairs, nTris, errorWord)) {}
   }
   if (TLAS) run_alone<kGridNodeRun, kGridTreeRun, LAYOUT, TRI, ANY, COUNT, THREADS, STACK>(L, inst, tl, st, nPairs, nTris, errorWord, 0x7FFFFFFF);
   if (i != kNoRay) write_result<ANY>(L, inst, out);
@@ -1490,7 +1479,7 @@ __global__ void __launch_bounds__(THREADS) k_trace_one(const float4* __restrict_
   L.cur = kDone;
   L.nodes = src.nodes;
   L.tris = src.tris;
-  constexpr int kStep = PoolStep<LAYOUT, ANY>::value;
+  constexpr int kStep = PoolStep<LAYOUT>::value;
   bool exhausted = false;
   while (true)
   {
@@ -1654,39 +1643,39 @@ template <int LAYOUT, int TRI, bool ANY, bool COUNT, int THREADS, bool TLAS, int
 cudaError_t launch(const TraceArgs& a, const TraceConfig& c, int numSMs, cudaStream_t s)
 {
   const uint32_t n = (uint32_t)a.n;
-  const Segments sg{a.rayOffsets, a.segInst, a.nSeg, a.nInst, nullptr};
   const Tlas tl{a.tlasRecs, a.tlasTris, a.nInst};
   const int shared = STACK == kStackLocal ? 0
                      : STACK == kStackSplit ? shared_entries<StackDepth<LAYOUT, TLAS>::value>(c.stackEntries)
                                             : StackDepth<LAYOUT, TLAS>::value;
   const size_t smem = sizeof(uint32_t) * (size_t)shared * THREADS;
   const RayOrder order = ray_order(n, c.imageWidth, c.raysPerWarp);
-  if (c.persistent && !COUNT)
+  if constexpr (!COUNT)
   {
-    cudaError_t e = allow_smem(k_trace_pool<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK>, smem);
-    if (e != cudaSuccess) return e;
-    int perSM = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &perSM, k_trace_pool<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK>, THREADS, smem);
-    if (e != cudaSuccess) return e;
-    if (perSM < 1) perSM = 1;
-    uint64_t blocks = (uint64_t)numSMs * perSM;
-    const uint64_t need = ((uint64_t)order.nWork + THREADS - 1) / THREADS;
-    if (blocks > need) blocks = need;
-    e = cudaMemsetAsync(a.rayCounter, 0, sizeof(unsigned int), s);
-    if (e != cudaSuccess) return e;
-    k_trace_pool<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK><<<(uint32_t)blocks, THREADS, smem, s>>>(
-        a.rays, n, a.inst, sg, tl, a.hits, a.counters, a.errorWord, a.rayCounter, c.stepsPerRefill, c.refillLanes,
-        c.alone, shared, order);
+    if (c.persistent)
+    {
+      cudaError_t e = allow_smem(k_trace_pool<LAYOUT, TRI, ANY, THREADS, TLAS, STACK>, smem);
+      if (e != cudaSuccess) return e;
+      int perSM = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_trace_pool<LAYOUT, TRI, ANY, THREADS, TLAS, STACK>,
+                                                        THREADS, smem);
+      if (e != cudaSuccess) return e;
+      if (perSM < 1) perSM = 1;
+      uint64_t blocks = (uint64_t)numSMs * perSM;
+      const uint64_t need = ((uint64_t)order.nWork + THREADS - 1) / THREADS;
+      if (blocks > need) blocks = need;
+      e = cudaMemsetAsync(a.rayCounter, 0, sizeof(unsigned int), s);
+      if (e != cudaSuccess) return e;
+      k_trace_pool<LAYOUT, TRI, ANY, THREADS, TLAS, STACK><<<(uint32_t)blocks, THREADS, smem, s>>>(
+          a.rays, n, a.inst, a.nInst, tl, a.hits, a.errorWord, a.rayCounter, c.stepsPerRefill, c.refillLanes, c.alone,
+          shared, order);
+      return cudaGetLastError();
+    }
   }
-  else
-  {
-    cudaError_t e = allow_smem(k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK>, smem);
-    if (e != cudaSuccess) return e;
-    const uint32_t blocks = grid_blocks<THREADS>(order);
-    k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK><<<blocks, THREADS, smem, s>>>(
-        a.rays, n, a.inst, sg, tl, a.hits, a.counters, a.errorWord, shared, order);
-  }
+  cudaError_t e = allow_smem(k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK>, smem);
+  if (e != cudaSuccess) return e;
+  const uint32_t blocks = grid_blocks<THREADS>(order);
+  k_trace_grid<LAYOUT, TRI, ANY, COUNT, THREADS, TLAS, STACK><<<blocks, THREADS, smem, s>>>(
+      a.rays, n, a.inst, a.nInst, tl, a.hits, a.counters, a.errorWord, shared, order);
   return cudaGetLastError();
 }
 
@@ -1723,17 +1712,18 @@ cudaError_t trace_tlas(const TraceArgs& a, int kind, int counting, const TraceCo
   }
 }
 
-// Counting runs use the one-thread-per-ray grid at 128 threads: the counts do
-// not depend on the schedule.  A scene with an instance tree uses the
-// two-level kernels, except in segmented queries (one instance per ray).  A
-// scene of one untransformed instance uses the single-instance kernels.
+// Counting runs use the one-thread-per-ray grid at 128 threads (the counts do
+// not depend on the schedule) and have no segments.  Segmented queries and a
+// scene of one untransformed instance use the one-instance kernels, a scene with
+// an instance tree the two-level ones.
 template <int LAYOUT, int TRI>
 cudaError_t trace_layout(const TraceArgs& a, int kind, int counting, const TraceConfig& c, int numSMs, cudaStream_t s)
 {
-  if (a.rayOffsets != nullptr && !counting) return trace_one<LAYOUT, TRI, true>(a, kind, c, numSMs, s);
-  if (a.one != nullptr && !counting && a.rayOffsets == nullptr && a.tlasRecs == nullptr)
+  if (a.rayOffsets != nullptr)
+    return counting ? cudaErrorInvalidValue : trace_one<LAYOUT, TRI, true>(a, kind, c, numSMs, s);
+  if (a.one != nullptr && !counting && a.tlasRecs == nullptr)
     return trace_one<LAYOUT, TRI, false>(a, kind, c, numSMs, s);
-  if (a.tlasRecs != nullptr && a.rayOffsets == nullptr)
+  if (a.tlasRecs != nullptr)
     return trace_tlas<LAYOUT, TRI, true>(a, kind, counting, c, numSMs, s);
   return trace_tlas<LAYOUT, TRI, false>(a, kind, counting, c, numSMs, s);
 }
