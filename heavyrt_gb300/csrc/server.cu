@@ -563,15 +563,12 @@ int hrt_server_create(hrt_context* ctx, const hrt_server_config* config, hrt_ser
   S->proto.bvh4Merge = c.bvh4Merge;
   S->proto.mortonFrame = c.mortonFrame;
   S->proto.bvh4Collapse = c.bvh4Collapse;
-  for (int k = 0; k < 2; k++)
-  {
-    S->trace[k].threadsPerBlock = 256;  // segmented batches: fastest shape of the batched-scene sweep
-    S->trace[k].persistent = 1;
-    S->trace[k].stepsPerRefill = 16;
-    S->trace[k].refillLanes = 8;
-  }
+  // segmented batches in the pool: 256 threads were fastest in the batched-scene
+  // sweep; the rest, and small batches, are the launch's choice (trace.cu)
+  for (int k = 0; k < 2; k++) S->trace[k].threadsPerBlock = 256;
   // single requests: the single-instance kernels' shapes of the RTAO frame's
-  // sweep (nearest hits written in place switch to one thread per ray)
+  // sweep (nearest hits written in place switch to one thread per ray), for
+  // batches that the GPU does not hold at once
   S->traceOne[0].threadsPerBlock = 64;
   S->traceOne[0].persistent = 0;
   S->traceOne[1].threadsPerBlock = 128;
