@@ -1891,6 +1891,7 @@ int hrt_scene_autotune(hrt_scene* s, const hrt_query_desc* q, int repeats, hrt_t
     c.threadsPerBlock = tpb;
     c.persistent = 0;
     grid.push_back(c);
+    if (trace_spreads(q->n, ctx->numSMs)) continue;  // pools go one thread per ray too
     for (int steps : {4, 8, 16, 32, 64})
       for (int lanes : {2, 4, 8, 16, 24, 28, 32})
       {

@@ -258,5 +258,8 @@ struct TraceConfig
 // 2 4-wide FP16, 3 4-wide 8-bit.
 cudaError_t trace(const TraceArgs& a, int kind, int counting, int layout, const TraceConfig& c, int numSMs,
                   cudaStream_t stream);
+// Whether a batch of n rays is so small that it is spread over warps, one thread
+// per ray, whatever shape is set (no pool refills in it).
+bool trace_spreads(uint64_t n, int numSMs);
 
 }  // namespace hrt

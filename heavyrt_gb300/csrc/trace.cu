@@ -27,9 +27,11 @@ constexpr int kRefillLanes = 8, kAdvances = 8, kTreePhases = 32, kTreeSteps = 4;
 // warps of 32 rays an SM) from which nearest hits go by vote.
 constexpr int kTreeResidentWarps = 24, kGeneralResidentWarps = 18, kVoteWarps = 128;
 
-// The shape of one launch.  A shape that the caller set is kept; only how many
-// rays a warp of a one-thread-per-ray launch holds, which no shape says, follows
-// the batch.
+// The shape of one launch.  A shape that the caller set is kept, but for a pool
+// in a batch so small that it is spread over warps (below): a pool of any block
+// and stack size holds such a batch at once and would refill nothing, so it goes
+// one thread per ray, with the block and the stack that were set (1,000 rays, a
+// pool of 128 threads 82 us, so 49; FP16 nodes, any hits).
 //
 // A batch that does not fill the GPU's warps is bound by the slowest warp's
 // chain of dependent instructions, and a warp of 32 rays that part ways runs
@@ -84,11 +86,14 @@ TraceConfig launch_shape(const TraceArgs& a, const TraceConfig& c, int kind, int
     s.persistent = 0;
     s.threadsPerBlock = 64;
   }
+  if (trace_spreads(a.n, numSMs)) s.persistent = 0;
   if (!s.persistent) s.raysPerWarp = perWarp;
   return s;
 }
 
 }  // namespace
+
+bool trace_spreads(uint64_t n, int numSMs) { return n <= (uint64_t)numSMs * kSpreadWarps * 16; }
 
 cudaError_t trace(const TraceArgs& a, int kind, int counting, int layout, const TraceConfig& config, int numSMs,
                   cudaStream_t s)

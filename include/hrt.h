@@ -291,8 +291,9 @@ int hrt_scene_check(hrt_scene* scene);
  * kind the engine may pick a better one per launch (looks every 8 steps for 8
  * idle lanes; batches whose rays all fit on the GPU at once, and eye rays of
  * hrt_frame_*, one thread per ray; an instance tree's stack in local memory).  A
- * shape that is set is launched as it is.  Either way a small batch that goes one
- * thread per ray has fewer rays a warp.
+ * shape that is set is launched as it is, but for batches of at most 208 rays an
+ * SM, in which a pool would refill nothing: they go one thread per ray, with few
+ * rays a warp, in the block size and with the stack that were set.
  * imageWidth is a property of the rays the kind's queries pass (the
  * autotuner keeps it).
  * stackEntries: traversal stack entries per ray kept in shared memory; deeper
@@ -383,8 +384,9 @@ int hrt_graph_destroy(hrt_graph* graph);
 /* Launch-shape autotuner: times `query` (repeats timed runs after one
  * warm-up) under every trace configuration of a fixed grid (64/128/256
  * threads; one ray per thread, or the persistent pool with 4..64 steps per
- * refill and 2..32 idle lanes to refill), then the best of those with 16, 24,
- * 32, 48 and 64 shared-memory stack entries; sets the fastest as the scene's
+ * refill and 2..32 idle lanes to refill, where the batch is not so small that
+ * a pool would refill nothing), then the best of those with 16, 24, 32, 48 and
+ * 64 shared-memory stack entries; sets the fastest as the scene's
  * configuration for query->kind, and returns it with its mean time in ms.
  * Synchronous; overwrites query->out (with identical results). */
 int hrt_scene_autotune(hrt_scene* scene, const hrt_query_desc* query, int repeats, hrt_trace_config* best,
