@@ -1667,10 +1667,23 @@ def run_engine(args):
             cfg["oracle_anyhit_mismatch"] = int(np.count_nonzero(d_any.cpu().numpy().astype(bool) != want_any))
             cfg["oracle_e2e_anyhit_mismatch"] = int(np.count_nonzero(got_any.astype(bool) != want_any))
     summarize(line)
+    details = detach_details(line)
     if rank == 0:
+        print(json.dumps({"details": details}), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     replicas.finish(rk)
     return 0
+
+
+# Sections whose key figures are in the line's config; whole on stderr.
+DETAIL_SECTIONS = ("e2e_device_raygen", "reference_tree", "even_depth_collapse", "plain", "l2_window", "watertight",
+                   "frames", "served", "served_3x", "batched", "precision")
+
+
+def detach_details(line: dict) -> dict:
+    """Takes the long sections out of the line: whole it is 20 KB, which a
+    reader that keeps the end of the output loses the start of."""
+    return {k: line.pop(k) for k in DETAIL_SECTIONS if k in line}
 
 
 def summarize(line: dict):
