@@ -29,12 +29,16 @@
 // array in local memory (S is a launch parameter, full depth by default; the
 // two-level kernels keep the whole stack in local memory by default).
 //
-// What bounds it: instruction issue (73% of cycles with the pools full) at 12
-// to 17 of 32 threads per instruction, since a warp's rays part ways; DRAM is
-// at 3 to 5%.  So the slab test runs on packed pairs of floats, picks entry
-// planes by the direction's sign, and takes its min and max three at a time;
-// lanes visit runs of nodes between leaves; results are written when a warp
-// refills.  Against four 128-bit loads, scalar slabs and one node or leaf per
+// What bounds it (profiles/trace_kernels_cases.txt): in 8-bit and FP16 nodes
+// instruction issue, 58 to 75% of cycles, at 11 to 17 of 32 threads per
+// instruction, since a warp's rays part ways; in binary and FP32 nodes, where 41
+// to 45% of cycles issue, the latency of nodes that miss L1 (9 to 15 stall
+// cycles an issue).  DRAM moves 2 to 7% of the copy bandwidth for occlusion and
+// random rays, a quarter of it for full-HD eye rays, whose rays and hits are
+// half the traffic.  So the slab test runs on packed pairs of floats, picks
+// entry planes by the direction's sign, and takes its min and max three at a
+// time; lanes visit runs of nodes between leaves; results are written when a
+// warp refills.  Against four 128-bit loads, scalar slabs and one node or leaf per
 // step: 4M occlusion rays on 2M triangles, FP16 nodes 680 -> 577 us; 1M random
 // rays into 1M triangles, 8-bit nodes, watertight 1,953 -> 1,475 us; full-HD
 // eye rays, binary 185 -> 155 us.
