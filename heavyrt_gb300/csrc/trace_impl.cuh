@@ -749,11 +749,14 @@ __device__ __forceinline__ float min_or_nan(float a, float b)
 // A box is entered when its interval meets the ray's: tn <= tf, tf >= tNear,
 // tn <= t (core/raytrace_common.h:67-80).  Taken as one comparison of the
 // clamped ends, which also asks tNear <= t: without that no triangle can be
-// accepted.  Each of those comparisons fails on a NaN, and so does this one: the
-// ends keep a NaN operand (a ray without a number for its origin, tNear or t
-// ends at the root; with a min and max that drop it, it walked the whole tree).
-__device__ __forceinline__ bool box_hit(float tn, float tf, float tNear, float t)
+// accepted (a ray whose tFar lies before its tNear ends at the root), so only
+// the counting kernels, whose visits are the reference's, compare one by one.
+// Each of those comparisons fails on a NaN, and so does this one: the ends keep
+// a NaN operand (a ray without a number for its origin, tNear or t ends at the
+// root; with a min and max that drop it, it walked the whole tree).
+template <bool COUNT> __device__ __forceinline__ bool box_hit(float tn, float tf, float tNear, float t)
 {
+  if (COUNT) return tn <= tf && tf >= tNear && tn <= t;
   return max_or_nan(tn, tNear) <= min_or_nan(tf, t);
 }
 
@@ -802,8 +805,8 @@ __device__ __forceinline__ int visit_pair(LaneT& L, const Ray<LAYOUT>& r, const 
   }
   const float2 ref = unpack2(b[2]);
   const uint32_t ref0 = __float_as_uint(ref.x), ref1 = __float_as_uint(ref.y);
-  const bool h0 = box_hit(t0n, t0f, r.tNear, L.h.t);
-  const bool h1 = box_hit(t1n, t1f, r.tNear, L.h.t);
+  const bool h0 = box_hit<COUNT>(t0n, t0f, r.tNear, L.h.t);
+  const bool h1 = box_hit<COUNT>(t1n, t1f, r.tNear, L.h.t);
   if (!h0 && !h1) return 1;
   const bool first0 = h0 && (!h1 || t0n <= t1n);
   L.cur = first0 ? ref0 : ref1;
@@ -842,7 +845,7 @@ __device__ __forceinline__ int visit_node(LaneT& L, Stack<THREADS, STACK>& st, u
     bool hit[4];
 #pragma unroll
     for (int k = 0; k < 4; k++)
-      hit[k] = box_hit(key[k], tf[k], L.r.tNear, L.h.t) && (ANY || k < 2 || ref[k] != kEmptyRef);
+      hit[k] = box_hit<COUNT>(key[k], tf[k], L.r.tNear, L.h.t) && (ANY || k < 2 || ref[k] != kEmptyRef);
     // at most three pushes; near the stack's bound they are counted first
     if (L.top > DEPTH - 3 && L.top + (int)hit[0] + (int)hit[1] + (int)hit[2] + (int)hit[3] - 1 > DEPTH)
     {
