@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(kThreads) k_seg_box_final(const uint32_t* __re
       bc::zindex_scale(mn, mx, &params[s], cubic);
       params[s].nLeaves = 0;
       params[s].error = 0;
+      params[s].rootRecord = 0;
+      params[s].pad = 0;
     }
   }
 }
